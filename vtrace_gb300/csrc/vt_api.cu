@@ -211,23 +211,10 @@ static cudaError_t build_launches(const void* d_src, uint32_t format, const uint
     if (e == cudaSuccess) e = launch_brick_scan(s, g.bricks, stream);
     if (e == cudaSuccess)
         e = launch_brick_compact(d_src, format, nx, ny, nz, s, g.dir, g.masks, g.payload, stream);
-    // the occupancy words are no longer needed: their scratch (16 words per brick) holds the
-    // occupancy bitmask of the passes along x (words 13 on), the octant passes, and then the
-    // long-box runs and window minima (words 0-12)
-    uint32_t* occ = (uint32_t*)s.words + 13 * g.bricks;
+    const int32_t bx = (int32_t)g.bx, by = (int32_t)g.by, bz = (int32_t)g.bz;
+    if (e == cudaSuccess) e = launch_brick_lattice(g.dir, g.oct, g.lng, s.lattice, bx, by, bz, stream);
     if (e == cudaSuccess)
-        e = launch_brick_xmask(g.dir, occ, (int32_t)g.bx, (int32_t)g.by, (int32_t)g.bz, stream);
-    if (e == cudaSuccess)
-        e = launch_brick_distance(s, g.dir, (int32_t)g.bx, (int32_t)g.by, (int32_t)g.bz, stream,
-                                  nullptr, occ);
-    if (e == cudaSuccess)
-        e = launch_brick_octants(g.dir, (uint8_t*)s.words,
-                                 (uint16_t*)((uint8_t*)s.words + ((g.bricks + 255) / 256) * 256),
-                                 g.oct, (int32_t)g.bx, (int32_t)g.by, (int32_t)g.bz, stream,
-                                 nullptr, occ);
-    if (e == cudaSuccess)
-        e = launch_brick_long(g.dir, g.oct, (uint32_t*)s.words, g.lng, (int32_t)g.bx,
-                              (int32_t)g.by, (int32_t)g.bz, stream, nullptr, occ);
+        e = launch_brick_distance(g.dir, g.oct, s.lattice, bx, by, bz, stream, nullptr, true);
     return e;
 }
 
@@ -247,7 +234,7 @@ struct SmallBuild {
     void* in = nullptr;          // the shape's dense voxels
     void* tmpl = nullptr;        // block layout with a slot per brick
     void* scratch = nullptr;
-    uint32_t* counts = nullptr;  // last slot offset, last flag, occupied voxels (u64)
+    uint32_t* counts = nullptr;  // last slot offset, last flag, occupied voxels (u64), deep bricks?
     cudaGraphExec_t exec = nullptr;
     uint64_t last_use = 0;
 };
@@ -295,8 +282,9 @@ static int32_t small_entry(const Grid& shape, bool nonzero, SmallBuild*& out) {
     const BlockLayout L = block_layout(shape.bricks, shape.bricks, shape.format);
     if (cudaMalloc(&b.in, (size_t)shape.nx * shape.ny * shape.nz * elem) != cudaSuccess ||
         cudaMalloc(&b.tmpl, L.total) != cudaSuccess ||
-        cudaMalloc(&b.scratch, build_scratch_bytes(shape.bricks)) != cudaSuccess ||
-        cudaMalloc(&b.counts, 16) != cudaSuccess) {
+        cudaMalloc(&b.scratch, build_scratch_bytes((int32_t)shape.bx, (int32_t)shape.by, (int32_t)shape.bz)) !=
+            cudaSuccess ||
+        cudaMalloc(&b.counts, 32) != cudaSuccess) {
         cudaGetLastError();
         small_free(b);
         return fail(VT_ENOMEM, "cudaMalloc(small grid build) failed");
@@ -311,7 +299,8 @@ static int32_t small_entry(const Grid& shape, bool nonzero, SmallBuild*& out) {
     t.bricks = shape.bricks;
     t.format = shape.format;
     point_into_block(t, b.tmpl, L, shape.bricks);
-    const BuildScratch s = carve_build_scratch(b.scratch, shape.bricks);
+    const BuildScratch s =
+        carve_build_scratch(b.scratch, (int32_t)shape.bx, (int32_t)shape.by, (int32_t)shape.bz);
     cudaStream_t cs;
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);
@@ -327,6 +316,8 @@ static int32_t small_entry(const Grid& shape, bool nonzero, SmallBuild*& out) {
                                      cudaMemcpyDeviceToDevice, cs);
             if (le == cudaSuccess)
                 le = cudaMemcpyAsync(b.counts + 2, s.occupied, 8, cudaMemcpyDeviceToDevice, cs);
+            if (le == cudaSuccess)
+                le = cudaMemcpyAsync(b.counts + 4, s.lattice.deep, 4, cudaMemcpyDeviceToDevice, cs);
             e = cudaStreamEndCapture(cs, &graph);
             if (e == cudaSuccess) e = le;
         }
@@ -363,7 +354,7 @@ static int32_t build_small(const void* src, bool src_host, const uint32_t* palet
     }
     point_into_block(*g, block, L, g->bricks);
     g->pooled = true;
-    uint32_t hc[4] = {0, 0, 0, 0};
+    uint32_t hc[5] = {0, 0, 0, 0, 0};
     cudaError_t e = cudaMemcpyAsync(b->in, src, (size_t)g->nx * g->ny * g->nz * elem,
                                     src_host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice,
                                     stream);
@@ -372,11 +363,12 @@ static int32_t build_small(const void* src, bool src_host, const uint32_t* palet
                             stream);
     if (e == cudaSuccess) e = cudaGraphLaunch(b->exec, stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(block, b->tmpl, L.total, cudaMemcpyDeviceToDevice, stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(hc, b->counts, 16, cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(hc, b->counts, 20, cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess) return cuda_fail(e, "small grid build");
     g->nonempty = (uint64_t)hc[0] + hc[1];
     g->occupied = (uint64_t)hc[2] | ((uint64_t)hc[3] << 32);
+    g->deep = hc[4] != 0u;
     g->bytes = g->block_bytes;
     g->slots_used = g->nonempty;
     return VT_OK;
@@ -441,7 +433,8 @@ int32_t build_grid(const void* d_src, uint32_t format, const uint32_t* palette_h
     // compaction copy whole brick blocks instead of re-reading the dense grid (as large again as
     // the padded grid, for the duration of the build; without it the build is the same, slower).
     void* scratch = nullptr;
-    const size_t sbytes = build_scratch_bytes(g->bricks);
+    const int32_t bx = (int32_t)g->bx, by = (int32_t)g->by, bz = (int32_t)g->bz;
+    const size_t sbytes = build_scratch_bytes(bx, by, bz);
     const size_t staged_at = sbytes + 1024;  // 256-aligned: sbytes is
     cudaError_t e = cudaMallocAsync(&scratch, staged_at + build_staging_bytes(g->bricks, format), stream);
     bool staging = e == cudaSuccess;
@@ -453,7 +446,7 @@ int32_t build_grid(const void* d_src, uint32_t format, const uint32_t* palette_h
         cudaGetLastError();
         return fail(VT_ENOMEM, "cudaMallocAsync(brick build scratch) failed");
     }
-    BuildScratch s = carve_build_scratch(scratch, g->bricks);
+    BuildScratch s = carve_build_scratch(scratch, bx, by, bz);
     if (staging) s.staged = (char*)scratch + staged_at;
     uint32_t* d_palette = (uint32_t*)((char*)scratch + sbytes);
     uint32_t counts[2] = {0, 0};
@@ -488,25 +481,19 @@ int32_t build_grid(const void* d_src, uint32_t format, const uint32_t* palette_h
             e = cudaMemcpyAsync(g->palette, d_palette, 1024, cudaMemcpyDeviceToDevice, stream);
             if (e != cudaSuccess) { rc = cuda_fail(e, "cudaMemcpy(palette)"); break; }
         }
-        // compaction (from the words and slot offsets in the scratch), then the distance,
-        // octant and long-box passes: build_launches' sequence after its scan
+        // compaction (from the words and slot offsets in the scratch), then the lattice passes, and
+        // the distance passes when a brick lies far from all occupied ones
         e = launch_brick_compact(d_src, format, (int32_t)nx, (int32_t)ny, (int32_t)nz, s, g->dir,
                                  g->masks, g->payload, stream);
-        uint32_t* occ = (uint32_t*)s.words + 13 * g->bricks;  // as in build_launches
-        if (e == cudaSuccess)
-            e = launch_brick_xmask(g->dir, occ, (int32_t)g->bx, (int32_t)g->by, (int32_t)g->bz, stream);
-        if (e == cudaSuccess)
-            e = launch_brick_distance(s, g->dir, (int32_t)g->bx, (int32_t)g->by, (int32_t)g->bz,
-                                      stream, nullptr, occ);
-        if (e == cudaSuccess)
-            e = launch_brick_octants(g->dir, (uint8_t*)s.words,
-                                     (uint16_t*)((uint8_t*)s.words + ((g->bricks + 255) / 256) * 256),
-                                     g->oct, (int32_t)g->bx, (int32_t)g->by, (int32_t)g->bz, stream,
-                                     nullptr, occ);
-        if (e == cudaSuccess)
-            e = launch_brick_long(g->dir, g->oct, (uint32_t*)s.words, g->lng, (int32_t)g->bx,
-                                  (int32_t)g->by, (int32_t)g->bz, stream, nullptr, occ);
+        if (e == cudaSuccess) e = launch_brick_lattice(g->dir, g->oct, g->lng, s.lattice, bx, by, bz, stream);
+        uint32_t deep = 0;
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&deep, s.lattice.deep, 4, cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+        if (e == cudaSuccess && deep) {
+            g->deep = true;
+            e = launch_brick_distance(g->dir, g->oct, s.lattice, bx, by, bz, stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+        }
         if (e != cudaSuccess) { rc = cuda_fail(e, "brick build"); break; }
         g->bytes = g->block_bytes;
         g->slots_used = g->nonempty;

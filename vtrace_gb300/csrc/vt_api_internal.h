@@ -38,6 +38,8 @@ struct Grid {
     void* block = nullptr;
     size_t block_bytes = 0;
     bool pooled = false;  // `block` comes from the stream-ordered pool
+    // some brick has, or has had, no occupied brick within 14: updates run the distance passes
+    bool deep = false;
     size_t bytes = 0;
     // slots of masks/payload: allocated, handed out (high-water mark), and freed by updates
     uint64_t slot_capacity = 0, slots_used = 0;

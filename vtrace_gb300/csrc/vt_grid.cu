@@ -37,20 +37,30 @@ static uint64_t scan_partials(uint64_t n) {
     return total + 64;
 }
 
-size_t build_scratch_bytes(uint64_t bricks) {
-    return (size_t)(align_up(bricks * 64, 256) + align_up(bricks * 4, 256) * 2 +
-                    align_up(scan_partials(bricks) * 4, 256) + 256 + align_up(bricks, 256) * 2);
+// The occupancy words are not read after the compaction: the lattice passes take their space.
+static uint64_t words_bytes(int32_t bx, int32_t by, int32_t bz) {
+    const uint64_t words = (uint64_t)bx * by * bz * 64;
+    const uint64_t lattice = lattice_scratch_bytes(bx, by, bz);
+    return align_up(words > lattice ? words : lattice, 256);
+}
+
+size_t build_scratch_bytes(int32_t bx, int32_t by, int32_t bz) {
+    const uint64_t bricks = (uint64_t)bx * by * bz;
+    return (size_t)(words_bytes(bx, by, bz) + align_up(bricks * 4, 256) * 2 +
+                    align_up(scan_partials(bricks) * 4, 256) + 256);
 }
 
 size_t build_staging_bytes(uint64_t bricks, uint32_t format) {
     return (size_t)align_up(bricks * 512 * (format == VT_PAYLOAD_RGBA8 ? 4 : 1), 256);
 }
 
-BuildScratch carve_build_scratch(void* base, uint64_t bricks) {
+BuildScratch carve_build_scratch(void* base, int32_t bx, int32_t by, int32_t bz) {
+    const uint64_t bricks = (uint64_t)bx * by * bz;
     char* p = (char*)base;
     BuildScratch s;
     s.words = (uint64_t*)p;
-    p += align_up(bricks * 64, 256);
+    s.lattice = carve_lattice_scratch(p, bx, by, bz);
+    p += words_bytes(bx, by, bz);
     s.flags = (uint32_t*)p;
     p += align_up(bricks * 4, 256);
     s.offsets = (uint32_t*)p;
@@ -58,10 +68,6 @@ BuildScratch carve_build_scratch(void* base, uint64_t bricks) {
     s.block_sums = (uint32_t*)p;
     p += align_up(scan_partials(bricks) * 4, 256);
     s.occupied = (unsigned long long*)p;
-    p += 256;
-    s.dist_a = (uint8_t*)p;
-    p += align_up(bricks, 256);
-    s.dist_b = (uint8_t*)p;
     return s;
 }
 
@@ -76,19 +82,6 @@ __device__ __forceinline__ BrickCoord brick_coord(uint64_t brick, int32_t bx, in
     c.byi = (int32_t)(r % (uint64_t)by);
     c.bzi = (int32_t)(r / (uint64_t)by);
     return c;
-}
-
-// Brick of thread (blockIdx.x * blockDim.x + threadIdx.x) in `box`; false past its end.
-__device__ __forceinline__ bool box_brick(const BrickBox& box, int32_t bx, int32_t by,
-                                          BrickCoord& c, uint64_t& b) {
-    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (uint64_t)box.nx * box.ny * box.nz) return false;
-    c.bxi = box.x0 + (int32_t)(t % (uint64_t)box.nx);
-    const uint64_t r = t / (uint64_t)box.nx;
-    c.byi = box.y0 + (int32_t)(r % (uint64_t)box.ny);
-    c.bzi = box.z0 + (int32_t)(r / (uint64_t)box.ny);
-    b = (uint64_t)c.bxi + (uint64_t)bx * ((uint64_t)c.byi + (uint64_t)by * (uint64_t)c.bzi);
-    return true;
 }
 
 // Occupancy bits of 8 u8 voxels packed in a u64 when "occupied" means "nonzero index": the high
@@ -354,7 +347,7 @@ __global__ void __launch_bounds__(256) brick_compact_kernel(
     if (brick >= bricks) return;
     const uint32_t f = __ldg(flags + brick);
     const uint32_t slot = __ldg(offsets + brick);
-    if (lz == 0) dir[brick] = f ? slot : kEmptyBit;  // distance filled in by the distance passes
+    if (lz == 0) dir[brick] = f ? slot : kEmptyBit;  // distance filled in by the lattice passes
     if (!f) return;
     masks[(size_t)slot * 8 + lz] = __ldg(words + brick * 8 + lz);
     if (staged) {
@@ -384,486 +377,6 @@ cudaError_t launch_brick_compact(const void* src, uint32_t format, int32_t nx, i
         brick_compact_kernel<VT_PAYLOAD_RGBA8><<<blocks, 256, 0, stream>>>(
             src, nx, ny, nz, bx, by, bricks, s.words, s.flags, s.offsets, dir, masks, payload,
             s.staged);
-    return cudaGetLastError();
-}
-
-// Occupancy bitmask of the brick lattice for the passes along x: row (y, z) is occ_words(bx) words,
-// bit x of the row set iff brick (x, y, z) is occupied.  One thread per word.
-__host__ __device__ __forceinline__ int32_t occ_words(int32_t bx) { return (bx + 31) >> 5; }
-
-__global__ void __launch_bounds__(256) brick_xmask_kernel(const uint32_t* __restrict__ dir,
-                                                          uint32_t* __restrict__ occ, int32_t bx,
-                                                          int32_t by, int32_t y0, int32_t ny,
-                                                          int32_t z0, uint64_t words) {
-    // words of the rows y0 .. y0 + ny - 1 of the planes z0 ..
-    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= words) return;
-    const int32_t rw = occ_words(bx);
-    const uint64_t r = t / (uint64_t)rw;
-    const uint64_t row = (uint64_t)(z0 + (int32_t)(r / (uint64_t)ny)) * by + y0 + (int32_t)(r % (uint64_t)ny);
-    const int32_t x0 = (int32_t)(t - r * (uint64_t)rw) * 32;
-    const uint64_t w = row * rw + (uint64_t)(x0 >> 5);
-    const uint32_t* d = dir + row * (uint64_t)bx + x0;
-    const int32_t n = min(32, bx - x0);
-    uint32_t m = 0;
-    for (int32_t k = 0; k < n; ++k) m |= (uint32_t)!brick_empty(__ldg(d + k)) << k;
-    occ[w] = m;
-}
-
-// Steps from brick x of an occupancy row to the nearest occupied brick in direction s (+1 / -1),
-// the brick itself included (0 when occupied), or `cap` (<= 31) when none lies within cap - 1
-// steps; beyond the row counts as empty.  Reads at most two words.
-__device__ __forceinline__ int32_t occ_fwd(const uint32_t* __restrict__ row, int32_t rw, int32_t x,
-                                           int32_t s, int32_t cap) {
-    const int32_t w = x >> 5, b = x & 31;
-    if (s > 0) {
-        uint64_t v = __ldg(row + w);
-        if (w + 1 < rw) v |= (uint64_t)__ldg(row + w + 1) << 32;
-        const uint32_t m = (uint32_t)(v >> b) & ((1u << cap) - 1u);  // bit k: brick x + k
-        return m ? __ffs(m) - 1 : cap;
-    }
-    uint64_t v = (uint64_t)__ldg(row + w) << 32;
-    if (w > 0) v |= __ldg(row + w - 1);
-    const uint32_t m = (uint32_t)((v << (31 - b)) >> 32) & ~((1u << (32 - cap)) - 1u);  // bit 31 - k: brick x - k
-    return m ? __clz(m) : cap;
-}
-
-cudaError_t launch_brick_xmask(const uint32_t* dir, uint32_t* occ, int32_t bx, int32_t by,
-                               int32_t bz, cudaStream_t stream, const BrickBox* changed) {
-    // after a change, the rows the passes along x read: those of the distance pass's window (its
-    // y and z reach, kMaxBrickDistance twice over, covers the octant and long-box windows)
-    int32_t y0 = 0, ny = by, z0 = 0, nz = bz;
-    if (changed) {
-        const int32_t R = 2 * (int32_t)kMaxBrickDistance;
-        y0 = max(changed->y0 - R, 0);
-        z0 = max(changed->z0 - R, 0);
-        ny = min(changed->y0 + changed->ny + R, by) - y0;
-        nz = min(changed->z0 + changed->nz + R, bz) - z0;
-    }
-    const uint64_t words = (uint64_t)occ_words(bx) * ny * nz;
-    brick_xmask_kernel<<<(unsigned)((words + 255) / 256), 256, 0, stream>>>(dir, occ, bx, by, y0,
-                                                                             ny, z0, words);
-    return cudaGetLastError();
-}
-
-size_t brick_xmask_words(int32_t bx, int32_t by, int32_t bz) {
-    return (size_t)occ_words(bx) * by * bz;
-}
-
-// Chebyshev (L-infinity) distance, in bricks, from each empty brick to the nearest occupied one,
-// capped at kMaxBrickDistance.  The transform is separable: pass x computes the 1D distance
-// along x; passes y and z take min over the line of max(|offset|, previous pass), which composes
-// max over axes.  Each thread handles one brick and scans a window of +-kMaxBrickDistance.
-template <int AXIS>
-__global__ void __launch_bounds__(256) brick_distance_kernel(uint32_t* __restrict__ dir,
-                                                             const uint8_t* __restrict__ in,
-                                                             uint8_t* __restrict__ out,
-                                                             int32_t bx, int32_t by, int32_t bz,
-                                                             BrickBox box,
-                                                             const uint32_t* __restrict__ occ) {
-    BrickCoord c;
-    uint64_t b;
-    if (!box_brick(box, bx, by, c, b)) return;
-    if (AXIS == 0 && occ) {  // pass x from the occupancy rows
-        const int32_t rw = occ_words(bx);
-        const uint32_t* row = occ + ((uint64_t)c.bzi * by + c.byi) * rw;
-        const int32_t cap = (int32_t)kMaxBrickDistance;
-        out[b] = (uint8_t)min(occ_fwd(row, rw, c.bxi, 1, cap), occ_fwd(row, rw, c.bxi, -1, cap));
-        return;
-    }
-    const int32_t pos = AXIS == 0 ? c.bxi : (AXIS == 1 ? c.byi : c.bzi);
-    const int32_t n = AXIS == 0 ? bx : (AXIS == 1 ? by : bz);
-    const int64_t stride = AXIS == 0 ? 1 : (AXIS == 1 ? (int64_t)bx : (int64_t)bx * by);
-    const int32_t cap = (int32_t)kMaxBrickDistance;
-    // min over offsets j of max(|j|, val(pos + j)), visiting |j| = 0, 1, 2, ... and stopping once
-    // |j| reaches the best value found (no farther offset can improve it)
-    int32_t best = cap;
-    for (int32_t r = 0; r < best; ++r) {
-#pragma unroll
-        for (int sgn = 0; sgn < 2; ++sgn) {
-            if (r == 0 && sgn) continue;
-            const int32_t p = sgn ? pos - r : pos + r;
-            if (p < 0 || p >= n) continue;
-            const int64_t idx = (int64_t)b + (int64_t)(p - pos) * stride;
-            const int32_t val = AXIS == 0 ? (brick_empty(__ldg(dir + idx)) ? cap : 0) : (int32_t)__ldg(in + idx);
-            best = min(best, max(r, val));
-        }
-    }
-    if (AXIS < 2) {
-        out[b] = (uint8_t)best;
-    } else if (brick_empty(dir[b])) {
-        dir[b] = kEmptyBit | (uint32_t)max(best, 1);
-    }
-}
-
-// Forward (octant) distances: for every brick and each of the 8 sign combinations (sx, sy, sz) of
-// a ray direction, the largest K <= kMaxOctantDistance such that the box of K x K x K bricks
-// starting at the brick and extending in the directions (sx, sy, sz) holds no occupied brick
-// (0 for an occupied brick).  Separable: pass x gives the 1D forward distance for sx = +/-1,
-// pass y takes min_j max(j, pass_x(b + j*sy)) for the four (sx, sy), pass z likewise for all
-// eight.  Packed 4 bits per octant, octant index (sx<0) | (sy<0)<<1 | (sz<0)<<2.
-constexpr int kMaxOctantDistance = 15;
-
-__global__ void __launch_bounds__(256) brick_octant_x_kernel(const uint32_t* __restrict__ dir,
-                                                             uint8_t* __restrict__ out,
-                                                             int32_t bx, int32_t by,
-                                                             BrickBox box,
-                                                             const uint32_t* __restrict__ occ) {
-    BrickCoord c;
-    uint64_t b;
-    if (!box_brick(box, bx, by, c, b)) return;
-    if (occ) {
-        const int32_t rw = occ_words(bx);
-        const uint32_t* row = occ + ((uint64_t)c.bzi * by + c.byi) * rw;
-        const int32_t cap = (int32_t)kMaxOctantDistance;
-        out[b] = (uint8_t)(occ_fwd(row, rw, c.bxi, 1, cap) | (occ_fwd(row, rw, c.bxi, -1, cap) << 4));
-        return;
-    }
-    uint32_t packed = 0;
-#pragma unroll
-    for (int neg = 0; neg < 2; ++neg) {
-        const int32_t sx = neg ? -1 : 1;
-        int32_t best = kMaxOctantDistance;
-        for (int32_t k = 0; k < kMaxOctantDistance; ++k) {
-            const int32_t x = c.bxi + k * sx;
-            if (x < 0 || x >= bx) break;
-            if (!brick_empty(__ldg(dir + (int64_t)b + (int64_t)k * sx))) {
-                best = k;
-                break;
-            }
-        }
-        packed |= (uint32_t)best << (4 * neg);
-    }
-    out[b] = (uint8_t)packed;
-}
-
-__global__ void __launch_bounds__(256) brick_octant_y_kernel(const uint8_t* __restrict__ in,
-                                                             uint16_t* __restrict__ out,
-                                                             int32_t bx, int32_t by,
-                                                             BrickBox box) {
-    BrickCoord c;
-    uint64_t b;
-    if (!box_brick(box, bx, by, c, b)) return;
-    uint32_t packed = 0;
-#pragma unroll
-    for (int ny = 0; ny < 2; ++ny) {  // one walk per sy serves both sx
-        const int32_t sy = ny ? -1 : 1;
-        int32_t best[2] = {(int32_t)kMaxOctantDistance, (int32_t)kMaxOctantDistance};
-        for (int32_t j = 0; j < max(best[0], best[1]); ++j) {
-            const int32_t y = c.byi + j * sy;
-            if (y < 0 || y >= by) break;
-            const uint32_t f = __ldg(in + (int64_t)b + (int64_t)j * sy * bx);
-#pragma unroll
-            for (int nx = 0; nx < 2; ++nx) best[nx] = min(best[nx], max(j, (int32_t)((f >> (4 * nx)) & 15u)));
-        }
-#pragma unroll
-        for (int nx = 0; nx < 2; ++nx) packed |= (uint32_t)best[nx] << (4 * (nx | (ny << 1)));
-    }
-    out[b] = (uint16_t)packed;
-}
-
-__global__ void __launch_bounds__(256) brick_octant_z_kernel(const uint16_t* __restrict__ in,
-                                                             uint32_t* __restrict__ out,
-                                                             int32_t bx, int32_t by, int32_t bz,
-                                                             BrickBox box) {
-    BrickCoord c;
-    uint64_t b;
-    if (!box_brick(box, bx, by, c, b)) return;
-    const int64_t plane = (int64_t)bx * by;
-    uint32_t packed = 0;
-#pragma unroll
-    for (int nz = 0; nz < 2; ++nz) {  // one walk per sz serves the four (sx, sy)
-        const int32_t sz = nz ? -1 : 1;
-        int32_t best[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) best[q] = (int32_t)kMaxOctantDistance;
-        int32_t lim = (int32_t)kMaxOctantDistance;
-        for (int32_t l = 0; l < lim; ++l) {
-            const int32_t z = c.bzi + l * sz;
-            if (z < 0 || z >= bz) break;
-            const uint32_t f = __ldg(in + (int64_t)b + (int64_t)l * sz * plane);
-            lim = 0;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                best[q] = min(best[q], max(l, (int32_t)((f >> (4 * q)) & 15u)));
-                lim = max(lim, best[q]);
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) packed |= (uint32_t)best[q] << (4 * (q | (nz << 2)));
-    }
-    out[b] = packed;
-}
-
-// Forward empty runs: for axis a and direction s = +1 / -1, the number of consecutive empty
-// bricks from this one (itself included) toward s along a, capped at kMaxOctantDistance; beyond the
-// grid counts as empty.  Nibble 2a + (s < 0).
-__global__ void __launch_bounds__(256) brick_run_kernel(const uint32_t* __restrict__ dir,
-                                                        uint32_t* __restrict__ run, int32_t bx,
-                                                        int32_t by, int32_t bz, BrickBox box,
-                                                        const uint32_t* __restrict__ occ) {
-    BrickCoord c;
-    uint64_t b;
-    if (!box_brick(box, bx, by, c, b)) return;
-    const int32_t pos[3] = {c.bxi, c.byi, c.bzi}, n[3] = {bx, by, bz};
-    const int64_t stride[3] = {1, (int64_t)bx, (int64_t)bx * by};
-    uint32_t packed = 0;
-    int a0 = 0;
-    if (occ) {  // axis x from the occupancy rows
-        const int32_t rw = occ_words(bx);
-        const uint32_t* row = occ + ((uint64_t)c.bzi * by + c.byi) * rw;
-        const int32_t cap = (int32_t)kMaxOctantDistance;
-        packed = (uint32_t)occ_fwd(row, rw, c.bxi, 1, cap) | ((uint32_t)occ_fwd(row, rw, c.bxi, -1, cap) << 4);
-        a0 = 1;
-    }
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        if (a < a0) continue;
-#pragma unroll
-        for (int neg = 0; neg < 2; ++neg) {
-            const int32_t sg = neg ? -1 : 1;
-            int32_t best = kMaxOctantDistance;
-            for (int32_t k = 0; k < (int32_t)kMaxOctantDistance; ++k) {
-                const int32_t p = pos[a] + k * sg;
-                if (p < 0 || p >= n[a]) break;
-                if (!brick_empty(__ldg(dir + (int64_t)b + (int64_t)k * sg * stride[a]))) {
-                    best = k;
-                    break;
-                }
-            }
-            packed |= (uint32_t)best << (4 * (2 * a + neg));
-        }
-    }
-    run[b] = packed;
-}
-
-// Window minima of the runs: level p of axis a holds, for octant o (nibble o), the smallest run
-// along a toward o over the 2^p x 2^p bricks across from the brick toward o (cells beyond the
-// grid count as the cap).  Level 0 repacks the runs per octant; level p + 1 is the minimum of four
-// level-p blocks.  The levels are stored for the bricks of the index window `pw` (the whole
-// lattice for a full build): pyr[(p * 3 + a) * |pw| + local index in pw].
-__device__ __forceinline__ int64_t pyr_index(const BrickBox& pw, int32_t x, int32_t y, int32_t z) {
-    if (x < pw.x0 || y < pw.y0 || z < pw.z0 || x >= pw.x0 + pw.nx || y >= pw.y0 + pw.ny ||
-        z >= pw.z0 + pw.nz)
-        return -1;  // not stored: the windows of a partial pass are nested so that this is not read
-    return (int64_t)(x - pw.x0) + (int64_t)pw.nx * ((int64_t)(y - pw.y0) + (int64_t)pw.ny * (z - pw.z0));
-}
-
-// WIN: `pw` is a window of the lattice (a partial pass, whose windows are nested so that every
-// neighbour read lies in it; checked all the same); otherwise it is the whole lattice and the local
-// index is the brick index.  Neighbours are addressed by local strides.
-template <bool WIN>
-__device__ __forceinline__ bool pyr_in(const BrickBox& pw, int a, int32_t v) {
-    if (!WIN) return true;
-    const int32_t lo = a == 0 ? pw.x0 : (a == 1 ? pw.y0 : pw.z0);
-    const int32_t n = a == 0 ? pw.nx : (a == 1 ? pw.ny : pw.nz);
-    return v >= lo && v < lo + n;
-}
-
-template <bool WIN>
-__global__ void __launch_bounds__(256) brick_pyramid_kernel(const uint32_t* __restrict__ run,
-                                                            uint32_t* __restrict__ pyr, int32_t p,
-                                                            int32_t bx, int32_t by, int32_t bz,
-                                                            BrickBox box, BrickBox pw) {
-    BrickCoord c;
-    uint64_t b;
-    if (!box_brick(box, bx, by, c, b)) return;
-    const uint64_t pn = (uint64_t)pw.nx * pw.ny * pw.nz;
-    const int32_t pos[3] = {c.bxi, c.byi, c.bzi}, n[3] = {bx, by, bz};
-    const int64_t ls[3] = {1, (int64_t)pw.nx, (int64_t)pw.nx * pw.ny};
-    const int64_t self_i = WIN ? pyr_index(pw, c.bxi, c.byi, c.bzi) : (int64_t)b;
-    if (self_i < 0) return;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        uint32_t packed = 0;
-        if (p == 0) {
-            const uint32_t r = __ldg(run + b);
-#pragma unroll
-            for (int o = 0; o < 8; ++o) packed |= ((r >> (4 * (2 * a + ((o >> a) & 1)))) & 15u) << (4 * o);
-        } else {
-            const int e1 = (a + 1) % 3, e2 = (a + 2) % 3;
-            const int32_t h = 1 << (p - 1);
-            const uint32_t* prev = pyr + (uint64_t)((p - 1) * 3 + a) * pn;
-            const uint32_t self = __ldg(prev + self_i);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {  // lateral signs (bit 0: e1 negative, bit 1: e2 negative)
-                const int32_t s1 = (q & 1) ? -1 : 1, s2 = (q & 2) ? -1 : 1;
-                const int32_t c1 = pos[e1] + h * s1, c2 = pos[e2] + h * s2;
-                const bool in1 = c1 >= 0 && c1 < n[e1] && pyr_in<WIN>(pw, e1, c1);
-                const bool in2 = c2 >= 0 && c2 < n[e2] && pyr_in<WIN>(pw, e2, c2);
-                const int64_t d1 = (int64_t)h * s1 * ls[e1], d2 = (int64_t)h * s2 * ls[e2];
-                const uint32_t w1 = in1 ? __ldg(prev + self_i + d1) : 0xFFFFFFFFu;
-                const uint32_t w2 = in2 ? __ldg(prev + self_i + d2) : 0xFFFFFFFFu;
-                const uint32_t w3 = in1 && in2 ? __ldg(prev + self_i + d1 + d2) : 0xFFFFFFFFu;
-#pragma unroll
-                for (int o = 0; o < 8; ++o) {
-                    if (((o >> e1) & 1) != (q & 1) || ((o >> e2) & 1) != ((q >> 1) & 1)) continue;
-                    const uint32_t sh = 4 * o;
-                    const uint32_t m = min(min((self >> sh) & 15u, (w1 >> sh) & 15u),
-                                           min((w2 >> sh) & 15u, (w3 >> sh) & 15u));
-                    packed |= m << sh;
-                }
-            }
-        }
-        pyr[(uint64_t)(p * 3 + a) * pn + self_i] = packed;
-    }
-}
-
-// Long forward boxes: for axis a and octant o with forward cube K (octant word), the largest
-// L <= kMaxOctantDistance such that the box L bricks long along a and K x K across, all toward o,
-// is empty: the smallest run along a over the box's K x K cross-section, read as the minimum of
-// four overlapping 2^p blocks of the pyramid (2^p <= K < 2^(p+1)).  L >= K since the cube is
-// empty; K = 0 (occupied brick) gives 0 and K at the cap gives the cap.
-template <bool WIN>
-__global__ void __launch_bounds__(256) brick_long_kernel(const uint32_t* __restrict__ oct,
-                                                         const uint32_t* __restrict__ pyr,
-                                                         uint32_t* __restrict__ lng, int32_t bx,
-                                                         int32_t by, int32_t bz, BrickBox box,
-                                                         BrickBox pw) {
-    BrickCoord c;
-    uint64_t b;
-    if (!box_brick(box, bx, by, c, b)) return;
-    const uint64_t bricks = (uint64_t)bx * by * bz;
-    const uint64_t pn = (uint64_t)pw.nx * pw.ny * pw.nz;
-    const int32_t pos[3] = {c.bxi, c.byi, c.bzi}, n[3] = {bx, by, bz};
-    const int64_t ls[3] = {1, (int64_t)pw.nx, (int64_t)pw.nx * pw.ny};
-    const int64_t self_i = WIN ? pyr_index(pw, c.bxi, c.byi, c.bzi) : (int64_t)b;
-    const uint32_t ow = __ldg(oct + b);
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const int e1 = (a + 1) % 3, e2 = (a + 2) % 3;
-        uint32_t packed = 0;
-        for (int o = 0; o < 8; ++o) {
-            const int32_t K = (int32_t)((ow >> (4 * o)) & 15u);
-            int32_t L = K;
-            if (K > 0 && K < (int32_t)kMaxOctantDistance && self_i >= 0) {
-                const int32_t p = 31 - __clz(K);  // 2^p <= K < 2^(p+1), p <= 3
-                const int32_t off = K - (1 << p);
-                const int32_t s1 = (o >> e1) & 1 ? -1 : 1, s2 = (o >> e2) & 1 ? -1 : 1;
-                const uint32_t* lev = pyr + (uint64_t)(p * 3 + a) * pn;
-                L = kMaxOctantDistance;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const int32_t o1 = (k & 1) ? off : 0, o2 = (k & 2) ? off : 0;
-                    const int32_t c1 = pos[e1] + o1 * s1, c2 = pos[e2] + o2 * s2;
-                    if (c1 < 0 || c1 >= n[e1] || c2 < 0 || c2 >= n[e2]) continue;
-                    if (!pyr_in<WIN>(pw, e1, c1) || !pyr_in<WIN>(pw, e2, c2)) continue;
-                    const int64_t cc = self_i + (int64_t)o1 * s1 * ls[e1] + (int64_t)o2 * s2 * ls[e2];
-                    L = min(L, (int32_t)((__ldg(lev + cc) >> (4 * o)) & 15u));
-                }
-                L = max(L, K);
-            }
-            packed |= (uint32_t)L << (4 * o);
-        }
-        lng[(uint64_t)a * bricks + b] = packed;
-    }
-}
-
-static unsigned box_blocks(const BrickBox& b) {
-    return (unsigned)(((uint64_t)b.nx * b.ny * b.nz + 255) / 256);
-}
-
-// The box grown by (gx, gy, gz) bricks on each side, clipped to the lattice.
-static BrickBox grow(const BrickBox& b, int32_t gx, int32_t gy, int32_t gz, int32_t bx, int32_t by,
-                     int32_t bz) {
-    BrickBox r;
-    r.x0 = max(b.x0 - gx, 0);
-    r.y0 = max(b.y0 - gy, 0);
-    r.z0 = max(b.z0 - gz, 0);
-    r.nx = min(b.x0 + b.nx + gx, bx) - r.x0;
-    r.ny = min(b.y0 + b.ny + gy, by) - r.y0;
-    r.nz = min(b.z0 + b.nz + gz, bz) - r.z0;
-    return r;
-}
-
-cudaError_t launch_brick_octants(const uint32_t* dir, uint8_t* tmp_x, uint16_t* tmp_y,
-                                 uint32_t* oct, int32_t bx, int32_t by, int32_t bz,
-                                 cudaStream_t stream, const BrickBox* changed,
-                                 const uint32_t* occ) {
-    // pass z at the bricks within reach of a change reads pass y up to 14 bricks away in z, which
-    // reads pass x up to 14 away in y
-    const int32_t R = (int32_t)kMaxOctantDistance - 1;
-    const BrickBox all = {0, 0, 0, bx, by, bz};
-    const BrickBox w = changed ? grow(*changed, R, R, R, bx, by, bz) : all;
-    const BrickBox wy = grow(w, 0, 0, R, bx, by, bz), wx = grow(w, 0, R, R, bx, by, bz);
-    brick_octant_x_kernel<<<box_blocks(wx), 256, 0, stream>>>(dir, tmp_x, bx, by, wx, occ);
-    brick_octant_y_kernel<<<box_blocks(wy), 256, 0, stream>>>(tmp_x, tmp_y, bx, by, wy);
-    brick_octant_z_kernel<<<box_blocks(w), 256, 0, stream>>>(tmp_y, oct, bx, by, bz, w);
-    return cudaGetLastError();
-}
-
-// Index windows of the long-box passes after a change inside `changed`: long words within 15
-// bricks of it; the pyramid's level 3 within 6 more (the long kernel reads level p up to
-// K - 2^p <= 6 bricks across), level 2 within 4 more, level 1 within 2, level 0 and the runs
-// within 1 (level p + 1 reads level p 2^p bricks across).
-struct LongWindows {
-    BrickBox w, wp[4];
-};
-
-static LongWindows long_windows(const BrickBox& changed, int32_t bx, int32_t by, int32_t bz);
-
-size_t brick_long_scratch_words(const BrickBox* changed, int32_t bx, int32_t by, int32_t bz) {
-    const uint64_t bricks = (uint64_t)bx * by * bz;
-    if (!changed) return (size_t)(13 * bricks);
-    const BrickBox& p0 = long_windows(*changed, bx, by, bz).wp[0];
-    return (size_t)(bricks + 12ull * (uint64_t)p0.nx * p0.ny * p0.nz);
-}
-
-cudaError_t launch_brick_long(const uint32_t* dir, const uint32_t* oct, uint32_t* tmp,
-                              uint32_t* lng, int32_t bx, int32_t by, int32_t bz,
-                              cudaStream_t stream, const BrickBox* changed,
-                              const uint32_t* occ) {
-    // tmp: runs (1 word per brick), then the pyramid (12 words per brick of its index window)
-    const uint64_t bricks = (uint64_t)bx * by * bz;
-    uint32_t* run = tmp;
-    uint32_t* pyr = tmp + bricks;
-    const BrickBox all = {0, 0, 0, bx, by, bz};
-    LongWindows L;
-    if (changed) {
-        L = long_windows(*changed, bx, by, bz);
-    } else {
-        L.w = all;
-        for (int p = 0; p < 4; ++p) L.wp[p] = all;
-    }
-    brick_run_kernel<<<box_blocks(L.wp[0]), 256, 0, stream>>>(dir, run, bx, by, bz, L.wp[0], occ);
-    for (int32_t p = 0; p < 4; ++p) {
-        if (changed)
-            brick_pyramid_kernel<true><<<box_blocks(L.wp[p]), 256, 0, stream>>>(
-                run, pyr, p, bx, by, bz, L.wp[p], L.wp[0]);
-        else
-            brick_pyramid_kernel<false><<<box_blocks(L.wp[p]), 256, 0, stream>>>(
-                run, pyr, p, bx, by, bz, L.wp[p], L.wp[0]);
-    }
-    if (changed)
-        brick_long_kernel<true><<<box_blocks(L.w), 256, 0, stream>>>(oct, pyr, lng, bx, by, bz, L.w, L.wp[0]);
-    else
-        brick_long_kernel<false><<<box_blocks(L.w), 256, 0, stream>>>(oct, pyr, lng, bx, by, bz, L.w, L.wp[0]);
-    return cudaGetLastError();
-}
-
-static LongWindows long_windows(const BrickBox& changed, int32_t bx, int32_t by, int32_t bz) {
-    const int32_t R = (int32_t)kMaxOctantDistance;
-    LongWindows L;
-    L.w = grow(changed, R, R, R, bx, by, bz);
-    L.wp[3] = grow(L.w, 6, 6, 6, bx, by, bz);
-    L.wp[2] = grow(L.wp[3], 4, 4, 4, bx, by, bz);
-    L.wp[1] = grow(L.wp[2], 2, 2, 2, bx, by, bz);
-    L.wp[0] = grow(L.wp[1], 1, 1, 1, bx, by, bz);
-    return L;
-}
-
-cudaError_t launch_brick_distance(const BuildScratch& s, uint32_t* dir, int32_t bx, int32_t by,
-                                  int32_t bz, cudaStream_t stream, const BrickBox* changed,
-                                  const uint32_t* occ) {
-    // distances change only within kMaxBrickDistance of a change; each pass reads the previous
-    // one up to that far along its axis
-    const int32_t R = (int32_t)kMaxBrickDistance;
-    const BrickBox all = {0, 0, 0, bx, by, bz};
-    const BrickBox w = changed ? grow(*changed, R, R, R, bx, by, bz) : all;
-    const BrickBox w1 = grow(w, 0, 0, R, bx, by, bz), w0 = grow(w, 0, R, R, bx, by, bz);
-    brick_distance_kernel<0><<<box_blocks(w0), 256, 0, stream>>>(dir, nullptr, s.dist_a, bx, by, bz, w0, occ);
-    brick_distance_kernel<1><<<box_blocks(w1), 256, 0, stream>>>(dir, s.dist_a, s.dist_b, bx, by, bz, w1, nullptr);
-    brick_distance_kernel<2><<<box_blocks(w), 256, 0, stream>>>(dir, s.dist_b, nullptr, bx, by, bz, w, nullptr);
     return cudaGetLastError();
 }
 

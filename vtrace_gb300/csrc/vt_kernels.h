@@ -54,23 +54,38 @@ cudaError_t launch_trace_rays(const GridView& g, const vt_ray* rays, uint64_t n,
                               Counters* counters, cudaStream_t stream,
                               const unsigned int* n_dev = nullptr);
 
-// Scratch of one brick build, sized for `bricks` bricks.
+// A box of bricks: origin and extent in brick coordinates.
+struct BrickBox {
+    int32_t x0, y0, z0, nx, ny, nz;
+};
+
+// Scratch of the lattice passes (vt_lattice.cu): occupancy bit rows along x, y and z, one byte per
+// brick for the distance passes, and a word that is nonzero when some brick has no occupied brick
+// within 14.
+struct LatticeScratch {
+    uint32_t* rows[3] = {nullptr, nullptr, nullptr};
+    uint8_t* dist = nullptr;
+    uint32_t* deep = nullptr;
+};
+size_t lattice_scratch_bytes(int32_t bx, int32_t by, int32_t bz);  // at most 13 per brick + padding
+LatticeScratch carve_lattice_scratch(void* base, int32_t bx, int32_t by, int32_t bz);  // 16-byte aligned
+
+// Scratch of one brick build of bx x by x bz bricks.
 struct BuildScratch {
     uint64_t* words = nullptr;      // bricks * 8 occupancy words
     uint32_t* flags = nullptr;      // bricks: 1 if the brick holds an occupied voxel
     uint32_t* offsets = nullptr;    // bricks: exclusive prefix sum of flags (the slot)
     uint32_t* block_sums = nullptr; // scan partials
     unsigned long long* occupied = nullptr;
-    uint8_t* dist_a = nullptr;      // bricks: distance transform, first pass
-    uint8_t* dist_b = nullptr;      // bricks: distance transform, second pass
+    LatticeScratch lattice;         // in the place of `words`, which the compaction reads last
     // nullptr, or build_staging_bytes(): the voxels of each occupied brick as a 512-voxel block
     // at brick * 512, written by the words pass and copied by the compaction
     void* staged = nullptr;
 };
-size_t build_scratch_bytes(uint64_t bricks);
+size_t build_scratch_bytes(int32_t bx, int32_t by, int32_t bz);
 size_t build_staging_bytes(uint64_t bricks, uint32_t format);
-// Carves BuildScratch out of one buffer of build_scratch_bytes(bricks) bytes.
-BuildScratch carve_build_scratch(void* base, uint64_t bricks);
+// Carves BuildScratch out of one buffer of build_scratch_bytes(bx, by, bz) bytes.
+BuildScratch carve_build_scratch(void* base, int32_t bx, int32_t by, int32_t bz);
 
 // Phase 1: occupancy words, brick flags and the occupied-voxel count; phase 2: slots.
 cudaError_t launch_brick_words(const void* src, uint32_t format, const uint32_t* d_palette,
@@ -86,38 +101,18 @@ cudaError_t launch_brick_compact(const void* src, uint32_t format, int32_t nx, i
                                  int32_t nz, const BuildScratch& s, uint32_t* dir,
                                  uint64_t* masks, void* payload, cudaStream_t stream);
 
-// Phase 5: forward distances per ray octant (4 bits x 8 per brick) into `oct`; tmp_x holds one
-// byte and tmp_y two bytes per brick.
-// A box of bricks: origin and extent in brick coordinates.
-struct BrickBox {
-    int32_t x0, y0, z0, nx, ny, nz;
-};
-// Octant words of every brick, or (changed != nullptr) of the bricks a change of occupancy inside
-// `changed` can affect.
-cudaError_t launch_brick_octants(const uint32_t* dir, uint8_t* tmp_x, uint16_t* tmp_y,
-                                 uint32_t* oct, int32_t bx, int32_t by, int32_t bz,
-                                 cudaStream_t stream, const BrickBox* changed = nullptr,
-                                 const uint32_t* occ = nullptr);
-// Occupancy bitmask of the directory (brick_xmask_words() words: one bit per brick, rows along x
-// padded to 32 bits), from which the passes along x read their distances when it is given
-// (`occ` of the distance, octant and long-box launches) instead of scanning the directory; with
-// `changed`, only the rows those passes read after a change inside it.
-cudaError_t launch_brick_xmask(const uint32_t* dir, uint32_t* occ, int32_t bx, int32_t by,
-                               int32_t bz, cudaStream_t stream, const BrickBox* changed = nullptr);
-size_t brick_xmask_words(int32_t bx, int32_t by, int32_t bz);
-
-// Phase 4: Chebyshev distance of every empty brick to the nearest occupied one, into dir.
-// Long forward boxes (3 words per brick, axis-major) from the directory and the octant words, for
-// every brick or (changed != nullptr) for the bricks a change inside `changed` can affect; tmp
-// holds brick_long_scratch_words() words (13 per brick for a full pass, the runs of every brick
-// and a windowed pyramid after a change).
-cudaError_t launch_brick_long(const uint32_t* dir, const uint32_t* oct, uint32_t* tmp,
-                              uint32_t* lng, int32_t bx, int32_t by, int32_t bz,
-                              cudaStream_t stream, const BrickBox* changed = nullptr,
-                              const uint32_t* occ = nullptr);
-size_t brick_long_scratch_words(const BrickBox* changed, int32_t bx, int32_t by, int32_t bz);
-cudaError_t launch_brick_distance(const BuildScratch& s, uint32_t* dir, int32_t bx, int32_t by,
-                                  int32_t bz, cudaStream_t stream,
-                                  const BrickBox* changed = nullptr, const uint32_t* occ = nullptr);
+// Phase 4: octant words, long-box words and the distances below 15 of empty bricks, for every
+// brick or (changed != nullptr) for the bricks a change of occupancy inside `changed` can affect.
+// *s.deep tells afterwards whether a brick of those has no occupied brick within 14: its directory
+// entry then says 15 until launch_brick_distance settles it.
+cudaError_t launch_brick_lattice(uint32_t* dir, uint32_t* oct, uint32_t* lng,
+                                 const LatticeScratch& s, int32_t bx, int32_t by, int32_t bz,
+                                 cudaStream_t stream, const BrickBox* changed = nullptr);
+// Phase 5: distances (up to 31) of the bricks whose octant word is at the cap in all octants, after
+// launch_brick_lattice on the same scratch, or of every empty brick (oct == nullptr: no lattice pass
+// before).  With only_if_deep the kernels return at once unless *s.deep is set (not with `changed`).
+cudaError_t launch_brick_distance(uint32_t* dir, const uint32_t* oct, const LatticeScratch& s,
+                                  int32_t bx, int32_t by, int32_t bz, cudaStream_t stream,
+                                  const BrickBox* changed = nullptr, bool only_if_deep = false);
 
 }  // namespace vt

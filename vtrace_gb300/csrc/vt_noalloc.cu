@@ -5,7 +5,7 @@
 // device and would stall the frame), code recording into a stream that must not see an
 // allocation, or a host that owns a fixed device memory budget.  Those callers pass every input
 // and output buffer themselves; the build's scratch (occupancy words, brick flags, slots, scan
-// partials, distance-transform passes) lives in the file-scope array below instead of a
+// partials, occupancy rows, distance pass) lives in the file-scope array below instead of a
 // cudaMalloc'd buffer.  The kernels are the ones of the allocating build (vt_grid.cu).
 #include <cuda_runtime.h>
 
@@ -18,7 +18,7 @@
 namespace vt {
 
 // Largest grid the scratch covers: 32768 bricks (for example 256^3 voxels).  build_scratch_bytes
-// of that many bricks is 2,425,600 bytes; the array is 2.5 MiB and is resident on every device
+// of 32^3 bricks is 2,360,064 bytes; the array is 2.5 MiB and is resident on every device
 // that loads the library until the process exits.
 constexpr uint64_t kNoAllocMaxBricks = 32768;
 constexpr size_t kNoAllocScratchBytes = 2621440;
@@ -79,21 +79,21 @@ extern "C" int32_t vt_grid_build_u8_noalloc(const uint8_t* d_voxels, const uint3
         ((uintptr_t)d_directory & 3u) || ((uintptr_t)d_palette & 3u))
         return VT_EINVAL;
     if (nx == 0 || ny == 0 || nz == 0 || nx > 65535 || ny > 65535 || nz > 65535) return VT_EINVAL;
-    const uint64_t bricks = (uint64_t)((nx + 7) / 8) * ((ny + 7) / 8) * ((nz + 7) / 8);
-    if (bricks > kNoAllocMaxBricks || build_scratch_bytes(bricks) > kNoAllocScratchBytes)
+    const int32_t bx = (int32_t)((nx + 7) / 8), by = (int32_t)((ny + 7) / 8),
+                  bz = (int32_t)((nz + 7) / 8);
+    const uint64_t bricks = (uint64_t)bx * by * bz;
+    if (bricks > kNoAllocMaxBricks || build_scratch_bytes(bx, by, bz) > kNoAllocScratchBytes)
         return VT_ELIMIT;
     void* scratch = nullptr;
     if (scratch_address(&scratch) != cudaSuccess) return VT_ECUDA;
     cudaStream_t st = (cudaStream_t)stream;
-    const BuildScratch s = carve_build_scratch(scratch, bricks);
-    const int32_t bx = (int32_t)((nx + 7) / 8), by = (int32_t)((ny + 7) / 8),
-                  bz = (int32_t)((nz + 7) / 8);
+    const BuildScratch s = carve_build_scratch(scratch, bx, by, bz);
     if (launch_brick_words(d_voxels, VT_PAYLOAD_U8, d_palette, (int32_t)nx, (int32_t)ny,
                            (int32_t)nz, s, st) != cudaSuccess ||
         launch_brick_scan(s, bricks, st) != cudaSuccess ||
         launch_brick_compact(d_voxels, VT_PAYLOAD_U8, (int32_t)nx, (int32_t)ny, (int32_t)nz, s,
                              d_directory, d_masks, d_payload, st) != cudaSuccess ||
-        launch_brick_distance(s, d_directory, bx, by, bz, st) != cudaSuccess)
+        launch_brick_distance(d_directory, nullptr, s.lattice, bx, by, bz, st) != cudaSuccess)
         return VT_ECUDA;
     noalloc_counts_kernel<<<1, 32, 0, st>>>(s.flags, s.offsets, bricks, s.occupied, d_counts);
     return cudaGetLastError() == cudaSuccess ? VT_OK : VT_ECUDA;

@@ -13,9 +13,9 @@
 //      that became occupied;
 //   4. the new words and payloads are scattered into their slots and the directory entries
 //      rewritten;
-//   5. the Chebyshev distance field, the octant forward distances and the long forward boxes are
-//      recomputed for the bricks within their caps (31, 15 and 15 bricks) of the affected ones:
-//      a change cannot reach farther, and each pass reads the previous one only that far.
+//   5. the octant forward distances, the long forward boxes and the Chebyshev distances are
+//      recomputed for the bricks within 14 bricks of the affected ones (distances above 14, in grids
+//      that have any, within 31): a change cannot reach farther.
 //
 // The grid afterwards traverses exactly as a grid built from the updated dense array (same
 // occupancy, payload, distances and octant words; only slot numbers may differ).
@@ -189,17 +189,14 @@ extern "C" int32_t vt_grid_update(int32_t grid, const void* voxels, uint32_t ord
     const uint64_t K = (uint64_t)u.kx * u.ky * u.kz;
     const size_t box = (size_t)w * h * d * elem;
     auto al = [](size_t v) { return (v + 255) / 256 * 256; };
-    // scratch: box (x2 for reordering), words, payloads, flags, old entries, slots, delta,
-    // distance and octant temporaries
+    // scratch: box (x2 for reordering), words, payloads, flags, old entries, slots, delta, lattice
+    // passes
     const size_t o_box = 0, o_box2 = al(box), o_words = o_box2 + (order == VT_ORDER_Z_FASTEST ? al(box) : 0);
     const size_t o_pay = o_words + al(K * 64), o_flags = o_pay + al(K * 512 * elem);
     const size_t o_old = o_flags + al(K * 4), o_slots = o_old + al(K * 4), o_delta = o_slots + al(K * 4);
-    const size_t o_da = o_delta + 256, o_db = o_da + al(g->bricks), o_ty = o_db + al(g->bricks);
-    const size_t o_run = o_ty + al(g->bricks * 2);
+    const int32_t bx = (int32_t)g->bx, by = (int32_t)g->by, bz = (int32_t)g->bz;
     const BrickBox changed = {u.bx0, u.by0, u.bz0, u.kx, u.ky, u.kz};
-    const size_t o_occ = o_run + al(4 * brick_long_scratch_words(&changed, (int32_t)g->bx,
-                                                                  (int32_t)g->by, (int32_t)g->bz));
-    const size_t total = o_occ + al(4 * brick_xmask_words((int32_t)g->bx, (int32_t)g->by, (int32_t)g->bz));
+    const size_t o_lat = o_delta + 256, total = o_lat + lattice_scratch_bytes(bx, by, bz);
     char* scr = nullptr;
     cudaError_t e = cudaMallocAsync((void**)&scr, total, st);
     if (e != cudaSuccess) return cuda_fail(e, "vt_grid_update: scratch");
@@ -268,24 +265,19 @@ extern "C" int32_t vt_grid_update(int32_t grid, const void* voxels, uint32_t ord
                 v2, u, (const uint64_t*)(scr + o_words), (const uint32_t*)(scr + o_pay),
                 (const uint32_t*)(scr + o_slots), g->dir, g->masks, (uint32_t*)g->payload);
         e = cudaGetLastError();
-        // 5. distances and octant words over the whole directory
-        BuildScratch bs;
-        bs.dist_a = (uint8_t*)(scr + o_da);
-        bs.dist_b = (uint8_t*)(scr + o_db);
-        uint32_t* occ = (uint32_t*)(scr + o_occ);
-        if (e == cudaSuccess)
-            e = launch_brick_xmask(g->dir, occ, (int32_t)g->bx, (int32_t)g->by, (int32_t)g->bz, st,
-                                   &changed);
-        if (e == cudaSuccess)
-            e = launch_brick_distance(bs, g->dir, (int32_t)g->bx, (int32_t)g->by, (int32_t)g->bz, st,
-                                      &changed, occ);
-        if (e == cudaSuccess)
-            e = launch_brick_octants(g->dir, (uint8_t*)(scr + o_da), (uint16_t*)(scr + o_ty), g->oct,
-                                     (int32_t)g->bx, (int32_t)g->by, (int32_t)g->bz, st, &changed, occ);
-        if (e == cudaSuccess)
-            e = launch_brick_long(g->dir, g->oct, (uint32_t*)(scr + o_run), g->lng, (int32_t)g->bx,
-                                  (int32_t)g->by, (int32_t)g->bz, st, &changed, occ);
+        // 5. octant words, long boxes and distances around the change; the distance passes only in
+        // grids that have, or now get, bricks far from all occupied ones
+        const LatticeScratch ls = carve_lattice_scratch(scr + o_lat, bx, by, bz);
+        uint32_t deep = 0;
+        if (e == cudaSuccess) e = launch_brick_lattice(g->dir, g->oct, g->lng, ls, bx, by, bz, st, &changed);
+        if (e == cudaSuccess && g->deep) e = launch_brick_distance(g->dir, g->oct, ls, bx, by, bz, st, &changed);
+        if (e == cudaSuccess && !g->deep) e = cudaMemcpyAsync(&deep, ls.deep, 4, cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        if (e == cudaSuccess && deep) {
+            g->deep = true;
+            e = launch_brick_distance(g->dir, g->oct, ls, bx, by, bz, st, &changed);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        }
         if (e != cudaSuccess) { rc = cuda_fail(e, "vt_grid_update: scatter"); break; }
         uint64_t nonempty = 0;
         for (uint64_t k = 0; k < K; ++k) {
