@@ -40,9 +40,9 @@ __device__ __forceinline__ bool brick_empty(uint32_t e) { return (e & kEmptyBit)
 
 struct GridView {
     const uint32_t* dir;
-    const uint32_t* oct;  // forward distances per ray octant (4 bits x 8), or nullptr
+    const uint32_t* oct;  // forward distances per ray octant (4 bits x 8)
     const uint32_t* lng;  // long forward boxes: 3 words per brick, axis-major (lng[a * bricks +
-                          // brick], 4 bits x 8 octants), or nullptr
+                          // brick], 4 bits x 8 octants)
     const uint64_t* masks;
     const uint8_t* payload8;    // VT_PAYLOAD_U8
     const uint32_t* payload32;  // VT_PAYLOAD_RGBA8
@@ -233,21 +233,6 @@ __device__ __forceinline__ void dda_literal(const GridView& g, int32_t vx, int32
         ++steps;                                                             \
     }
 
-// VT_DDA_STEP on brick-local voxel coordinates (lx, ly, lz).
-#define VT_DDA_STEP_LOCAL                                                    \
-    {                                                                        \
-        const float mn = fminf(fminf(sx, sy), sz);                          \
-        mx = sx == mn;                                                       \
-        my = sy == mn;                                                       \
-        mz = sz == mn;                                                       \
-        if (mx) sx = __fadd_rn(sx, dlx);                                     \
-        if (my) sy = __fadd_rn(sy, dly);                                     \
-        if (mz) sz = __fadd_rn(sz, dlz);                                     \
-        if (mx) lx += stx;                                                   \
-        if (my) ly += sty;                                                   \
-        if (mz) lz += stz;                                                   \
-    }
-
 // The reference DDA (trace.frag:68-87) from grid-space point (px,py,pz) along (dx,dy,dz).
 //
 // Same voxel sequence, step count and hit as the literal loop; the work is organised by brick:
@@ -324,7 +309,7 @@ __device__ __forceinline__ void dda(const GridView& g, float px, float py, float
 // recurrence for one axis, trace.frag:84).  Every addition is the same operation on the running
 // value, so only their count matters: the low three bits of k as predicated groups of 1, 2 and 4,
 // then groups of 8 (the warp runs the loop as often as its longest chain needs; 8% faster frames
-// than one loop in groups of 4 with a remainder loop).  k >= 0.
+// than one loop in groups of 4 with a remainder loop).  k >= 0 (a negative k gives a value of no use).
 __device__ __forceinline__ float add_chain(float s, float d, int32_t k) {
     if (k & 1) s = __fadd_rn(s, d);
     if (k & 2) {
@@ -351,70 +336,87 @@ __device__ __forceinline__ float add_chain(float s, float d, int32_t k) {
     return s;
 }
 
-// Number of an axis's events S(k) <= t_star among k < n_exit, with S(k) evaluated exactly; the
-// axis is known not to reach its exit (S(n_exit - 1) > t_star).  Starts from the estimate
-// floor((t_star - s) / delta) and settles it with exact additions and comparisons.
-__device__ __forceinline__ void advance_axis(float& s, int32_t& v, float delta, int32_t st,
-                                             int32_t n_exit, float t_star, bool& stepped_last) {
-    if (s > t_star) {  // also every axis with no step: its side distance is +inf
-        stepped_last = false;
-        return;
-    }
-    // t_star - s >= 0, and S(n_exit - 1) > t_star >= S(0) gives n_exit >= 2: k >= 0 for add_chain
-    int32_t k = min((int32_t)__fdividef(__fsub_rn(t_star, s), delta), n_exit - 2);
-    float x = add_chain(s, delta, k);  // S(k)
-    if (x > t_star) {                  // the estimate overshot: walk up from S(0)
-        k = 0;
-        x = s;
-    }
-    float y = __fadd_rn(x, delta);  // S(k + 1)
-    while (y <= t_star && k + 1 < n_exit) {
-        x = y;
-        y = __fadd_rn(y, delta);
-        ++k;
-    }
-    s = y;
-    v += st * (k + 1);
-    stepped_last = x == t_star;
+// State of the skipping traversal.
+struct SkipRay {
+    float sx, sy, sz, dlx, dly, dlz;
+    float rl;            // about 1 / length of the direction: |d_a| rl is about 1 / delta_a
+    int32_t vx, vy, vz, stx, sty, stz;
+    uint32_t oshift;     // nibble of the ray's octant in the octant and long-box words
+    int32_t dom;         // dominant axis of the direction
+};
+
+// Set-up past dda_setup_axis.
+__device__ __forceinline__ void skip_setup(const float d[3], float len, SkipRay& R) {
+    R.oshift = (R.stx < 0 ? 4u : 0u) | (R.sty < 0 ? 8u : 0u) | (R.stz < 0 ? 16u : 0u);
+    R.rl = __frcp_rn(len);
+    // largest |component|, ties to the lower axis
+    const float ax = fabsf(d[0]), ay = fabsf(d[1]), az = fabsf(d[2]);
+    R.dom = ax >= ay ? (ax >= az ? 0 : 2) : (ay >= az ? 1 : 2);
 }
 
-// Number of additions for an axis that cannot leave the box first: the estimate
-// floor((amin - s) / delta) of its events after S(0) up to `amin` (the smallest approximate exit),
-// at most n_exit - 2; 0 when its first event is already past it (also the axes with no step, whose
-// side distance is +inf).  Only a speed hint: finish_axis checks the prefix exactly.  A margin of
-// one addition below the estimate (so that the prefix never passes T*) measured 2% slower frames
-// than settling the rare overshoot from S(0).
-__device__ __forceinline__ int32_t prefix_count(float s, float delta, int32_t n_exit, float amin) {
-    if (s > amin) return 0;
-    return max(min((int32_t)__fdividef(__fsub_rn(amin, s), delta), n_exit - 2), 0);
+// Directions the skipping traversal hands to the literal loop: a NaN side distance, or none finite.
+__device__ __forceinline__ bool skip_degenerate(float sx, float sy, float sz) {
+    return isnan(sx) || isnan(sy) || isnan(sz) || !(fminf(fminf(sx, sy), sz) < INFINITY);
 }
 
-// State of one axis after the crossing, from h = S(k) (its one chain): an axis whose chain ends at
-// or before t_star walks up exactly to its last event at or before t_star; a candidate that leaves
-// first (h = S(N - 1) = t_star, k = N - 1) stops at once and steps out of the box.  A chain past
-// t_star with k = 0 means no event in the crossing (also the axes with no step); with k > 0 it is
-// a candidate that does not leave first, or a prefix past t_star (an event of this axis between
-// T* and amin, or the estimate's rounding), settled from S(0) by advance_axis.  One path for the
-// leaving and the staying axes, so lanes of a warp that leave along different axes do not diverge
-// here (3% faster frames than a separate exit step for the candidates).
-__device__ __forceinline__ void finish_axis(float& s, int32_t& v, float h, int32_t k, float delta,
-                                            int32_t st, int32_t n_exit, float t_star,
-                                            bool& stepped_last) {
-    if (h <= t_star) {
-        float x = h, y = __fadd_rn(h, delta);
-        while (y <= t_star && k + 1 < n_exit) {
-            x = y;
-            y = __fadd_rn(y, delta);
-            ++k;
+__device__ __forceinline__ uint32_t skip_brick(const GridView& g, const SkipRay& R) {
+    // fewer than 2^31 bricks (vt_grid_create checks): the index fits 32 bits
+    return (uint32_t)(R.vx >> 3) + (uint32_t)g.bx * ((uint32_t)(R.vy >> 3) + (uint32_t)g.by * (uint32_t)(R.vz >> 3));
+}
+
+// One iteration of trace.frag:83-86 on the coordinates (x, y, z).
+#define VT_SKIP_STEP(x, y, z)                                                \
+    {                                                                        \
+        const float mn = fminf(fminf(sx, sy), sz);                           \
+        mx = sx == mn;                                                       \
+        my = sy == mn;                                                       \
+        mz = sz == mn;                                                       \
+        if (mx) sx = __fadd_rn(sx, dlx);                                     \
+        if (my) sy = __fadd_rn(sy, dly);                                     \
+        if (mz) sz = __fadd_rn(sz, dlz);                                     \
+        if (mx) x += stx;                                                    \
+        if (my) y += sty;                                                    \
+        if (mz) z += stz;                                                    \
+    }
+
+// The rest of the occupied brick in slot `slot`, voxel by voxel: true at a hit.  In brick-local
+// coordinates: the walk ends when one leaves 0..7.  Where a grid face cuts the brick, the voxels
+// past the face have no occupancy bits, so walking on to the brick's face only defers the loop's
+// grid-exit test: the ray misses either way, and a miss keeps none of the walk's state.  Every
+// iteration steps an axis whose step is not 0 (an axis with step 0 has side +inf, the minimum only
+// when all three are, which skip_degenerate excludes), so the brick is left within 22.
+__device__ __forceinline__ bool skip_walk(const GridView& g, SkipRay& R, uint32_t slot, bool& mx,
+                                          bool& my, bool& mz) {
+    float sx = R.sx, sy = R.sy, sz = R.sz;
+    const float dlx = R.dlx, dly = R.dly, dlz = R.dlz;
+    const int32_t stx = R.stx, sty = R.sty, stz = R.stz;
+    const uint64_t* mk = g.masks + (size_t)slot * 8;
+    int32_t lx = R.vx & 7, ly = R.vy & 7, lz = R.vz & 7;
+    bool hit = false;
+    for (;;) {
+        const uint64_t w = __ldg(mk + lz);
+        if ((w >> ((ly << 3) | lx)) & 1ull) {
+            hit = true;
+            break;
         }
-        s = y;
-        v += st * (k + 1);
-        stepped_last = x == t_star;
-    } else if (k == 0) {
-        stepped_last = false;
-    } else {
-        advance_axis(s, v, delta, st, n_exit, t_star, stepped_last);
+        VT_SKIP_STEP(lx, ly, lz)
+        if ((lx | ly | lz) & ~7) break;
     }
+    R.sx = sx;
+    R.sy = sy;
+    R.sz = sz;
+    R.vx = (R.vx & ~7) + lx;
+    R.vy = (R.vy & ~7) + ly;
+    R.vz = (R.vz & ~7) + lz;
+    return hit;
+}
+
+// Moves along one axis from voxel v to the far face of a box reaching r bricks forward (this brick
+// included) in direction st, clipped to the grid's n voxels; at least 1.  With m = -1 for negative
+// directions, v ^ m is v or -1 - v: its low three bits count the voxels of the brick already passed.
+__device__ __forceinline__ int32_t axis_moves(int32_t r, int32_t v, int32_t st, int32_t n) {
+    const int32_t m = st >> 1, t = v ^ m;
+    return min(8 * r - (t & 7), (m ? 0 : n) - t);
 }
 
 // Crossing of an empty box of voxels by the reference DDA, computed per axis.
@@ -425,154 +427,116 @@ __device__ __forceinline__ void finish_axis(float& s, int32_t& v, float h, int32
 // taken n_b = #{k : S_b(k) <= T} steps.  The box is left on the iteration where some axis takes
 // its N_a-th step (N_a = moves to the box face), i.e. at T* = min_a S_a(N_a - 1).  Nothing in
 // the box is occupied, so that iteration is reached without a hit, and the state after it is:
-// side_b = S_b(n_b), voxel_b += step_b * n_b, and the axes that stepped on it are those whose
-// last processed value equals T*.
+// side_b = S_b(n_b), voxel_b += step_b * n_b, and the axes that stepped on it are those whose last
+// processed value equals T*.
 //
-// Only the axes that can leave first need their exit value S_a(N_a - 1) exactly: the
-// approximation s + (N-1) * delta (one fused multiply-add) is within (N + 2) * 2^-24 of the exact
-// chain relative to its magnitude, so any axis whose approximation exceeds the smallest by more
-// than the sum of both bounds (taken 4x larger here) cannot be the minimum.  Each axis runs one
-// chain of additions, so a warp whose lanes leave their boxes along different axes runs three
-// chains rather than one per axis and role (4% faster frames than exit chains followed by
-// separate advances): the candidates to their exit value, the others to the prefix of their
-// estimated count, from which finish_axis walks up once T* is known.  Every value compared
-// is computed with real binary32 additions, so the result is bit-identical to iterating the
-// reference loop.
-__device__ __forceinline__ void cross_region(float& sx, float& sy, float& sz, int32_t& vx,
-                                             int32_t& vy, int32_t& vz, float dlx, float dly,
-                                             float dlz, int32_t stx, int32_t sty, int32_t stz,
-                                             int32_t nxe, int32_t nye, int32_t nze, bool& mx,
-                                             bool& my, bool& mz) {
-    // An axis with no step (N = 0, side and delta +inf) gives NaN here, which fminf and the
-    // candidate comparison below pass over.
-    const float ax = __fmaf_rn(__int2float_rn(nxe - 1), dlx, sx);
-    const float ay = __fmaf_rn(__int2float_rn(nye - 1), dly, sy);
-    const float az = __fmaf_rn(__int2float_rn(nze - 1), dlz, sz);
-    // Candidates: an axis within 2 * amin of the smallest approximation carries at most
-    // (Nmax + 2) * 2 * amin * 2^-24 of error, so (Nmax + 2) * amin * 2^-20 bounds the errors of
-    // both sides of its comparison with the smallest (with the 4x margin above); axes beyond it
-    // cannot leave first.
-    const float amin = fminf(fminf(ax, ay), az);
-    const int32_t nmax = max(max(nxe, nye), nze);
-    const float lim = __fmaf_rn(__int2float_rn(nmax + 2) * 0x1p-20f, amin, amin);
-    const bool cx = ax <= lim;
-    const bool cy = ay <= lim;
-    const bool cz = az <= lim;
-    const int32_t kx = cx ? nxe - 1 : prefix_count(sx, dlx, nxe, amin);
-    const int32_t ky = cy ? nye - 1 : prefix_count(sy, dly, nye, amin);
-    const int32_t kz = cz ? nze - 1 : prefix_count(sz, dlz, nze, amin);
-    VT_PHASE_MARK(__activemask(), VT_PHASE_CROSS_BOX);
-    const float hx = add_chain(sx, dlx, kx);
-    const float hy = add_chain(sy, dly, ky);
-    const float hz = add_chain(sz, dlz, kz);
-    const float ts = fminf(fminf(cx ? hx : INFINITY, cy ? hy : INFINITY), cz ? hz : INFINITY);
-    VT_PHASE_MARK(__activemask(), VT_PHASE_CROSS_CHAINS);
-    finish_axis(sx, vx, hx, kx, dlx, stx, nxe, ts, mx);
-    finish_axis(sy, vy, hy, ky, dly, sty, nye, ts, my);
-    finish_axis(sz, vz, hz, kz, dlz, stz, nze, ts, mz);
-}
-
-// Moves along one axis from voxel v (in brick bi) to the far face of a box reaching r bricks
-// forward (this brick included) in step direction st, clipped to the grid's n voxels: the face is
-// the first voxel past the box for st = +1 (at most n) and the first voxel before it for st = -1
-// (at least -1).  0 for st = 0 (unused).
-__device__ __forceinline__ int32_t axis_moves(int32_t bi, int32_t r, int32_t v, int32_t st,
-                                              int32_t n) {
-    const int32_t neg = st < 0 ? 1 : 0;
-    const int32_t f = min(max(((bi + st * r + neg) << 3) - neg, -1), n);
-    return (f - v) * st;
-}
-
-// Voxel moves to the far face, along each stepping axis, of the empty box the ray crosses next
-// from the empty brick (bxi, byi, bzi).  Three boxes are known empty: the cube of bricks within
-// Chebyshev distance D - 1 (D from the directory entry `e`), which reaches D bricks forward along
-// every stepping direction; the box of K bricks from this brick toward the ray's octant (K from
-// the octant word `ow`); and, when K >= D, the box that is K bricks across and L >= K bricks
-// long along the ray's dominant axis `dom` (L from the long-box word `lw`).  The ray only moves
-// forward, so the crossing uses the forward reach of the chosen box per axis, clipped to the
-// grid.  Axes with no step get 0 (unused by cross_region).
-__device__ __forceinline__ void empty_moves(const GridView& g, uint32_t e, uint32_t ow,
-                                            uint32_t lw, int32_t bxi, int32_t byi, int32_t bzi,
-                                            int32_t vx, int32_t vy, int32_t vz, int32_t stx,
-                                            int32_t sty, int32_t stz, uint32_t oct_shift,
-                                            int32_t dom, int32_t& nxe, int32_t& nye,
-                                            int32_t& nze) {
-    const int32_t D = max((int32_t)(e & 0xFFu), 1);
-    const int32_t K = (int32_t)((ow >> oct_shift) & 15u);
-    const int32_t L = max(K, (int32_t)((lw >> oct_shift) & 15u));
-    // the box across (rk) and along the dominant axis (rl) by selects: lanes choosing the cube and
-    // lanes choosing the long box run the same instructions (1% faster frames than a branch)
+// The common case runs without a branch.  The axis whose approximate exit s + (N - 1) delta is
+// smallest runs its chain of real additions to its exit value, taken for T*.  Every other axis takes
+// n = floor((approximate T* - s) / delta) + 1 steps, at least 0 and at most N - 1 (a NaN quotient, of
+// an axis with no step, gives 0): right if S(n - 1) <= T* < S(n), both exact values.  If that holds for
+// all of them, no other axis leaves the box before T*, which is then the minimum.  Where it does not -
+// an event of another axis within the rounding of T*, a tie of two exits: about one crossing in a
+// thousand - the lane iterates the step itself from S(0) until it leaves the brick.  So the result is
+// bit-identical to iterating, and lanes that leave along different axes run the same instructions.  The quotient comes
+// from |d| / length, once per ray, instead of a division by delta.
+//
+// Bound by instruction issue and the integer/compare pipe: 1080p frame with shadow rays over 1024^3
+// voxels 661 -> 621 us (0.624 -> 0.585 G warp instructions, a third fewer branches) against candidate
+// bounds, per-axis walk-ups and settles behind per-lane branches; 16.8 M cave rays 2.00 -> 1.92 ms.
+__device__ __forceinline__ void skip_cross(const GridView& g, SkipRay& R, const float d[3], uint32_t e,
+                                           uint32_t bidx, bool& mx, bool& my, bool& mz) {
+    // Three boxes are known empty: the cube of bricks within Chebyshev distance D - 1 (D from the
+    // directory entry), which reaches D bricks forward along every axis; the box of K bricks from
+    // this brick toward the ray's octant; and, when K >= D, the box that is K bricks across and
+    // L >= K bricks long along the ray's dominant axis.  Chosen by selects, so that lanes choosing
+    // either run the same instructions.
+    const uint32_t ow = __ldg(g.oct + bidx);
+    const uint32_t lw = __ldg(g.lng + (size_t)R.dom * g.bricks + bidx);
+    const int32_t D = (int32_t)(e & 0xFFu);
+    const int32_t K = (int32_t)((ow >> R.oshift) & 15u), L = (int32_t)((lw >> R.oshift) & 15u);
     const bool box = K >= D;
     const int32_t rk = box ? K : D, rl = box ? L : D;
-    const int32_t rx = dom == 0 ? rl : rk;
-    const int32_t ry = dom == 1 ? rl : rk;
-    const int32_t rz = dom == 2 ? rl : rk;
-    nxe = axis_moves(bxi, rx, vx, stx, g.nx);
-    nye = axis_moves(byi, ry, vy, sty, g.ny);
-    nze = axis_moves(bzi, rz, vz, stz, g.nz);
-}
-
-// Dominant axis of a direction (largest |component|; ties to the lower axis).
-__device__ __forceinline__ int32_t dominant_axis(float dx, float dy, float dz) {
-    const float ax = fabsf(dx), ay = fabsf(dy), az = fabsf(dz);
-    return ax >= ay ? (ax >= az ? 0 : 2) : (ay >= az ? 1 : 2);
-}
-
-// The long-box words of the ray's dominant axis, or nullptr.
-__device__ __forceinline__ const uint32_t* long_words(const GridView& g, int32_t dom) {
-    return g.lng ? g.lng + (size_t)dom * g.bricks : nullptr;
-}
-
-// The octant word of brick `bidx`; 0 (no forward boxes) for a grid built without octant words.
-// Loaded together with the directory entry, before the entry is tested, so that both loads are in
-// flight at once.
-__device__ __forceinline__ uint32_t octant_word(const GridView& g, uint32_t bidx) {
-    return g.oct ? __ldg(g.oct + bidx) : 0u;
-}
-
-__device__ __forceinline__ uint32_t octant_shift(int32_t stx, int32_t sty, int32_t stz) {
-    return 4u * ((stx < 0 ? 1u : 0u) | (sty < 0 ? 2u : 0u) | (stz < 0 ? 4u : 0u));
+    const int32_t nx = axis_moves(R.dom == 0 ? rl : rk, R.vx, R.stx, g.nx);
+    const int32_t ny = axis_moves(R.dom == 1 ? rl : rk, R.vy, R.sty, g.ny);
+    const int32_t nz = axis_moves(R.dom == 2 ? rl : rk, R.vz, R.stz, g.nz);
+    const int32_t stx = R.stx, sty = R.sty, stz = R.stz;
+    float sx = R.sx, sy = R.sy, sz = R.sz;
+    const float dlx = R.dlx, dly = R.dly, dlz = R.dlz;
+    // an axis with no step (side and delta +inf) gives +inf or NaN, which the minimum passes over
+    const float ax = __fmaf_rn(__int2float_rn(nx - 1), dlx, sx);
+    const float ay = __fmaf_rn(__int2float_rn(ny - 1), dly, sy);
+    const float az = __fmaf_rn(__int2float_rn(nz - 1), dlz, sz);
+    const float amin = fminf(fminf(ax, ay), az);
+    const bool cx = ax == amin, cy = !cx && ay == amin, cz = !cx && !cy;
+    const uint32_t ix = cx ? (uint32_t)nx : min(__float2uint_rz(__fmaf_rn(amin - sx, fabsf(d[0]) * R.rl, 1.0f)), (uint32_t)(nx - 1));
+    const uint32_t iy = cy ? (uint32_t)ny : min(__float2uint_rz(__fmaf_rn(amin - sy, fabsf(d[1]) * R.rl, 1.0f)), (uint32_t)(ny - 1));
+    const uint32_t iz = cz ? (uint32_t)nz : min(__float2uint_rz(__fmaf_rn(amin - sz, fabsf(d[2]) * R.rl, 1.0f)), (uint32_t)(nz - 1));
+    VT_PHASE_MARK(__activemask(), VT_PHASE_CROSS_BOX);
+    // S(n - 1); not used where n = 0
+    const float hx = add_chain(sx, dlx, (int32_t)ix - 1);
+    const float hy = add_chain(sy, dly, (int32_t)iy - 1);
+    const float hz = add_chain(sz, dlz, (int32_t)iz - 1);
+    const float ts = cx ? hx : (cy ? hy : hz);
+    VT_PHASE_MARK(__activemask(), VT_PHASE_CROSS_CHAINS);
+    const bool tx = ix != 0u, ty = iy != 0u, tz = iz != 0u;
+    const float ux = tx ? __fadd_rn(hx, dlx) : sx;  // S(n)
+    const float uy = ty ? __fadd_rn(hy, dly) : sy;
+    const float uz = tz ? __fadd_rn(hz, dlz) : sz;
+    if (ux <= ts || uy <= ts || uz <= ts || (tx && hx > ts) || (ty && hy > ts) || (tz && hz > ts)) {
+        const int32_t vx = R.vx, vy = R.vy, vz = R.vz;
+        do {
+            VT_SKIP_STEP(R.vx, R.vy, R.vz)
+        } while ((((R.vx ^ vx) | (R.vy ^ vy) | (R.vz ^ vz)) & ~7) == 0);
+    } else {
+        sx = ux;
+        sy = uy;
+        sz = uz;
+        R.vx += stx * (int32_t)ix;
+        R.vy += sty * (int32_t)iy;
+        R.vz += stz * (int32_t)iz;
+        mx = tx && hx == ts;
+        my = ty && hy == ts;
+        mz = tz && hz == ts;
+    }
+    R.sx = sx;
+    R.sy = sy;
+    R.sz = sz;
 }
 
 // Same result as dda() (hit, voxel, slot, final mask), organised for speed: occupied bricks are
-// walked voxel by voxel against their occupancy bits; from an empty brick the ray crosses the
-// empty box of empty_moves() in one cross_region().  The step count and tie flag of the literal
+// walked voxel by voxel against their occupancy bits (skip_walk); from an empty brick the ray
+// crosses a box of empty bricks in one skip_cross().  The step count and tie flag of the literal
 // loop are not tracked here (the counting kernels use dda()).
 __device__ __forceinline__ void dda_skip(const GridView& g, float px, float py, float pz,
                                          float dx, float dy, float dz, DDAResult& r) {
     const float len = __fsqrt_rn(
         __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)));
-    int32_t vx, vy, vz, stx, sty, stz;
-    float dlx, dly, dlz, sx, sy, sz;
-    dda_setup_axis(px, dx, g.nx, len, vx, stx, dlx, sx);
-    dda_setup_axis(py, dy, g.ny, len, vy, sty, dly, sy);
-    dda_setup_axis(pz, dz, g.nz, len, vz, stz, dlz, sz);
-    if (isnan(sx) || isnan(sy) || isnan(sz)) {
+    SkipRay R;
+    dda_setup_axis(px, dx, g.nx, len, R.vx, R.stx, R.dlx, R.sx);
+    dda_setup_axis(py, dy, g.ny, len, R.vy, R.sty, R.dly, R.sy);
+    dda_setup_axis(pz, dz, g.nz, len, R.vz, R.stz, R.dlz, R.sz);
+    if (skip_degenerate(R.sx, R.sy, R.sz)) {
         Tally<false> tl;
-        dda_literal<false>(g, vx, vy, vz, stx, sty, stz, dlx, dly, dlz, sx, sy, sz, r, tl);
+        dda_literal<false>(g, R.vx, R.vy, R.vz, R.stx, R.sty, R.stz, R.dlx, R.dly, R.dlz, R.sx, R.sy,
+                           R.sz, r, tl);
         return;
     }
-    const uint32_t max_steps = g.max_steps;
-    const uint32_t oshift = octant_shift(stx, sty, stz);
-    const int32_t dom = dominant_axis(dx, dy, dz);
-    const uint32_t* lp = long_words(g, dom);
-    uint32_t steps = 0, slot = kEmptyBit;  // steps: counted by VT_DDA_STEP, not used here
+    const float d[3] = {dx, dy, dz};
+    skip_setup(d, len, R);
+    uint32_t slot = kEmptyBit;
     bool mx = false, my = false, mz = false, hit = false;
-    // guard: passes that run a unit; each advances at least one axis, monotonically, inside the
-    // grid.  pend_w / pend_c: lanes needing a walk / a crossing were passed over last pass.
-    int32_t guard = g.nx + g.ny + g.nz + 2;
+    // Ends: every pass runs a unit on at least one of the lanes in the loop together, and a unit
+    // advances at least one axis, monotonically, toward the grid's face.
+    // pend_w / pend_c: lanes needing a walk / a crossing were passed over last pass.
     bool pend_w = false, pend_c = false;
-    while (grid_inside(g, vx, vy, vz) && guard > 0) {
-        const int32_t bxi = vx >> 3, byi = vy >> 3, bzi = vz >> 3;
-        // fewer than 2^31 bricks (vt_grid_create checks): the index fits 32 bits
-        const uint32_t bidx = (uint32_t)bxi + (uint32_t)g.bx * ((uint32_t)byi + (uint32_t)g.by * (uint32_t)bzi);
+    while (grid_inside(g, R.vx, R.vy, R.vz)) {
+        const uint32_t bidx = skip_brick(g, R);
         const uint32_t e = __ldg(g.dir + bidx);
         {
             // One kind of unit per pass among the lanes running this loop together: the kind
             // more of them need (walk or crossing) runs while the others wait, and a kind passed
             // over runs next, so a warp issues one kind's instructions per pass instead of both
-            // (5% faster frames).  Every pass runs a unit on at least one of these lanes, so the
-            // waits end.
+            // (5% faster frames).
             const bool walk = !brick_empty(e);
             const uint32_t act = __activemask();
             VT_PHASE_MARK(act, VT_PHASE_LOOP);
@@ -584,47 +548,20 @@ __device__ __forceinline__ void dda_skip(const GridView& g, float px, float py, 
             VT_PHASE_PASS(act, run_walk);
             if (walk != run_walk) continue;
         }
-        --guard;
         if (!brick_empty(e)) {
             slot = e;
-            const uint64_t* mk = g.masks + (size_t)slot * 8;
-            // Brick-local coordinates; the walk ends when one leaves 0..7.  Where a grid face cuts
-            // the brick, the voxels past the face have no occupancy bits, so walking on to the
-            // brick's face only defers the loop's grid-exit test: the ray misses either way, and a
-            // miss keeps none of the walk's state.  Ends: with no side distance NaN, every
-            // iteration steps an axis whose step is not 0 (an axis with step 0 has side +inf, the
-            // minimum only when all three are), so the brick is left within 22 iterations.
-            int32_t lx = vx & 7, ly = vy & 7, lz = vz & 7;
-            for (;;) {
-                const uint64_t w = __ldg(mk + lz);
-                if ((w >> ((ly << 3) | lx)) & 1ull) {
-                    hit = true;
-                    break;
-                }
-                VT_DDA_STEP_LOCAL
-                if ((lx | ly | lz) & ~7) break;
-            }
-            vx = (bxi << 3) + lx;
-            vy = (byi << 3) + ly;
-            vz = (bzi << 3) + lz;
+            hit = skip_walk(g, R, e, mx, my, mz);
             VT_PHASE_MARK(__activemask(), VT_PHASE_WALK);
             if (hit) break;
         } else {
-            const uint32_t ow = octant_word(g, bidx);
-            const uint32_t lw = lp ? __ldg(lp + bidx) : 0u;
-            int32_t nxe, nye, nze;
-            empty_moves(g, e, ow, lw, bxi, byi, bzi, vx, vy, vz, stx, sty, stz, oshift, dom, nxe,
-                        nye, nze);
-            cross_region(sx, sy, sz, vx, vy, vz, dlx, dly, dlz, stx, sty, stz, nxe, nye, nze, mx,
-                         my, mz);
+            skip_cross(g, R, d, e, bidx, mx, my, mz);
             VT_PHASE_MARK(__activemask(), VT_PHASE_CROSS_FINISH);
         }
     }
-    (void)max_steps;
-    r.vx = vx;
-    r.vy = vy;
-    r.vz = vz;
-    r.steps = steps;
+    r.vx = R.vx;
+    r.vy = R.vy;
+    r.vz = R.vz;
+    r.steps = 0;
     r.slot = slot;
     r.last = (mx ? 1 : 0) | (my ? 2 : 0) | (mz ? 4 : 0);
     r.hit = hit;

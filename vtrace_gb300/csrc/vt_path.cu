@@ -523,8 +523,8 @@ __device__ __forceinline__ void bounce_dir(const PathParams& P, uint32_t px, uin
 // launch shape: the rays of a warp start together and stay coherent): camera ray, traversal,
 // shading, the sun ray traced in the same thread (as the render kernel traces its shadow rays),
 // and the bounce ray appended to the queue of vertex 1.
-// Held to 48 registers: ten blocks per SM (0.4% shorter path frames than nine at 54).
-__global__ void __launch_bounds__(128, 10) wave_primary_kernel(
+// Eight blocks per SM at up to 64 registers (see trace_rays_persistent_kernel).
+__global__ void __launch_bounds__(128, 8) wave_primary_kernel(
     GridView g, vt_camera cam, PathParams P, uint32_t s0, uint32_t sn, uint32_t tiles_x,
     uint64_t total, vt_ray* __restrict__ nq, uint32_t* __restrict__ nqid,
     unsigned int* __restrict__ nqn, WaveState* __restrict__ st, float4* __restrict__ samples,

@@ -70,9 +70,9 @@ __device__ __forceinline__ void phase_kind(uint32_t mask, int kind) {
 
 namespace vt {
 
-// render_kernel<false> with its default shape: 8 x 4-pixel warp tiles, 2 x 2 warps per block, ten
-// blocks per SM as the render kernel's 48 registers allow.
-__global__ void __launch_bounds__(kPhaseWarps * 32, 10) render_phase_kernel(
+// render_kernel<false> with its default shape: 8 x 4-pixel warp tiles, 2 x 2 warps per block, eight
+// blocks per SM as the render kernel has.
+__global__ void __launch_bounds__(kPhaseWarps * 32, 8) render_phase_kernel(
     GridView g, vt_camera cam, LightView light, uint4* __restrict__ out,
     unsigned long long* __restrict__ totals) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;

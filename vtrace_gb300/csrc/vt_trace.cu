@@ -43,9 +43,11 @@ static RenderShape render_shape(const TraceTuning* tune) {
     return best;
 }
 
-// Rows row0 .. row1 - 1 of the image (a band; the whole image when 0 .. height).
-template <bool STATS>
-__global__ void __launch_bounds__(256) render_kernel(GridView g, vt_camera cam, LightView light,
+// Rows row0 .. row1 - 1 of the image (a band; the whole image when 0 .. height).  Bounded for eight
+// blocks of 128 threads (53 registers, so that nine are resident): the 1080p frame with shadow rays
+// takes 621 us, bounded for nine 627, for ten (48 registers, 4 bytes of spills) 628.
+template <bool STATS, int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == 128 ? 8 : 4) render_kernel(GridView g, vt_camera cam, LightView light,
                                                      uint4* __restrict__ out,
                                                      Counters* __restrict__ counters,
                                                      uint32_t row0, uint32_t row1,
@@ -92,9 +94,11 @@ cudaError_t launch_render(const GridView& g, const vt_camera& cam, const LightVi
     dim3 grid((cam.width + sh.block_w() - 1) / sh.block_w(),
               (row1 - row0 + sh.block_h() - 1) / sh.block_h());
     if (counters)
-        render_kernel<true><<<grid, threads, 0, stream>>>(g, cam, light, out, counters, row0, row1, sh);
+        render_kernel<true, 256><<<grid, threads, 0, stream>>>(g, cam, light, out, counters, row0, row1, sh);
+    else if (threads <= 128)
+        render_kernel<false, 128><<<grid, threads, 0, stream>>>(g, cam, light, out, nullptr, row0, row1, sh);
     else
-        render_kernel<false><<<grid, threads, 0, stream>>>(g, cam, light, out, nullptr, row0, row1, sh);
+        render_kernel<false, 256><<<grid, threads, 0, stream>>>(g, cam, light, out, nullptr, row0, row1, sh);
     return cudaGetLastError();
 }
 
@@ -239,11 +243,11 @@ __global__ void __launch_bounds__(256) render_persistent_kernel(
 constexpr int kUnitWait = 4;
 
 // n_dev: nullptr, or the device-side ray count (at most n), read at the start (ray queues whose
-// length the host does not know).  Held to 48 registers (a few bytes of spills) so that five
-// blocks fit an SM instead of four: the short rays of dense grids wait on their mask and directory
-// loads, and the fifth block hides more of that (16.7M cave rays 2.29 -> 2.17 ms; six blocks at
-// 40 registers spill more and lose).
-__global__ void __launch_bounds__(256, 5) trace_rays_persistent_kernel(
+// length the host does not know).  Blocks of 128 threads, nine per SM at 56 registers: 16.7M cave
+// rays 1.899 ms, path-traced 1080p frame 4.28 ms, against 1.905 and 4.32 ms for five blocks of 256 at
+// 48 registers (a few bytes of spills) and 2.00 ms for four at 64 registers.
+constexpr int kRayThreads = 128;
+__global__ void __launch_bounds__(kRayThreads, 9) trace_rays_persistent_kernel(
     GridView g, const float2* __restrict__ rays, uint64_t n, uint4* __restrict__ out,
     unsigned long long* __restrict__ counter, uint32_t refill_min,
     const unsigned int* __restrict__ n_dev) {
@@ -304,9 +308,9 @@ __global__ void __launch_bounds__(256, 5) trace_rays_persistent_kernel(
     }
 }
 
-static int resident_blocks(const void* kernel) {
+static int resident_blocks(const void* kernel, int threads = 256) {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, 256, 0) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, 0) != cudaSuccess) {
         cudaGetLastError();
         n = 1;
     }
@@ -335,13 +339,14 @@ cudaError_t launch_trace_rays_persistent(const GridView& g, const vt_ray* rays, 
                                          const TraceTuning& tune, int sm_count,
                                          cudaStream_t stream, const unsigned int* n_dev) {
     if (n == 0) return cudaSuccess;
-    static int per_sm = resident_blocks((const void*)trace_rays_persistent_kernel);
-    const int bps = tune.blocks_per_sm > 0 ? min(tune.blocks_per_sm, per_sm) : per_sm;
-    const uint64_t need = (n + 255) / 256;
+    static int per_sm = resident_blocks((const void*)trace_rays_persistent_kernel, kRayThreads);
+    // the tuning counts blocks of 256 threads
+    const int bps = tune.blocks_per_sm > 0 ? min(tune.blocks_per_sm * (256 / kRayThreads), per_sm) : per_sm;
+    const uint64_t need = (n + kRayThreads - 1) / kRayThreads;
     const unsigned blocks = (unsigned)std::min<uint64_t>((uint64_t)sm_count * bps, need);
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), stream);
     if (e != cudaSuccess) return e;
-    trace_rays_persistent_kernel<<<blocks, 256, 0, stream>>>(
+    trace_rays_persistent_kernel<<<blocks, kRayThreads, 0, stream>>>(
         g, reinterpret_cast<const float2*>(rays), n, out, counter, tune.refill_min, n_dev);
     return cudaGetLastError();
 }
