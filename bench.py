@@ -79,13 +79,13 @@ def parse_args():
 def path_launches(tuning, spp, bounces, pixels):
     """Kernels one vt_path_trace launches under `tuning`, per frame.
 
-    Wavefront form, per chunk of samples (up to 16 spp, 16M paths): the vertex-0 kernel, then
-    per later vertex the path-ray trace, the shading, the sun-ray trace and the sun light, then
-    the resolve.  Persistent form: the path kernel and the resolve
+    Wavefront form with a sun, per chunk of samples (up to 16 spp, 16M paths): the vertex-0 kernel,
+    then per later vertex one trace (bounce rays and the sun rays of the vertex before) and the
+    shading, the last vertex's sun rays and their light, then the resolve.  Persistent form: the path kernel and the resolve
     per chunk (up to 16 spp, 64M samples).  Per-pixel form: one kernel."""
     if tuning["wavefront"]:
         sn = max(1, min(spp, 16, (16 << 20) // pixels))
-        return -(-spp // sn) * (2 + 4 * bounces)
+        return -(-spp // sn) * (2 + 2 * bounces + (2 if bounces else 0))
     if tuning["persistent"]:
         sn = max(1, min(spp, 16, (64 << 20) // pixels))
         return -(-spp // sn) * 2

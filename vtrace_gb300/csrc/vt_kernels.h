@@ -37,8 +37,7 @@ cudaError_t launch_render_persistent(const GridView& g, const vt_camera& cam,
 cudaError_t launch_trace_rays_persistent(const GridView& g, const vt_ray* rays, uint64_t n,
                                          uint4* out, unsigned long long* counter,
                                          const TraceTuning& tune, int sm_count,
-                                         cudaStream_t stream,
-                                         const unsigned int* n_dev = nullptr);
+                                         cudaStream_t stream);
 
 // `tune` selects the warp tile and block shape (nullptr: 8 x 4 pixels per warp, 4 warps).
 cudaError_t launch_render(const GridView& g, const vt_camera& cam, const LightView& light,
@@ -49,10 +48,8 @@ cudaError_t launch_render(const GridView& g, const vt_camera& cam, const LightVi
 unsigned phase_profile_words();
 cudaError_t launch_render_phases(const GridView& g, const vt_camera& cam, const LightView& light,
                                  uint4* out, unsigned long long* totals, cudaStream_t stream);
-// n_dev as for launch_trace_rays_persistent: the device-side ray count (at most n), or nullptr.
 cudaError_t launch_trace_rays(const GridView& g, const vt_ray* rays, uint64_t n, uint4* out,
-                              Counters* counters, cudaStream_t stream,
-                              const unsigned int* n_dev = nullptr);
+                              Counters* counters, cudaStream_t stream);
 
 // A box of bricks: origin and extent in brick coordinates.
 struct BrickBox {

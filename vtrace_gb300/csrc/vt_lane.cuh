@@ -115,4 +115,67 @@ __device__ __forceinline__ uint64_t warp_fetch(unsigned long long* counter, uint
     return base;
 }
 
+// Passes a unit kind may be passed over in trace_persistent.
+constexpr int kUnitWait = 4;
+
+// Resident-warp tracing of `n` rays: a ray per lane, lanes whose rays ended refilled from `counter`
+// once `refill_min` of the warp's lanes are idle.  `io.load(item, o, d)` gives an item's ray and
+// `io.store(item, R, status)` takes its result; every lane of the warp calls this together.
+template <class Io>
+__device__ __forceinline__ void trace_persistent(const GridView& g, const Io& io, uint64_t n,
+                                                 unsigned long long* __restrict__ counter,
+                                                 uint32_t refill_min) {
+    const uint32_t lane = threadIdx.x & 31u;
+    LaneRay R;
+    bool busy = false;
+    typename Io::Index idx = 0;
+    bool more = true;
+    int wait_w = 0, wait_c = 0;  // warp-uniform: iterations a unit kind was passed over
+    for (;;) {
+        uint32_t idle = __ballot_sync(0xFFFFFFFFu, !busy);
+        while (more && __popc(idle) >= (int)refill_min) {
+            uint64_t item;
+            const uint64_t base = warp_fetch(counter, idle, lane, item);
+            if (base + __popc(idle) >= n) more = false;
+            if (!busy && item < n) {
+                float o[3], d[3];
+                io.load((typename Io::Index)item, o, d);
+                const int st = ray_begin(g, o, d, R);
+                if (st == kRayRunning) {
+                    busy = true;
+                    idx = (typename Io::Index)item;
+                } else {
+                    io.store((typename Io::Index)item, R, st);
+                }
+            }
+            idle = __ballot_sync(0xFFFFFFFFu, !busy);
+        }
+        if (!more && idle == 0xFFFFFFFFu) break;
+        // One kind of unit per pass: the lanes whose next unit is the more common kind (walk or
+        // crossing) run it, the others wait, unless their kind has already waited kUnitWait
+        // passes.  A warp then issues one kind's instructions per pass instead of both; every
+        // pass with busy lanes runs at least one unit.  2% faster on the 16M incoherent rays.
+        const uint32_t e = busy ? ray_entry(g, R) : kEmptyBit;
+        const bool walk = busy && !brick_empty(e);
+        const uint32_t wb = __ballot_sync(0xFFFFFFFFu, walk);
+        const uint32_t cb = __ballot_sync(0xFFFFFFFFu, busy && !walk);
+        bool run_walk = __popc(wb) >= __popc(cb);
+        if (run_walk ? (cb && wait_c >= kUnitWait) : (wb && wait_w >= kUnitWait)) run_walk = !run_walk;
+        if (run_walk) {
+            wait_w = 0;
+            wait_c = cb ? wait_c + 1 : 0;
+        } else {
+            wait_c = 0;
+            wait_w = wb ? wait_w + 1 : 0;
+        }
+        if (busy && walk == run_walk) {
+            const int st = ray_unit(g, R, e);
+            if (st != kRayRunning) {
+                io.store(idx, R, st);
+                busy = false;
+            }
+        }
+    }
+}
+
 }  // namespace vt

@@ -453,27 +453,26 @@ static cudaError_t launch_path_persistent(const GridView& g, const vt_camera& ca
 
 // ---------------------------------------------------------------------------------------------
 // Wavefront form: the paths of a chunk of samples advance one vertex at a time through ray
-// queues.  Vertex 0 (camera ray, shading, sun ray) runs a thread per path in 8 x 4 pixel tiles;
-// per vertex after that: trace the path rays, shade (sky on a miss; throughput, sun ray and
-// bounce ray otherwise), trace the sun rays and add their light, the two ray queues traced by the
-// persistent ray-buffer kernel.  Queues keep append order, which follows the pixel tiles:
-// neighbouring entries start at neighbouring surface points (bucketing the bounce rays by
-// direction octant and origin cell measured 9% slower in all).  Every path's radiance sees the
-// same operations in the same order as path_pixel; queue order only changes speed.  Queue
-// lengths stay on the device.
+// queues.  Vertex 0 (camera ray, shading, sun ray) runs a thread per path in 8 x 4 pixel tiles.
+// Then, per vertex: one launch of resident warps traces the bounce rays toward it together with the
+// sun rays of the vertex before, and the shading adds the light of those sun rays and makes the
+// vertex's sun and bounce rays (sky on a miss).  The sun rays of the last vertex are traced and added
+// on their own.  Queues keep append order, which follows the pixel tiles: neighbouring entries start
+// at neighbouring surface points (bucketing the bounce rays by direction octant and origin cell
+// measured 9% slower in all).  Every path's radiance sees the same operations in the same order as
+// path_pixel; queue order only changes speed.  Queue lengths stay on the device.
 // ---------------------------------------------------------------------------------------------
 
-struct WaveState {
-    float T[3], L[3], so[3];
-    uint32_t face;
-    uint32_t pad[2];
-};
+// Per path: throughput in xyz and, in w, the face of its last vertex | kSunPending when that
+// vertex's sun ray is queued.  Its radiance so far is its entry of the sample buffer.
+using WaveState = float4;
+constexpr uint32_t kSunPending = 8u;
 
 constexpr uint64_t kWaveChunkPaths = 16u << 20;
 constexpr uint32_t kWaveCounters = 256;  // 2 x 128 queue lengths: max_bounces <= 64
 
 // Appends the lanes with `want` to a queue: one atomic per warp; every lane of the warp calls it.
-__device__ __forceinline__ uint32_t wave_append(unsigned int* count, bool want) {
+__device__ __forceinline__ uint32_t warp_append(unsigned int* count, bool want) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t ballot = __ballot_sync(0xFFFFFFFFu, want);
     if (!ballot) return 0;
@@ -482,6 +481,40 @@ __device__ __forceinline__ uint32_t wave_append(unsigned int* count, bool want) 
     if ((int)lane == leader) base = atomicAdd(count, (unsigned int)__popc(ballot));
     base = __shfl_sync(0xFFFFFFFFu, base, leader);
     return base + __popc(ballot & ((1u << lane) - 1u));
+}
+
+// Places of the block's threads with `want` in two queues: one atomic per block and queue
+// (a queue's length is one address: with an atomic per warp the short shading waited for them; the
+// camera kernel, whose warps end at different times, keeps one per warp, 0.3% faster there).  Every
+// thread of the block calls it; blocks of WARPS warps.
+template <int WARPS>
+__device__ __forceinline__ void block_append(unsigned int* count0, bool want0, uint32_t& at0,
+                                             unsigned int* count1, bool want1, uint32_t& at1) {
+    __shared__ uint32_t base[2][WARPS];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t b0 = __ballot_sync(0xFFFFFFFFu, want0), b1 = __ballot_sync(0xFFFFFFFFu, want1);
+    if (lane == 0) {
+        base[0][warp] = __popc(b0);
+        base[1][warp] = __popc(b1);
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        uint32_t total = 0;
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) {
+            const uint32_t n = base[threadIdx.x][w];
+            base[threadIdx.x][w] = total;
+            total += n;
+        }
+        const uint32_t first = total ? atomicAdd(threadIdx.x ? count1 : count0, total) : 0u;
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) base[threadIdx.x][w] += first;
+    }
+    __syncthreads();
+    const uint32_t below = (1u << lane) - 1u;
+    at0 = base[0][warp] + __popc(b0 & below);
+    at1 = base[1][warp] + __popc(b1 & below);
+    __syncthreads();  // `base` may be written again
 }
 
 __device__ __forceinline__ void wave_path_pixel(uint32_t p, uint32_t sn, uint32_t s0, uint32_t w,
@@ -498,8 +531,9 @@ __device__ __forceinline__ void wave_path_pixel(uint32_t p, uint32_t sn, uint32_
 // path_pixel.
 __device__ __forceinline__ void bounce_dir(const PathParams& P, uint32_t px, uint32_t py,
                                            uint32_t s, uint32_t b, int a, bool npos, float nd[3]) {
-    float n3[3] = {0.0f, 0.0f, 0.0f}, u[3];
-    n3[a] = npos ? 1.0f : -1.0f;
+    float n3[3], u[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) n3[k] = k == a ? (npos ? 1.0f : -1.0f) : 0.0f;
     if (sphere_sample(P.seed, px, py, s, b, u)) {
 #pragma unroll
         for (int k = 0; k < 3; ++k) nd[k] = __fadd_rn(n3[k], u[k]);
@@ -519,11 +553,17 @@ __device__ __forceinline__ void bounce_dir(const PathParams& P, uint32_t px, uin
     }
 }
 
+// n.l of the sun on a face.
+__device__ __forceinline__ float sun_ndl(const PathParams& P, uint32_t face) {
+    const int a = (int)(face - 1) / 2;
+    const float la = a == 0 ? P.sun_dir[0] : (a == 1 ? P.sun_dir[1] : P.sun_dir[2]);
+    return (face & 1u) ? la : -la;
+}
+
 // Vertex 0 of the chunk's paths, one thread per path in 8 x 4 pixel tiles (the render kernel's
 // launch shape: the rays of a warp start together and stay coherent): camera ray, traversal,
 // shading, the sun ray traced in the same thread (as the render kernel traces its shadow rays),
 // and the bounce ray appended to the queue of vertex 1.
-// Eight blocks per SM at up to 64 registers (see trace_rays_persistent_kernel).
 __global__ void __launch_bounds__(128, 8) wave_primary_kernel(
     GridView g, vt_camera cam, PathParams P, uint32_t s0, uint32_t sn, uint32_t tiles_x,
     uint64_t total, vt_ray* __restrict__ nq, uint32_t* __restrict__ nqid,
@@ -568,11 +608,8 @@ __global__ void __launch_bounds__(128, 8) wave_primary_kernel(
             for (int c = 0; c < 3; ++c)
                 T[c] = __fmul_rn(T[c], __fdiv_rn(__uint2float_rn((h.w3 >> (8 * c)) & 0xFFu), 255.0f));
             shadow_origin(h, o, d, so);
-            const int a = (int)(face - 1) / 2;
-            const bool npos = (face & 1u) != 0u;
             if (P.sun_on) {
-                const float la = a == 0 ? P.sun_dir[0] : (a == 1 ? P.sun_dir[1] : P.sun_dir[2]);
-                const float ndl = npos ? la : -la;
+                const float ndl = sun_ndl(P, face);
                 if (ndl > 0.0f) {
                     const HitRec sh = trace_ray<false>(g, so, P.sun_dir, tl);
                     ++nrays;
@@ -585,21 +622,13 @@ __global__ void __launch_bounds__(128, 8) wave_primary_kernel(
             }
             if (P.max_bounces > 0) {
                 bounce = true;
-                bounce_dir(P, px, py, s0 + smp, 0u, a, npos, nd);
+                bounce_dir(P, px, py, s0 + smp, 0u, (int)(face - 1) / 2, (face & 1u) != 0u, nd);
+                st[p] = make_float4(T[0], T[1], T[2], __uint_as_float(face));
             }
         }
-        if (bounce) {
-            WaveState& S = st[p];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                S.T[c] = T[c];
-                S.L[c] = L[c];
-            }
-        } else {
-            samples[p] = make_float4(L[0], L[1], L[2], 0.0f);
-        }
+        samples[p] = make_float4(L[0], L[1], L[2], 0.0f);
     }
-    const uint32_t kb = wave_append(nqn, bounce);
+    const uint32_t kb = warp_append(nqn, bounce);
     if (bounce) {
         nq[kb] = vt_ray{{so[0], so[1], so[2]}, {nd[0], nd[1], nd[2]}};
         nqid[kb] = p;
@@ -610,98 +639,170 @@ __global__ void __launch_bounds__(128, 8) wave_primary_kernel(
     }
 }
 
-// Vertex b of every queued path: its ray ended with record h.
-__global__ void __launch_bounds__(256) wave_shade_kernel(
-    GridView g, PathParams P, uint32_t b, uint32_t s0, uint32_t sn, uint32_t w,
-    const vt_ray* __restrict__ q, const uint32_t* __restrict__ qid,
-    const unsigned int* __restrict__ qn, const uint4* __restrict__ hits,
-    WaveState* __restrict__ st, float4* __restrict__ samples, vt_ray* __restrict__ sq,
-    uint32_t* __restrict__ sid, unsigned int* __restrict__ sqn, vt_ray* __restrict__ nq,
-    uint32_t* __restrict__ nqid, unsigned int* __restrict__ nqn,
-    unsigned long long* __restrict__ rays_out) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t n = *qn;
-    if (rays_out && j == 0) atomicAdd(rays_out, (unsigned long long)n);
-    bool sun = false, bounce = false;
-    uint32_t p = 0;
-    float so[3] = {0.0f, 0.0f, 0.0f}, nd[3] = {0.0f, 0.0f, 0.0f};
-    if (j < n) {
-        p = qid[j];
-        const uint4 hv = hits[j];
-        HitRec h;
-        h.w0 = hv.x;
-        h.w1 = hv.y;
-        h.w2 = hv.z;
-        h.w3 = hv.w;
-        WaveState& S = st[p];
-        const uint32_t flags = h.w1 >> 24;
-        const uint32_t face = flags & VT_FACE_MASK;
-        if (!(flags & VT_HIT_FLAG_HIT) || face == 0) {
-            if (!(flags & VT_HIT_FLAG_HIT)) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) S.L[c] = __fadd_rn(S.L[c], __fmul_rn(S.T[c], P.sky[c]));
-            }
-            samples[p] = make_float4(S.L[0], S.L[1], S.L[2], 0.0f);
+// Bounce rays (items below `nb`: full records) and sun rays (the rest: only whether they are blocked,
+// written at their path).
+struct WaveIo {
+    using Index = uint32_t;
+    const GridView& g;
+    const float2* __restrict__ q;      // bounce rays, 24 bytes each
+    uint4* __restrict__ hits;
+    uint32_t nb;
+    const float* __restrict__ so;      // sun ray origins, three floats each
+    const uint32_t* __restrict__ sid;  // their paths
+    uint8_t* __restrict__ blocked;
+    float sx, sy, sz;
+    __device__ __forceinline__ void load(uint32_t i, float o[3], float d[3]) const {
+        if (i < nb) {
+            const float2 a = __ldg(q + 3 * (size_t)i), b = __ldg(q + 3 * (size_t)i + 1), c = __ldg(q + 3 * (size_t)i + 2);
+            o[0] = a.x;
+            o[1] = a.y;
+            o[2] = b.x;
+            d[0] = b.y;
+            d[1] = c.x;
+            d[2] = c.y;
         } else {
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-                S.T[c] = __fmul_rn(S.T[c], __fdiv_rn(__uint2float_rn((h.w3 >> (8 * c)) & 0xFFu), 255.0f));
-            const vt_ray r = q[j];
-            shadow_origin(h, r.origin, r.dir, so);
-#pragma unroll
-            for (int c = 0; c < 3; ++c) S.so[c] = so[c];
-            S.face = face;
-            const int a = (int)(face - 1) / 2;
-            const bool npos = (face & 1u) != 0u;
-            if (P.sun_on) {
-                const float la = a == 0 ? P.sun_dir[0] : (a == 1 ? P.sun_dir[1] : P.sun_dir[2]);
-                sun = (npos ? la : -la) > 0.0f;
-            }
-            if (b < P.max_bounces) {
-                bounce = true;
-                uint32_t px, py, s;
-                wave_path_pixel(p, sn, s0, w, px, py, s);
-                bounce_dir(P, px, py, s, b, a, npos, nd);
-            } else if (!sun) {
-                samples[p] = make_float4(S.L[0], S.L[1], S.L[2], 0.0f);  // the path ends here
-            }
+            const float* f = so + 3 * (size_t)(i - nb);
+            o[0] = __ldg(f);
+            o[1] = __ldg(f + 1);
+            o[2] = __ldg(f + 2);
+            d[0] = sx;
+            d[1] = sy;
+            d[2] = sz;
         }
     }
-    const uint32_t ks = wave_append(sqn, sun);
-    if (sun) {
-        sq[ks] = vt_ray{{so[0], so[1], so[2]}, {P.sun_dir[0], P.sun_dir[1], P.sun_dir[2]}};
-        sid[ks] = p;
+    __device__ __forceinline__ void store(uint32_t i, const LaneRay& R, int st) const {
+        if (i < nb) {
+            const HitRec h = ray_record(g, R, st, 0u);
+            hits[i] = make_uint4(h.w0, h.w1, h.w2, h.w3);
+        } else {
+            blocked[__ldg(sid + (i - nb))] = st == kRayHit ? 1 : 0;
+        }
     }
-    const uint32_t kb = wave_append(nqn, bounce);
-    if (bounce) {
-        nq[kb] = vt_ray{{so[0], so[1], so[2]}, {nd[0], nd[1], nd[2]}};
-        nqid[kb] = p;
+};
+
+// The launch shape of trace_rays_persistent_kernel.
+constexpr int kWaveThreads = 128;
+__global__ void __launch_bounds__(kWaveThreads, 9) wave_trace_kernel(
+    GridView g, PathParams P, const vt_ray* __restrict__ q, const unsigned int* __restrict__ qn,
+    uint4* __restrict__ hits, const float* __restrict__ so, const uint32_t* __restrict__ sid,
+    const unsigned int* __restrict__ sqn, uint8_t* __restrict__ blocked,
+    unsigned long long* __restrict__ counter, uint32_t refill_min,
+    unsigned long long* __restrict__ rays_out) {
+    const uint32_t nb = *qn, ns = *sqn;
+    if (rays_out && blockIdx.x == 0 && threadIdx.x == 0)
+        atomicAdd(rays_out, (unsigned long long)nb + ns);
+    const WaveIo io{g, reinterpret_cast<const float2*>(q), hits, nb, so, sid, blocked,
+                    P.sun_dir[0], P.sun_dir[1], P.sun_dir[2]};
+    trace_persistent(g, io, (uint64_t)nb + ns, counter, refill_min);
+}
+
+// The light of a path's queued sun ray (state S, before its throughput changes), if it is unblocked.
+__device__ __forceinline__ bool add_sun(const PathParams& P, const WaveState& S,
+                                        const uint8_t* __restrict__ blocked, uint32_t p, float4& L) {
+    const uint32_t bits = __float_as_uint(S.w);
+    if (!(bits & kSunPending) || blocked[p]) return false;
+    const float ndl = sun_ndl(P, bits & VT_FACE_MASK);
+    L.x = __fadd_rn(L.x, __fmul_rn(__fmul_rn(S.x, P.sun[0]), ndl));
+    L.y = __fadd_rn(L.y, __fmul_rn(__fmul_rn(S.y, P.sun[1]), ndl));
+    L.z = __fadd_rn(L.z, __fmul_rn(__fmul_rn(S.z, P.sun[2]), ndl));
+    return true;
+}
+
+// Vertex b of every queued path: its ray ended with record h.  First the light of the sun ray of the
+// vertex before, then the vertex's own sky, throughput, sun ray and bounce ray.
+__global__ void __launch_bounds__(256) wave_shade_kernel(
+    PathParams P, uint32_t b, uint32_t s0, uint32_t sn, uint32_t w,
+    const vt_ray* __restrict__ q, const uint32_t* __restrict__ qid,
+    const unsigned int* __restrict__ qn, const uint4* __restrict__ hits,
+    WaveState* __restrict__ st, float4* __restrict__ samples, const uint8_t* __restrict__ blocked,
+    float* __restrict__ sq, uint32_t* __restrict__ sid, unsigned int* __restrict__ sqn,
+    vt_ray* __restrict__ nq, uint32_t* __restrict__ nqid, unsigned int* __restrict__ nqn) {
+    const uint32_t n = *qn;
+    for (uint32_t j0 = blockIdx.x * 256u; j0 < n; j0 += gridDim.x * 256u) {
+        const uint32_t j = j0 + threadIdx.x;
+        bool sun = false, bounce = false;
+        uint32_t p = 0;
+        float so[3] = {0.0f, 0.0f, 0.0f}, nd[3] = {0.0f, 0.0f, 0.0f};
+        if (j < n) {
+            p = qid[j];
+            const uint4 hv = hits[j];
+            const HitRec h = {hv.x, hv.y, hv.z, hv.w};
+            const WaveState S = st[p];
+            const uint32_t flags = h.w1 >> 24;
+            const uint32_t face = flags & VT_FACE_MASK;
+            const bool pending = __float_as_uint(S.w) & kSunPending;
+            const bool missed = !(flags & VT_HIT_FLAG_HIT);
+            if (pending || missed) {  // the radiance may change
+                float4 L = samples[p];
+                bool changed = pending && add_sun(P, S, blocked, p, L);
+                if (missed) {
+                    L.x = __fadd_rn(L.x, __fmul_rn(S.x, P.sky[0]));
+                    L.y = __fadd_rn(L.y, __fmul_rn(S.y, P.sky[1]));
+                    L.z = __fadd_rn(L.z, __fmul_rn(S.z, P.sky[2]));
+                    changed = true;
+                }
+                if (changed) samples[p] = L;
+            }
+            if (!missed && face != 0) {
+                float T[3] = {S.x, S.y, S.z};
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                    T[c] = __fmul_rn(T[c], __fdiv_rn(__uint2float_rn((h.w3 >> (8 * c)) & 0xFFu), 255.0f));
+                const vt_ray r = q[j];
+                shadow_origin(h, r.origin, r.dir, so);
+                sun = P.sun_on && sun_ndl(P, face) > 0.0f;
+                if (b < P.max_bounces) {
+                    bounce = true;
+                    uint32_t px, py, s;
+                    wave_path_pixel(p, sn, s0, w, px, py, s);
+                    bounce_dir(P, px, py, s, b, (int)(face - 1) / 2, (face & 1u) != 0u, nd);
+                }
+                if (sun || bounce)
+                    st[p] = make_float4(T[0], T[1], T[2], __uint_as_float(face | (sun ? kSunPending : 0u)));
+            }
+        }
+        uint32_t ks, kb;
+        block_append<8>(sqn, sun, ks, nqn, bounce, kb);
+        if (sun) {
+            float* f = sq + 3 * (size_t)ks;
+            f[0] = so[0];
+            f[1] = so[1];
+            f[2] = so[2];
+            sid[ks] = p;
+        }
+        if (bounce) {
+            nq[kb] = vt_ray{{so[0], so[1], so[2]}, {nd[0], nd[1], nd[2]}};
+            nqid[kb] = p;
+        }
     }
 }
 
-// The sun rays of vertex b: light of the unblocked ones; paths ending at this vertex are done.
-__global__ void __launch_bounds__(256) wave_sun_kernel(PathParams P, bool last,
-                                                       const uint32_t* __restrict__ sid,
+// The light of the last vertex's sun rays.
+__global__ void __launch_bounds__(256) wave_sun_kernel(PathParams P, const uint32_t* __restrict__ sid,
                                                        const unsigned int* __restrict__ sqn,
-                                                       const uint4* __restrict__ hits,
-                                                       WaveState* __restrict__ st,
-                                                       float4* __restrict__ samples,
-                                                       unsigned long long* __restrict__ rays_out) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+                                                       const uint8_t* __restrict__ blocked,
+                                                       const WaveState* __restrict__ st,
+                                                       float4* __restrict__ samples) {
     const uint32_t n = *sqn;
-    if (rays_out && j == 0) atomicAdd(rays_out, (unsigned long long)n);
-    if (j >= n) return;
-    const uint32_t p = sid[j];
-    WaveState& S = st[p];
-    if (!((hits[j].y >> 24) & VT_HIT_FLAG_HIT)) {
-        const int a = (int)(S.face - 1) / 2;
-        const bool npos = (S.face & 1u) != 0u;
-        const float la = a == 0 ? P.sun_dir[0] : (a == 1 ? P.sun_dir[1] : P.sun_dir[2]);
-        const float ndl = npos ? la : -la;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) S.L[c] = __fadd_rn(S.L[c], __fmul_rn(__fmul_rn(S.T[c], P.sun[c]), ndl));
+    for (uint32_t j = blockIdx.x * 256u + threadIdx.x; j < n; j += gridDim.x * 256u) {
+        const uint32_t p = sid[j];
+        float4 L = samples[p];
+        if (add_sun(P, st[p], blocked, p, L)) samples[p] = L;
     }
-    if (last) samples[p] = make_float4(S.L[0], S.L[1], S.L[2], 0.0f);
+}
+
+static int wave_resident_blocks() {
+    static int n = -1;
+    if (n < 0) {
+        int k = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, (const void*)wave_trace_kernel,
+                                                          kWaveThreads, 0) != cudaSuccess) {
+            cudaGetLastError();
+            k = 1;
+        }
+        n = k < 1 ? 1 : k;
+    }
+    return n;
 }
 
 static cudaError_t launch_path_wave(const GridView& g, const vt_camera& cam, const PathParams& P,
@@ -714,30 +815,50 @@ static cudaError_t launch_path_wave(const GridView& g, const vt_camera& cam, con
         1, std::min<uint64_t>(std::min(P.spp, kPathChunkSpp), kWaveChunkPaths / npx));
     const uint64_t cap = (uint64_t)npx * sn;
     auto al = [](uint64_t v) { return (v + 255) / 256 * 256; };
-    // q, nq, sq (rays); qid, nqid, sid; hits; state; samples; sums; counts
-    const uint64_t o_q = 0, o_nq = al(cap * 24), o_sq = o_nq + al(cap * 24), o_qid = o_sq + al(cap * 24);
-    const uint64_t o_nqid = o_qid + al(cap * 4), o_sid = o_nqid + al(cap * 4), o_hit = o_sid + al(cap * 4);
+    // q, nq (rays); sq (two buffers: the sun rays being traced and those being made); qid, nqid,
+    // sid (two); hits; state; samples; sums; blocked; counts
+    const uint64_t o_q = 0, o_nq = al(cap * 24), o_sq = o_nq + al(cap * 24), o_sq2 = o_sq + al(cap * 12);
+    const uint64_t o_qid = o_sq2 + al(cap * 12), o_nqid = o_qid + al(cap * 4), o_sid = o_nqid + al(cap * 4);
+    const uint64_t o_sid2 = o_sid + al(cap * 4), o_hit = o_sid2 + al(cap * 4);
     const uint64_t o_st = o_hit + al(cap * 16), o_smp = o_st + al(cap * sizeof(WaveState));
-    const uint64_t o_sum = o_smp + al(cap * 16), o_cnt = o_sum + al((uint64_t)npx * 16);
+    const uint64_t o_sum = o_smp + al(cap * 16), o_blk = o_sum + al((uint64_t)npx * 16);
+    const uint64_t o_cnt = o_blk + al(cap);
     const uint64_t total_bytes = o_cnt + kWaveCounters * 4;
     char* buf = nullptr;
     cudaError_t e = cudaMallocAsync((void**)&buf, total_bytes, st);
     if (e != cudaSuccess) return e;
     vt_ray* q = (vt_ray*)(buf + o_q);
     vt_ray* nq = (vt_ray*)(buf + o_nq);
-    vt_ray* sq = (vt_ray*)(buf + o_sq);
+    float* sq = (float*)(buf + o_sq);    // sun rays of the vertex before
+    float* nsq = (float*)(buf + o_sq2);  // sun rays the shading makes
     uint32_t* qid = (uint32_t*)(buf + o_qid);
     uint32_t* nqid = (uint32_t*)(buf + o_nqid);
     uint32_t* sid = (uint32_t*)(buf + o_sid);
+    uint32_t* nsid = (uint32_t*)(buf + o_sid2);
     uint4* hits = (uint4*)(buf + o_hit);
     WaveState* wst = (WaveState*)(buf + o_st);
     float4* samples = (float4*)(buf + o_smp);
     float4* sums = (float4*)(buf + o_sum);
+    uint8_t* blocked = (uint8_t*)(buf + o_blk);
     // lengths of the path queue of each vertex (one counter per vertex, so that the bounce queue
     // built at vertex b is the path queue of vertex b + 1 without a copy) and of the sun queues
     unsigned int* qn = (unsigned int*)(buf + o_cnt);
     unsigned int* sqn = qn + kWaveCounters / 2;
-    const unsigned blocks = (unsigned)((cap + 255) / 256);
+    const uint64_t fit = (uint64_t)sm_count * 8;  // blocks of the grid-stride kernels
+    const unsigned blocks = (unsigned)std::min<uint64_t>((cap + 255) / 256, fit);
+    const TraceTuning& tune = S.tune_rays;  // its blocks are counted in 256 threads
+    const int per_sm = wave_resident_blocks();
+    const int bps = tune.blocks_per_sm > 0 ? std::min(tune.blocks_per_sm * (256 / kWaveThreads), per_sm) : per_sm;
+    const unsigned tblocks = (unsigned)std::min<uint64_t>((uint64_t)sm_count * bps,
+                                                          (2 * cap + kWaveThreads - 1) / kWaveThreads);
+    auto trace = [&](const unsigned int* bounces, const unsigned int* suns) {
+        unsigned long long* counter = next_counter();
+        cudaError_t r = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
+        if (r != cudaSuccess) return r;
+        wave_trace_kernel<<<tblocks, kWaveThreads, 0, st>>>(g, P, q, bounces, hits, sq, sid, suns, blocked,
+                                                            counter, tune.refill_min, rays);
+        return cudaGetLastError();
+    };
     for (uint32_t s0 = 0; s0 < P.spp && e == cudaSuccess; s0 += sn) {
         const uint32_t n = std::min(sn, P.spp - s0);
         const uint64_t items = (uint64_t)tiles_x * tiles_y * n * 32;
@@ -747,25 +868,25 @@ static cudaError_t launch_path_wave(const GridView& g, const vt_camera& cam, con
             g, cam, P, s0, n, tiles_x, items, q, qid, qn + 1, wst, samples, rays);
         e = cudaGetLastError();
         for (uint32_t b = 1; b <= P.max_bounces && e == cudaSuccess; ++b) {
-            // queue lengths: qn[b] paths at vertex b, qn[b + 1] bounce rays, sqn[b] sun rays
-            unsigned int* cq = qn + b;
-            unsigned int* cs = sqn + b;
-            e = launch_trace_rays_persistent(g, q, cap, hits, next_counter(), S.tune_rays,
-                                             sm_count, st, cq);
+            // queue lengths: qn[b] paths at vertex b, qn[b + 1] bounce rays, sqn[b] sun rays of vertex b
+            e = trace(qn + b, sqn + b - 1);
             if (e != cudaSuccess) break;
-            wave_shade_kernel<<<blocks, 256, 0, st>>>(g, P, b, s0, n, cam.width, q, qid, cq, hits,
-                                                      wst, samples, sq, sid, cs, nq, nqid, cq + 1,
-                                                      rays);
-            e = launch_trace_rays_persistent(g, sq, cap, hits, next_counter(), S.tune_rays,
-                                             sm_count, st, cs);
-            if (e != cudaSuccess) break;
-            wave_sun_kernel<<<blocks, 256, 0, st>>>(P, b >= P.max_bounces, sid, cs, hits, wst,
-                                                    samples, rays);
-            // the bounce rays stay in the order the shading appended them, which follows the
-            // path queue: neighbouring entries leave neighbouring surface points
+            wave_shade_kernel<<<blocks, 256, 0, st>>>(P, b, s0, n, cam.width, q, qid, qn + b, hits, wst,
+                                                      samples, blocked, nsq, nsid, sqn + b, nq, nqid,
+                                                      qn + b + 1);
             std::swap(q, nq);
             std::swap(qid, nqid);
+            std::swap(sq, nsq);
+            std::swap(sid, nsid);
             e = cudaGetLastError();
+        }
+        if (e == cudaSuccess && P.max_bounces > 0 && P.sun_on) {
+            // no bounce rays are left (that counter stays 0)
+            e = trace(qn + P.max_bounces + 1, sqn + P.max_bounces);
+            if (e == cudaSuccess) {
+                wave_sun_kernel<<<blocks, 256, 0, st>>>(P, sid, sqn + P.max_bounces, blocked, wst, samples);
+                e = cudaGetLastError();
+            }
         }
         if (e != cudaSuccess) break;
         path_resolve_kernel<<<(npx + 255) / 256, 256, 0, st>>>(samples, sums, npx, n, s0 == 0,

@@ -69,10 +69,8 @@ template <bool STATS>
 __global__ void __launch_bounds__(256) trace_rays_kernel(GridView g,
                                                          const float2* __restrict__ rays,
                                                          uint64_t n, uint4* __restrict__ out,
-                                                         Counters* __restrict__ counters,
-                                                         const unsigned int* __restrict__ n_dev) {
+                                                         Counters* __restrict__ counters) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n_dev) n = min((uint64_t)*n_dev, n);
     if (i >= n) return;
     Tally<STATS> tl;
     tl.bind(counters, g.bricks);
@@ -103,14 +101,14 @@ cudaError_t launch_render(const GridView& g, const vt_camera& cam, const LightVi
 }
 
 cudaError_t launch_trace_rays(const GridView& g, const vt_ray* rays, uint64_t n, uint4* out,
-                              Counters* counters, cudaStream_t stream, const unsigned int* n_dev) {
+                              Counters* counters, cudaStream_t stream) {
     if (n == 0) return cudaSuccess;
     const uint64_t blocks = (n + 255) / 256;
     const float2* r2 = reinterpret_cast<const float2*>(rays);
     if (counters)
-        trace_rays_kernel<true><<<(unsigned)blocks, 256, 0, stream>>>(g, r2, n, out, counters, n_dev);
+        trace_rays_kernel<true><<<(unsigned)blocks, 256, 0, stream>>>(g, r2, n, out, counters);
     else
-        trace_rays_kernel<false><<<(unsigned)blocks, 256, 0, stream>>>(g, r2, n, out, nullptr, n_dev);
+        trace_rays_kernel<false><<<(unsigned)blocks, 256, 0, stream>>>(g, r2, n, out, nullptr);
     return cudaGetLastError();
 }
 
@@ -240,72 +238,34 @@ __global__ void __launch_bounds__(256) render_persistent_kernel(
     }
 }
 
-constexpr int kUnitWait = 4;
+// Rays and records of a ray buffer (24-byte rays: three 8-byte loads).
+struct BufferIo {
+    using Index = uint64_t;
+    const GridView& g;
+    const float2* __restrict__ rays;
+    uint4* __restrict__ out;
+    __device__ __forceinline__ void load(uint64_t i, float o[3], float d[3]) const {
+        const float2 a = __ldg(rays + 3 * i), b = __ldg(rays + 3 * i + 1), c = __ldg(rays + 3 * i + 2);
+        o[0] = a.x;
+        o[1] = a.y;
+        o[2] = b.x;
+        d[0] = b.y;
+        d[1] = c.x;
+        d[2] = c.y;
+    }
+    __device__ __forceinline__ void store(uint64_t i, const LaneRay& R, int st) const {
+        const HitRec h = ray_record(g, R, st, 0u);
+        out[i] = make_uint4(h.w0, h.w1, h.w2, h.w3);
+    }
+};
 
-// n_dev: nullptr, or the device-side ray count (at most n), read at the start (ray queues whose
-// length the host does not know).  Blocks of 128 threads, nine per SM at 56 registers: 16.7M cave
-// rays 1.899 ms, path-traced 1080p frame 4.28 ms, against 1.905 and 4.32 ms for five blocks of 256 at
-// 48 registers (a few bytes of spills) and 2.00 ms for four at 64 registers.
+// Blocks of 128 threads, nine per SM at 56 registers: 16.7M cave rays 1.899 ms against 1.905 ms for
+// five blocks of 256 at 48 registers (a few bytes of spills) and 2.00 ms for four at 64 registers.
 constexpr int kRayThreads = 128;
 __global__ void __launch_bounds__(kRayThreads, 9) trace_rays_persistent_kernel(
     GridView g, const float2* __restrict__ rays, uint64_t n, uint4* __restrict__ out,
-    unsigned long long* __restrict__ counter, uint32_t refill_min,
-    const unsigned int* __restrict__ n_dev) {
-    if (n_dev) n = min((uint64_t)*n_dev, n);
-    const uint32_t lane = threadIdx.x & 31u;
-    LaneRay R;
-    bool busy = false;
-    uint64_t idx = 0;
-    bool more = true;
-    int wait_w = 0, wait_c = 0;  // warp-uniform: iterations a unit kind was passed over
-    for (;;) {
-        uint32_t idle = __ballot_sync(0xFFFFFFFFu, !busy);
-        while (more && __popc(idle) >= (int)refill_min) {
-            uint64_t item;
-            const uint64_t base = warp_fetch(counter, idle, lane, item);
-            if (base + __popc(idle) >= n) more = false;
-            if (!busy && item < n) {
-                const float2 a = __ldg(rays + 3 * item), b = __ldg(rays + 3 * item + 1),
-                             c = __ldg(rays + 3 * item + 2);
-                const float o[3] = {a.x, a.y, b.x}, d[3] = {b.y, c.x, c.y};
-                const int st = ray_begin(g, o, d, R);
-                if (st == kRayRunning) {
-                    busy = true;
-                    idx = item;
-                } else {
-                    const HitRec h = ray_record(g, R, st, 0u);
-                    out[item] = make_uint4(h.w0, h.w1, h.w2, h.w3);
-                }
-            }
-            idle = __ballot_sync(0xFFFFFFFFu, !busy);
-        }
-        if (!more && idle == 0xFFFFFFFFu) break;
-        // One kind of unit per pass: the lanes whose next unit is the more common kind (walk or
-        // crossing) run it, the others wait, unless their kind has already waited kUnitWait
-        // passes.  A warp then issues one kind's instructions per pass instead of both; every
-        // pass with busy lanes runs at least one unit.  2% faster on the 16M incoherent rays.
-        const uint32_t e = busy ? ray_entry(g, R) : kEmptyBit;
-        const bool walk = busy && !brick_empty(e);
-        const uint32_t wb = __ballot_sync(0xFFFFFFFFu, walk);
-        const uint32_t cb = __ballot_sync(0xFFFFFFFFu, busy && !walk);
-        bool run_walk = __popc(wb) >= __popc(cb);
-        if (run_walk ? (cb && wait_c >= kUnitWait) : (wb && wait_w >= kUnitWait)) run_walk = !run_walk;
-        if (run_walk) {
-            wait_w = 0;
-            wait_c = cb ? wait_c + 1 : 0;
-        } else {
-            wait_c = 0;
-            wait_w = wb ? wait_w + 1 : 0;
-        }
-        if (busy && walk == run_walk) {
-            const int st = ray_unit(g, R, e);
-            if (st != kRayRunning) {
-                const HitRec h = ray_record(g, R, st, 0u);
-                out[idx] = make_uint4(h.w0, h.w1, h.w2, h.w3);
-                busy = false;
-            }
-        }
-    }
+    unsigned long long* __restrict__ counter, uint32_t refill_min) {
+    trace_persistent(g, BufferIo{g, rays, out}, n, counter, refill_min);
 }
 
 static int resident_blocks(const void* kernel, int threads = 256) {
@@ -337,7 +297,7 @@ cudaError_t launch_render_persistent(const GridView& g, const vt_camera& cam,
 cudaError_t launch_trace_rays_persistent(const GridView& g, const vt_ray* rays, uint64_t n,
                                          uint4* out, unsigned long long* counter,
                                          const TraceTuning& tune, int sm_count,
-                                         cudaStream_t stream, const unsigned int* n_dev) {
+                                         cudaStream_t stream) {
     if (n == 0) return cudaSuccess;
     static int per_sm = resident_blocks((const void*)trace_rays_persistent_kernel, kRayThreads);
     // the tuning counts blocks of 256 threads
@@ -347,7 +307,7 @@ cudaError_t launch_trace_rays_persistent(const GridView& g, const vt_ray* rays, 
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), stream);
     if (e != cudaSuccess) return e;
     trace_rays_persistent_kernel<<<blocks, kRayThreads, 0, stream>>>(
-        g, reinterpret_cast<const float2*>(rays), n, out, counter, tune.refill_min, n_dev);
+        g, reinterpret_cast<const float2*>(rays), n, out, counter, tune.refill_min);
     return cudaGetLastError();
 }
 
