@@ -234,7 +234,7 @@ struct SmallBuild {
     void* in = nullptr;          // the shape's dense voxels
     void* tmpl = nullptr;        // block layout with a slot per brick
     void* scratch = nullptr;
-    uint32_t* counts = nullptr;  // last slot offset, last flag, occupied voxels (u64), deep bricks?
+    uint32_t* counts = nullptr;  // occupied voxels (u64), occupied bricks (u64), deep bricks?
     cudaGraphExec_t exec = nullptr;
     uint64_t last_use = 0;
 };
@@ -309,13 +309,7 @@ static int32_t small_entry(const Grid& shape, bool nonzero, SmallBuild*& out) {
         if (e == cudaSuccess) {
             cudaError_t le = build_launches(b.in, shape.format, t.palette, nonzero, t, s, cs);
             if (le == cudaSuccess)
-                le = cudaMemcpyAsync(b.counts, s.offsets + (shape.bricks - 1), 4,
-                                     cudaMemcpyDeviceToDevice, cs);
-            if (le == cudaSuccess)
-                le = cudaMemcpyAsync(b.counts + 1, s.flags + (shape.bricks - 1), 4,
-                                     cudaMemcpyDeviceToDevice, cs);
-            if (le == cudaSuccess)
-                le = cudaMemcpyAsync(b.counts + 2, s.occupied, 8, cudaMemcpyDeviceToDevice, cs);
+                le = cudaMemcpyAsync(b.counts, s.counts, 16, cudaMemcpyDeviceToDevice, cs);
             if (le == cudaSuccess)
                 le = cudaMemcpyAsync(b.counts + 4, s.lattice.deep, 4, cudaMemcpyDeviceToDevice, cs);
             e = cudaStreamEndCapture(cs, &graph);
@@ -366,8 +360,8 @@ static int32_t build_small(const void* src, bool src_host, const uint32_t* palet
     if (e == cudaSuccess) e = cudaMemcpyAsync(hc, b->counts, 20, cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess) return cuda_fail(e, "small grid build");
-    g->nonempty = (uint64_t)hc[0] + hc[1];
-    g->occupied = (uint64_t)hc[2] | ((uint64_t)hc[3] << 32);
+    g->nonempty = (uint64_t)hc[2] | ((uint64_t)hc[3] << 32);
+    g->occupied = (uint64_t)hc[0] | ((uint64_t)hc[1] << 32);
     g->deep = hc[4] != 0u;
     g->bytes = g->block_bytes;
     g->slots_used = g->nonempty;
@@ -449,8 +443,7 @@ int32_t build_grid(const void* d_src, uint32_t format, const uint32_t* palette_h
     BuildScratch s = carve_build_scratch(scratch, bx, by, bz);
     if (staging) s.staged = (char*)scratch + staged_at;
     uint32_t* d_palette = (uint32_t*)((char*)scratch + sbytes);
-    uint32_t counts[2] = {0, 0};
-    unsigned long long occ = 0;
+    unsigned long long counts[2] = {0, 0};
     do {
         if (format == VT_PAYLOAD_U8) {
             e = cudaMemcpyAsync(d_palette, palette_host, 1024, cudaMemcpyHostToDevice, stream);
@@ -459,15 +452,11 @@ int32_t build_grid(const void* d_src, uint32_t format, const uint32_t* palette_h
         e = launch_brick_words(d_src, format, d_palette, (int32_t)nx, (int32_t)ny, (int32_t)nz, s,
                                stream, nonzero);
         if (e == cudaSuccess) e = launch_brick_scan(s, g->bricks, stream);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(&counts[0], s.offsets + (g->bricks - 1), 4, cudaMemcpyDeviceToHost, stream);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(&counts[1], s.flags + (g->bricks - 1), 4, cudaMemcpyDeviceToHost, stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&occ, s.occupied, 8, cudaMemcpyDeviceToHost, stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(counts, s.counts, 16, cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) { rc = cuda_fail(e, "brick count"); break; }
-        g->nonempty = (uint64_t)counts[0] + counts[1];
-        g->occupied = occ;
+        g->nonempty = counts[1];
+        g->occupied = counts[0];
         const uint64_t slots = g->nonempty ? g->nonempty : 1;
         const BlockLayout L = block_layout(g->bricks, slots, format);
         void* block = nullptr;

@@ -2,14 +2,15 @@
 // lib/memory.c:286-385): x-fastest u8 palette indices or RGBA8 texels in device memory become
 // an 8^3-brick directory, 512-bit occupancy masks and dense payloads of occupied bricks only.
 //
-// Three passes, all coalesced along x:
-//   words   one thread per (brick, z-slice): reads 8 rows of 8 voxels, builds the 64-bit
-//           occupancy word; the 8 lanes of a brick OR their words into the brick's flag
-//   scan    exclusive prefix sum of the flags = each occupied brick's slot
-//   compact one thread per (brick, z-slice) of occupied bricks: copies the word and the slice's
-//           64 voxels into the slot; writes the directory
-// Lanes are assigned slice-fastest, so a warp covers 4 consecutive bricks along x: its reads are
-// 8 z-planes x 32 contiguous bytes per row and its word writes are 256 contiguous bytes.
+// Three passes:
+//   words   one thread per (brick, z-slice): reads 8 rows of 8 voxels and builds the 64-bit occupancy
+//           word; 32 consecutive bricks share one word of occupancy bits
+//   scan    exclusive prefix sum of those words' bit counts = each occupied brick's slot
+//   compact one warp per 32 bricks: copies the words and voxels of the occupied ones into their
+//           slots; writes the directory
+// In the words pass a warp's lanes are 32 consecutive bricks and a block's eight warps their eight
+// z-slices, so a load instruction reads 256 contiguous bytes of a row.  With lanes running over
+// the slices of four bricks it read eight pieces of 32 bytes from as many planes.
 // With a staging buffer (one 512-voxel block per brick, indexed by brick), the words pass also
 // writes the voxels of each occupied brick there, brick-major, while it holds them, and the
 // compaction copies whole staged blocks: without it the compaction re-reads the dense grid's rows,
@@ -28,13 +29,13 @@ constexpr uint64_t kScanBlock = (uint64_t)kScanThreads * kScanItems;
 static inline uint64_t align_up(uint64_t v, uint64_t a) { return (v + a - 1) / a * a; }
 
 static uint64_t scan_partials(uint64_t n) {
-    // partial sums of every recursion level of the scan
-    uint64_t total = 0;
-    while (n > kScanBlock) {
+    // block totals of every level of the scan, down to a single one
+    uint64_t total = 64;
+    do {
         n = (n + kScanBlock - 1) / kScanBlock;
         total += align_up(n, 64);
-    }
-    return total + 64;
+    } while (n > 1);
+    return total;
 }
 
 // The occupancy words are not read after the compaction: the lattice passes take their space.
@@ -44,10 +45,12 @@ static uint64_t words_bytes(int32_t bx, int32_t by, int32_t bz) {
     return align_up(words > lattice ? words : lattice, 256);
 }
 
+static uint64_t occ_count(uint64_t bricks) { return (bricks + 31) / 32; }
+
 size_t build_scratch_bytes(int32_t bx, int32_t by, int32_t bz) {
-    const uint64_t bricks = (uint64_t)bx * by * bz;
-    return (size_t)(words_bytes(bx, by, bz) + align_up(bricks * 4, 256) * 2 +
-                    align_up(scan_partials(bricks) * 4, 256) + 256);
+    const uint64_t n = occ_count((uint64_t)bx * by * bz);
+    return (size_t)(words_bytes(bx, by, bz) + align_up(n * 4, 256) * 2 +
+                    align_up(scan_partials(n) * 4, 256) + 256);
 }
 
 size_t build_staging_bytes(uint64_t bricks, uint32_t format) {
@@ -61,13 +64,14 @@ BuildScratch carve_build_scratch(void* base, int32_t bx, int32_t by, int32_t bz)
     s.words = (uint64_t*)p;
     s.lattice = carve_lattice_scratch(p, bx, by, bz);
     p += words_bytes(bx, by, bz);
-    s.flags = (uint32_t*)p;
-    p += align_up(bricks * 4, 256);
+    const uint64_t n = occ_count(bricks);
+    s.occ = (uint32_t*)p;
+    p += align_up(n * 4, 256);
     s.offsets = (uint32_t*)p;
-    p += align_up(bricks * 4, 256);
+    p += align_up(n * 4, 256);
     s.block_sums = (uint32_t*)p;
-    p += align_up(scan_partials(bricks) * 4, 256);
-    s.occupied = (unsigned long long*)p;
+    p += align_up(scan_partials(n) * 4, 256);
+    s.counts = (unsigned long long*)p;
     return s;
 }
 
@@ -76,11 +80,11 @@ struct BrickCoord {
 };
 
 __device__ __forceinline__ BrickCoord brick_coord(uint64_t brick, int32_t bx, int32_t by) {
+    const uint32_t b = (uint32_t)brick, r = b / (uint32_t)bx;  // fewer than 2^31 bricks
     BrickCoord c;
-    c.bxi = (int32_t)(brick % (uint64_t)bx);
-    const uint64_t r = brick / (uint64_t)bx;
-    c.byi = (int32_t)(r % (uint64_t)by);
-    c.bzi = (int32_t)(r / (uint64_t)by);
+    c.bxi = (int32_t)(b - r * (uint32_t)bx);
+    c.bzi = (int32_t)(r / (uint32_t)by);
+    c.byi = (int32_t)(r - (uint32_t)c.bzi * (uint32_t)by);
     return c;
 }
 
@@ -175,37 +179,40 @@ __device__ __forceinline__ void copy_slice(const void* __restrict__ src, int32_t
 
 // NZ: u8 grid whose palette has alpha 0 at index 0 only, so that occupancy is "index != 0" and the
 // row bits come from byte arithmetic instead of palette lookups.
+//
+// Bound by reading the dense grid: 1 GiB of u8 voxels in and 115 MB of staged ones and words out in
+// 202 us, 5.9 TB/s (0.87 of the measured copy rate); 276 us with lanes over slices, every brick's words
+// written and an atomic per warp on the voxel count.
 template <uint32_t FMT, bool NZ>
 __global__ void __launch_bounds__(256) brick_words_kernel(const void* __restrict__ src,
                                                           const uint32_t* __restrict__ palette,
                                                           int32_t nx, int32_t ny, int32_t nz,
                                                           int32_t bx, int32_t by, uint64_t bricks,
                                                           uint64_t* __restrict__ words,
-                                                          uint32_t* __restrict__ flags,
+                                                          uint32_t* __restrict__ occ,
                                                           unsigned long long* occupied,
                                                           void* __restrict__ staged) {
     __shared__ uint8_t lut[256];
+    __shared__ uint32_t s_any[8], s_count[8];
     if (FMT == VT_PAYLOAD_U8 && !NZ) {
         for (int i = threadIdx.x; i < 256; i += blockDim.x)
             lut[i] = (uint8_t)((__ldg(palette + i) >> 24) != 0u);
         __syncthreads();
     }
-    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t lz = (uint32_t)(t & 7u);
-    const uint64_t brick = t >> 3;
-    const bool valid = brick < bricks;
+    const uint32_t lane = threadIdx.x & 31u, lz = threadIdx.x >> 5;
+    const uint64_t brick = (uint64_t)blockIdx.x * 32u + lane;
     uint64_t w = 0;
     BrickCoord c = {0, 0, 0};
     bool whole = false;  // the slice's rows are in r[], 8-byte aligned and inside the grid
     uint64_t r[8];
-    if (valid) {
+    if (brick < bricks) {
         c = brick_coord(brick, bx, by);
         const int32_t z = c.bzi * 8 + (int32_t)lz, x0 = c.bxi * 8;
         if (z < nz) {
             const size_t plane = (size_t)nx * (size_t)ny * (size_t)z;
-            if (NZ && x0 + 8 <= nx && (nx & 7) == 0 && c.byi * 8 + 8 <= ny) {
+            const uint8_t* base = (const uint8_t*)src + plane + (size_t)nx * (size_t)(c.byi * 8) + x0;
+            if (NZ && x0 + 8 <= nx && (nx & 7) == 0 && (((uintptr_t)src) & 7u) == 0 && c.byi * 8 + 8 <= ny) {
                 // whole rows, 8-byte aligned: issue the eight loads before using any
-                const uint8_t* base = (const uint8_t*)src + plane + (size_t)nx * (size_t)(c.byi * 8) + x0;
                 whole = true;
 #pragma unroll
                 for (int ly = 0; ly < 8; ++ly) r[ly] = __ldg((const unsigned long long*)(base + (size_t)nx * ly));
@@ -221,14 +228,26 @@ __global__ void __launch_bounds__(256) brick_words_kernel(const void* __restrict
             }
         }
     }
-    uint64_t any = w;
-    any |= __shfl_xor_sync(0xFFFFFFFFu, any, 1);
-    any |= __shfl_xor_sync(0xFFFFFFFFu, any, 2);
-    any |= __shfl_xor_sync(0xFFFFFFFFu, any, 4);
-    if (valid) {
+    const uint32_t some = __ballot_sync(0xFFFFFFFFu, w != 0);
+    const uint32_t count = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)__popcll(w));
+    if (lane == 0) {
+        s_any[lz] = some;
+        s_count[lz] = count;
+    }
+    __syncthreads();
+    uint32_t any = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) any |= s_any[k];
+    if (threadIdx.x == 0) {
+        occ[blockIdx.x] = any;
+        uint32_t total = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) total += s_count[k];
+        if (total) atomicAdd(occupied, (unsigned long long)total);
+    }
+    if ((any >> lane) & 1u) {
         words[brick * 8 + lz] = w;
-        if (lz == 0) flags[brick] = any != 0 ? 1u : 0u;
-        if (staged && any) {  // the brick's block in the staging buffer, slice lz
+        if (staged) {  // the brick's block in the staging buffer, slice lz
             constexpr size_t E = FMT == VT_PAYLOAD_RGBA8 ? 4 : 1;
             uint8_t* dst = (uint8_t*)staged + (brick * 512 + lz * 64) * E;
             if (whole) {
@@ -242,13 +261,11 @@ __global__ void __launch_bounds__(256) brick_words_kernel(const void* __restrict
             }
         }
     }
-    unsigned long long pc = (unsigned long long)__popcll(w);
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) pc += __shfl_xor_sync(0xFFFFFFFFu, pc, off);
-    if ((threadIdx.x & 31) == 0 && pc) atomicAdd(occupied, pc);
 }
 
-// Exclusive scan of up to kScanBlock items per block; block totals go to `sums`.
+// Exclusive scan of up to kScanBlock items per block, of their bit counts with BITS; block totals go
+// to `sums`.
+template <bool BITS>
 __global__ void __launch_bounds__(kScanThreads) scan_block_kernel(const uint32_t* __restrict__ in,
                                                                   uint32_t* __restrict__ out,
                                                                   uint64_t n,
@@ -258,7 +275,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_block_kernel(const uint32_t
     uint32_t v[kScanItems], local = 0;
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
-        v[k] = base + k < n ? in[base + k] : 0u;
+        v[k] = base + k < n ? (BITS ? (uint32_t)__popc(in[base + k]) : in[base + k]) : 0u;
         local += v[k];
     }
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -295,22 +312,40 @@ __global__ void scan_add_kernel(uint32_t* __restrict__ out, uint64_t n,
     if (i < n) out[i] += block_offsets[i / kScanBlock];
 }
 
-static cudaError_t scan_exclusive(const uint32_t* in, uint32_t* out, uint64_t n, uint32_t* partial,
-                                  cudaStream_t stream) {
+// In-place exclusive scan of `n` block totals; `next` holds the totals one level up.
+static cudaError_t scan_totals(uint32_t* sums, uint64_t n, uint32_t* next, cudaStream_t stream) {
     const uint64_t blocks = (n + kScanBlock - 1) / kScanBlock;
-    scan_block_kernel<<<(unsigned)blocks, kScanThreads, 0, stream>>>(in, out, n, partial);
+    scan_block_kernel<false><<<(unsigned)blocks, kScanThreads, 0, stream>>>(sums, sums, n, next);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || blocks == 1) return e;
-    // scan the block totals in place one level up, then add them back
-    uint32_t* next = partial + align_up(blocks, 64);
-    e = scan_exclusive(partial, partial, blocks, next, stream);
+    e = scan_totals(next, blocks, next + align_up(blocks, 64), stream);
     if (e != cudaSuccess) return e;
-    scan_add_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(out, n, partial);
+    scan_add_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(sums, n, next);
     return cudaGetLastError();
 }
 
+// Slot of the first occupied brick of occupancy word `w`.
+__device__ __forceinline__ uint32_t first_slot(const uint32_t* offsets, const uint32_t* block_sums, uint64_t w) {
+    return __ldg(offsets + w) + __ldg(block_sums + w / kScanBlock);
+}
+
+// counts[1] = occupied bricks (counts[0], the occupied voxels, is summed by the words pass).
+__global__ void brick_count_kernel(const uint32_t* __restrict__ occ, const uint32_t* __restrict__ offsets,
+                                   const uint32_t* __restrict__ block_sums, uint64_t n,
+                                   unsigned long long* __restrict__ counts) {
+    counts[1] = (unsigned long long)first_slot(offsets, block_sums, n - 1) + (uint32_t)__popc(occ[n - 1]);
+}
+
 cudaError_t launch_brick_scan(const BuildScratch& s, uint64_t bricks, cudaStream_t stream) {
-    return scan_exclusive(s.flags, s.offsets, bricks, s.block_sums, stream);
+    // the totals of the lowest level are scanned in place; the compaction adds them to its words'
+    // offsets as it reads them
+    const uint64_t n = occ_count(bricks), blocks = (n + kScanBlock - 1) / kScanBlock;
+    scan_block_kernel<true><<<(unsigned)blocks, kScanThreads, 0, stream>>>(s.occ, s.offsets, n, s.block_sums);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = scan_totals(s.block_sums, blocks, s.block_sums + align_up(blocks, 64), stream);
+    if (e != cudaSuccess) return e;
+    brick_count_kernel<<<1, 1, 0, stream>>>(s.occ, s.offsets, s.block_sums, n, s.counts);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_brick_words(const void* src, uint32_t format, const uint32_t* d_palette,
@@ -318,49 +353,67 @@ cudaError_t launch_brick_words(const void* src, uint32_t format, const uint32_t*
                                cudaStream_t stream, bool nonzero_occupancy) {
     const int32_t bx = (nx + 7) / 8, by = (ny + 7) / 8, bz = (nz + 7) / 8;
     const uint64_t bricks = (uint64_t)bx * by * bz;
-    const uint64_t threads = bricks * 8;
-    const unsigned blocks = (unsigned)((threads + 255) / 256);
-    cudaError_t e = cudaMemsetAsync(s.occupied, 0, sizeof(unsigned long long), stream);
+    const unsigned blocks = (unsigned)occ_count(bricks);
+    cudaError_t e = cudaMemsetAsync(s.counts, 0, sizeof(unsigned long long), stream);
     if (e != cudaSuccess) return e;
     if (format == VT_PAYLOAD_U8 && nonzero_occupancy)
         brick_words_kernel<VT_PAYLOAD_U8, true><<<blocks, 256, 0, stream>>>(
-            src, d_palette, nx, ny, nz, bx, by, bricks, s.words, s.flags, s.occupied, s.staged);
+            src, d_palette, nx, ny, nz, bx, by, bricks, s.words, s.occ, s.counts, s.staged);
     else if (format == VT_PAYLOAD_U8)
         brick_words_kernel<VT_PAYLOAD_U8, false><<<blocks, 256, 0, stream>>>(
-            src, d_palette, nx, ny, nz, bx, by, bricks, s.words, s.flags, s.occupied, s.staged);
+            src, d_palette, nx, ny, nz, bx, by, bricks, s.words, s.occ, s.counts, s.staged);
     else
         brick_words_kernel<VT_PAYLOAD_RGBA8, false><<<blocks, 256, 0, stream>>>(
-            src, nullptr, nx, ny, nz, bx, by, bricks, s.words, s.flags, s.occupied, s.staged);
+            src, nullptr, nx, ny, nz, bx, by, bricks, s.words, s.occ, s.counts, s.staged);
     return cudaGetLastError();
 }
 
+// A warp per 32 bricks.  Bound by copying the payloads: 102 MB and their words in and out in 42 us,
+// 5.9 TB/s (74 us with a thread per slice of every brick, of which nine in ten found an empty one;
+// 58 us with one brick at a time per warp).
 template <uint32_t FMT>
 __global__ void __launch_bounds__(256) brick_compact_kernel(
     const void* __restrict__ src, int32_t nx, int32_t ny, int32_t nz, int32_t bx, int32_t by,
-    uint64_t bricks, const uint64_t* __restrict__ words, const uint32_t* __restrict__ flags,
-    const uint32_t* __restrict__ offsets, uint32_t* __restrict__ dir, uint64_t* __restrict__ masks,
-    void* __restrict__ payload, const void* __restrict__ staged) {
+    uint64_t bricks, const uint64_t* __restrict__ words, const uint32_t* __restrict__ occ,
+    const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ block_sums,
+    uint32_t* __restrict__ dir, uint64_t* __restrict__ masks, void* __restrict__ payload,
+    const void* __restrict__ staged) {
     constexpr size_t E = FMT == VT_PAYLOAD_RGBA8 ? 4 : 1;
-    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t lz = (uint32_t)(t & 7u);
-    const uint64_t brick = t >> 3;
-    if (brick >= bricks) return;
-    const uint32_t f = __ldg(flags + brick);
-    const uint32_t slot = __ldg(offsets + brick);
-    if (lz == 0) dir[brick] = f ? slot : kEmptyBit;  // distance filled in by the lattice passes
-    if (!f) return;
-    masks[(size_t)slot * 8 + lz] = __ldg(words + brick * 8 + lz);
-    if (staged) {
-        // the brick's staged block, 16 bytes per lane and load: the 8 lanes of a brick read 128
-        // contiguous bytes per instruction
-        const uint4* from = (const uint4*)((const uint8_t*)staged + brick * 512 * E);
-        uint4* to = (uint4*)((uint8_t*)payload + (size_t)slot * 512 * E);
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t group = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, b0 = group * 32;
+    if (b0 >= bricks) return;  // whole warps
+    uint32_t left = __ldg(occ + group);
+    uint32_t slot = first_slot(offsets, block_sums, group);
+    if (b0 + lane < bricks)  // distance filled in by the lattice passes
+        dir[b0 + lane] = (left >> lane) & 1u ? slot + __popc(left & ((1u << lane) - 1u)) : kEmptyBit;
+    // four occupied bricks at a time, eight lanes each; staged blocks in pieces of 128 contiguous
+    // bytes per brick and load, all of a lane's loads in flight together
+    const uint32_t mine = lane >> 3, lz = lane & 7u;
+    for (; left; slot += 4) {
+        uint32_t at = 32;
 #pragma unroll
-        for (uint32_t k = 0; k < 4 * E; ++k) to[lz + 8 * k] = __ldg(from + lz + 8 * k);
-        return;
+        for (uint32_t k = 0; k < 4; ++k) {
+            if (k == mine && left) at = (uint32_t)__ffs((int)left) - 1u;
+            left &= left ? left - 1u : 0u;
+        }
+        if (at < 32) {
+            const uint64_t b = b0 + at;
+            const size_t to = slot + mine;
+            masks[to * 8 + lz] = __ldg(words + b * 8 + lz);
+            if (staged) {
+                const uint4* in = (const uint4*)((const uint8_t*)staged + b * 512 * E) + lz;
+                uint4* out = (uint4*)((uint8_t*)payload + to * 512 * E) + lz;
+                uint4 v[4 * E];
+#pragma unroll
+                for (uint32_t k = 0; k < 4 * E; ++k) v[k] = __ldg(in + 8 * k);
+#pragma unroll
+                for (uint32_t k = 0; k < 4 * E; ++k) out[8 * k] = v[k];
+                continue;
+            }
+            copy_slice<FMT>(src, nx, ny, nz, brick_coord(b, bx, by), lz,
+                            (uint8_t*)payload + (to * 512 + lz * 64) * E);
+        }
     }
-    copy_slice<FMT>(src, nx, ny, nz, brick_coord(brick, bx, by), lz,
-                    (uint8_t*)payload + ((size_t)slot * 512 + lz * 64) * E);
 }
 
 cudaError_t launch_brick_compact(const void* src, uint32_t format, int32_t nx, int32_t ny,
@@ -368,14 +421,14 @@ cudaError_t launch_brick_compact(const void* src, uint32_t format, int32_t nx, i
                                  uint64_t* masks, void* payload, cudaStream_t stream) {
     const int32_t bx = (nx + 7) / 8, by = (ny + 7) / 8, bz = (nz + 7) / 8;
     const uint64_t bricks = (uint64_t)bx * by * bz;
-    const unsigned blocks = (unsigned)((bricks * 8 + 255) / 256);
+    const unsigned blocks = (unsigned)((occ_count(bricks) + 7) / 8);
     if (format == VT_PAYLOAD_U8)
         brick_compact_kernel<VT_PAYLOAD_U8><<<blocks, 256, 0, stream>>>(
-            src, nx, ny, nz, bx, by, bricks, s.words, s.flags, s.offsets, dir, masks, payload,
+            src, nx, ny, nz, bx, by, bricks, s.words, s.occ, s.offsets, s.block_sums, dir, masks, payload,
             s.staged);
     else
         brick_compact_kernel<VT_PAYLOAD_RGBA8><<<blocks, 256, 0, stream>>>(
-            src, nx, ny, nz, bx, by, bricks, s.words, s.flags, s.offsets, dir, masks, payload,
+            src, nx, ny, nz, bx, by, bricks, s.words, s.occ, s.offsets, s.block_sums, dir, masks, payload,
             s.staged);
     return cudaGetLastError();
 }

@@ -69,11 +69,11 @@ LatticeScratch carve_lattice_scratch(void* base, int32_t bx, int32_t by, int32_t
 
 // Scratch of one brick build of bx x by x bz bricks.
 struct BuildScratch {
-    uint64_t* words = nullptr;      // bricks * 8 occupancy words
-    uint32_t* flags = nullptr;      // bricks: 1 if the brick holds an occupied voxel
-    uint32_t* offsets = nullptr;    // bricks: exclusive prefix sum of flags (the slot)
-    uint32_t* block_sums = nullptr; // scan partials
-    unsigned long long* occupied = nullptr;
+    uint64_t* words = nullptr;      // bricks * 8 occupancy words (those of occupied bricks written)
+    uint32_t* occ = nullptr;        // one bit per brick: it holds an occupied voxel
+    uint32_t* offsets = nullptr;    // per word of occ: occupied bricks before it in its scan block
+    uint32_t* block_sums = nullptr; // occupied bricks before each scan block, then upper levels
+    unsigned long long* counts = nullptr;  // occupied voxels, occupied bricks
     LatticeScratch lattice;         // in the place of `words`, which the compaction reads last
     // nullptr, or build_staging_bytes(): the voxels of each occupied brick as a 512-voxel block
     // at brick * 512, written by the words pass and copied by the compaction

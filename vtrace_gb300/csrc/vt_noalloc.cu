@@ -18,7 +18,7 @@
 namespace vt {
 
 // Largest grid the scratch covers: 32768 bricks (for example 256^3 voxels).  build_scratch_bytes
-// of 32^3 bricks is 2,360,064 bytes; the array is 2.5 MiB and is resident on every device
+// of 32^3 bricks is 2,106,112 bytes; the array is 2.5 MiB and is resident on every device
 // that loads the library until the process exits.
 constexpr uint64_t kNoAllocMaxBricks = 32768;
 constexpr size_t kNoAllocScratchBytes = 2621440;
@@ -54,16 +54,6 @@ void noalloc_forget_addresses() {
     for (int d = 0; d < kNoAllocMaxDevices; ++d) g_scratch_addr[d] = nullptr;
 }
 
-__global__ void noalloc_counts_kernel(const uint32_t* __restrict__ flags,
-                                      const uint32_t* __restrict__ offsets, uint64_t bricks,
-                                      const unsigned long long* __restrict__ occupied,
-                                      uint64_t* __restrict__ counts) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        counts[0] = (uint64_t)offsets[bricks - 1] + flags[bricks - 1];
-        counts[1] = *occupied;
-    }
-}
-
 }  // namespace vt
 
 using namespace vt;
@@ -95,6 +85,9 @@ extern "C" int32_t vt_grid_build_u8_noalloc(const uint8_t* d_voxels, const uint3
                              d_directory, d_masks, d_payload, st) != cudaSuccess ||
         launch_brick_distance(d_directory, nullptr, s.lattice, bx, by, bz, st) != cudaSuccess)
         return VT_ECUDA;
-    noalloc_counts_kernel<<<1, 32, 0, st>>>(s.flags, s.offsets, bricks, s.occupied, d_counts);
-    return cudaGetLastError() == cudaSuccess ? VT_OK : VT_ECUDA;
+    // d_counts: occupied bricks, occupied voxels
+    if (cudaMemcpyAsync(d_counts, s.counts + 1, 8, cudaMemcpyDeviceToDevice, st) != cudaSuccess ||
+        cudaMemcpyAsync(d_counts + 1, s.counts, 8, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
+        return VT_ECUDA;
+    return VT_OK;
 }
