@@ -1066,8 +1066,8 @@ def run_config(args):
                          "d2h_bytes_per_step": 8 * 2 * 8 + 8,
                          "path": "vt_grid_update (C ABI), synchronous, host wall clock"},
                     frame_after_updates_ms=frame_ms,
-                    # merge, scatter, 3 distance, 3 octant, run and long-box kernels per chunk
-                    gpu_launches=10 * args.steps, clocks=clocks)
+                    # the update block and three lattice kernels per chunk
+                    gpu_launches=4 * args.steps, clocks=clocks)
         g.destroy()
     elif args.config == "pager_world":
         # the reference-compatible frame (render_tick) over vtrace's own world shape

@@ -629,6 +629,8 @@ void vt_shutdown(void) {
     s.staging_bytes = 0;
     cudaFree(s.counters);
     s.counters = nullptr;
+    cudaFreeHost(s.update_pin);
+    s.update_pin = s.update_pin_dev = nullptr;
     for (int k = 0; k < State::kAux; ++k) {
         cudaStreamSynchronize(s.aux[k]);
         cudaStreamDestroy(s.aux[k]);

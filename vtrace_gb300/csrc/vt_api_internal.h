@@ -68,6 +68,11 @@ struct State {
     std::atomic<uint64_t> grid_epoch{0};
     void* staging = nullptr;
     size_t staging_bytes = 0;
+    // page-locked exchange area of small grid updates (host pointer and device address), held for a
+    // call under update_mu
+    std::mutex update_mu;
+    void* update_pin = nullptr;
+    void* update_pin_dev = nullptr;
     // work counters of the persistent launches: each launch takes the next slot of the ring
     unsigned long long* counters = nullptr;
     std::atomic<uint32_t> counter_next{0};

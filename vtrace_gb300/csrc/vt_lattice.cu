@@ -24,9 +24,9 @@
 // shared-memory look-ups (72 % of their rate in the y and z passes): the tables' 20 bytes per brick
 // are the only global traffic of size.
 //
-// 128^3 bricks (1024^3 voxels, 9.5 % of the bricks occupied): rows 11 us, x 31 us, y and z 51 us,
-// together 93 us where per-brick walks (distances, octants) and a pyramid of run minima (long
-// boxes) took 615 us; after a 16^3 chunk's update 39 us where they took 110 us.
+// 128^3 bricks (1024^3 voxels, 9.5 % of the bricks occupied): rows 8 us, x 31 us, y and z 51 us,
+// together 90 us where per-brick walks (distances, octants) and a pyramid of run minima (long
+// boxes) took 615 us; after a 16^3 chunk's update 28 us where they took 110 us.
 #include <cuda_runtime.h>
 
 #include "vt_device.cuh"
@@ -96,11 +96,17 @@ __global__ void __launch_bounds__(256) lattice_rows_kernel(const uint32_t* __res
     const uint32_t* d = dir + (uint64_t)x0 + (uint64_t)bx * ((uint64_t)y0 + (uint64_t)by * (uint64_t)z0) + lane;
     const bool in_x = x0 + lane < bx;
     uint32_t line = 0;
-#pragma unroll 8
-    for (int32_t j = 0; j < 32; ++j) {
-        const bool o = in_x && j < n && !brick_empty(__ldg(d + step * (uint64_t)j));
-        const uint32_t w = __ballot_sync(0xFFFFFFFFu, o);
-        if (lane == j) line = w;
+#pragma unroll
+    for (int32_t h = 0; h < 32; h += 16) {  // sixteen loads in flight
+        uint32_t e[16];
+#pragma unroll
+        for (int32_t j = 0; j < 16; ++j)
+            e[j] = in_x && h + j < n ? __ldg(d + step * (uint64_t)(h + j)) : kEmptyBit;
+#pragma unroll
+        for (int32_t j = 0; j < 16; ++j) {
+            const uint32_t w = __ballot_sync(0xFFFFFFFFu, !brick_empty(e[j]));
+            if (lane == h + j) line = w;
+        }
     }
     const uint32_t across = transpose32(line);
     const int32_t wx = row_words(bx), wy = row_words(by), wz = row_words(bz);

@@ -17,11 +17,18 @@
 //      recomputed for the bricks within 14 bricks of the affected ones (distances above 14, in grids
 //      that have any, within 31): a change cannot reach farther.
 //
+// Small boxes (a 16^3 or 32^3 chunk) take steps 1 to 4 in one block: the box is read from page-locked
+// memory, the slots are handed out on the device in the order the host would, and the host learns
+// what happened when it waits for the whole update.
+//
 // The grid afterwards traverses exactly as a grid built from the updated dense array (same
 // occupancy, payload, distances and octant words; only slot numbers may differ).
 #include <cuda_runtime.h>
 
+#include <string.h>
+
 #include <algorithm>
+#include <mutex>
 #include <vector>
 
 #include "vt_api_internal.h"
@@ -123,6 +130,190 @@ __global__ void __launch_bounds__(256) update_scatter_kernel(GridView g, UpdateB
     for (int i = 0; i < 64; ++i) out[i] = in[i];
 }
 
+// ---- small boxes: everything but the lattice passes in one block
+
+constexpr uint32_t kSmallBricks = 128;          // affected bricks: eight threads each
+constexpr size_t kSmallBoxBytes = 128u << 10;   // voxels of the box, in shared memory
+
+// Exchange area in page-locked memory.
+struct SmallExchange {
+    // in: slots to hand out first, in the order the host's free list gives them
+    uint32_t free_slots[kSmallBricks];
+    // out
+    uint32_t old_dir[kSmallBricks], now[kSmallBricks];
+    long long occ_delta;
+    uint32_t fresh, freed;
+    uint32_t grow;  // nothing was written: the slot arrays are too small
+    uint32_t deep;  // as LatticeScratch::deep
+    uint4 box[kSmallBoxBytes / 16];
+};
+
+struct SmallUpdate {
+    uint32_t nfree;       // entries of free_slots
+    uint32_t slots_used;  // then new slots from here
+    uint32_t slot_capacity;
+    uint32_t z_fastest;
+};
+
+// Bound by the latency of one block (a 16^3 chunk is 64 threads' work) and of its reads over the host
+// link: 14 us for a 16^3 u8 chunk, cold.  A chunk paged into the resident 1024^3 grid takes 57 us in
+// all against 110 us with an upload, the reorder, the merge, three copies back, a wait, the slots'
+// upload and the scatter around the same lattice passes.
+template <typename T>
+__global__ void __launch_bounds__(1024) update_small_kernel(GridView g, UpdateBox u, SmallUpdate p,
+                                                            SmallExchange* __restrict__ x,
+                                                            uint32_t* __restrict__ dir,
+                                                            uint64_t* __restrict__ masks,
+                                                            T* __restrict__ payload) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T* box = reinterpret_cast<T*>(smem_raw);
+    __shared__ uint32_t s_alpha[8];            // palette entries that are occupied, one bit each
+    __shared__ uint32_t s_fresh[4], s_freed[4];
+    __shared__ uint32_t s_slot[kSmallBricks], s_free[kSmallBricks];
+    __shared__ int s_delta;
+    const uint32_t K = (uint32_t)(u.kx * u.ky * u.kz), t = threadIdx.x, lane = t & 31u;
+    const uint32_t n16 = (uint32_t)(((size_t)u.w * u.h * u.d * sizeof(T) + 15) / 16);
+    for (uint32_t i = t; i < n16; i += blockDim.x) reinterpret_cast<uint4*>(smem_raw)[i] = x->box[i];
+    if (sizeof(T) == 1) {
+        for (uint32_t i = t; i < 256; i += blockDim.x) {
+            const uint32_t m = __ballot_sync(0xFFFFFFFFu, (g.palette[i] >> 24) != 0u);
+            if (lane == 0) s_alpha[i >> 5] = m;
+        }
+    }
+    if (t == 0) s_delta = 0;
+    __syncthreads();
+    // the slice of this thread: brick k, z-slice lz
+    const uint32_t k = t >> 3;
+    const int32_t lz = (int32_t)(t & 7u);
+    const bool active = k < K;
+    const int32_t bxi = u.bx0 + (int32_t)(k % (uint32_t)u.kx);
+    const int32_t byi = u.by0 + (int32_t)(k / (uint32_t)u.kx % (uint32_t)u.ky);
+    const int32_t bzi = u.bz0 + (int32_t)(k / (uint32_t)(u.kx * u.ky));
+    const size_t b = (size_t)bxi + (size_t)g.bx * ((size_t)byi + (size_t)g.by * bzi);
+    const uint32_t e = active ? dir[b] : kEmptyBit;
+    const bool was = !brick_empty(e);
+    const int32_t z = bzi * 8 + lz;
+    const bool z_in = z >= u.z0 && z < u.z0 + u.d;
+    const size_t ex = p.z_fastest ? (size_t)u.d * u.h : 1, ey = p.z_fastest ? (size_t)u.d : (size_t)u.w,
+                 ez = p.z_fastest ? 1 : (size_t)u.w * u.h;
+    // voxels of row ly after the update; false when the box does not touch the row
+    auto merged = [&](int32_t ly, T v[8]) {
+        const int32_t y = byi * 8 + ly;
+        const bool in = z_in && y >= u.y0 && y < u.y0 + u.h;
+        const T* old = payload + (size_t)(was ? e : 0u) * 512 + lz * 64 + ly * 8;
+#pragma unroll
+        for (int32_t lx = 0; lx < 8; ++lx) {
+            const int32_t vx = bxi * 8 + lx;
+            if (in && vx >= u.x0 && vx < u.x0 + u.w)
+                v[lx] = box[ex * (size_t)(vx - u.x0) + ey * (size_t)(y - u.y0) + ez * (size_t)(z - u.z0)];
+            else
+                v[lx] = was ? old[lx] : (T)0;
+        }
+        return in;
+    };
+    uint64_t word = 0, old_word = 0;
+    if (active) {
+        if (was) old_word = masks[(size_t)e * 8 + lz];
+        word = old_word;
+#pragma unroll 2
+        for (int32_t ly = 0; ly < 8; ++ly) {
+            T v[8];
+            if (!merged(ly, v)) continue;
+            uint32_t bits = 0;
+#pragma unroll
+            for (int32_t lx = 0; lx < 8; ++lx) {
+                const bool o = sizeof(T) == 1 ? (s_alpha[(uint32_t)v[lx] >> 5] >> ((uint32_t)v[lx] & 31u)) & 1u
+                                              : ((uint32_t)v[lx] >> 24) != 0u;
+                bits |= (uint32_t)o << lx;
+            }
+            word = (word & ~(0xFFull << (8 * ly))) | ((uint64_t)bits << (8 * ly));
+        }
+    }
+    const int delta = __reduce_add_sync(0xFFFFFFFFu, __popcll(word) - __popcll(old_word));
+    if (lane == 0 && delta) atomicAdd(&s_delta, delta);
+    // lanes 8j .. 8j + 7 hold one brick
+    uint32_t any = word != 0ull;
+#pragma unroll
+    for (int s = 1; s < 8; s <<= 1) any |= __shfl_xor_sync(0xFFFFFFFFu, any, s);
+    if (active && lz == 0) {
+        s_slot[k] = any ? 1u : 0u;
+        s_free[k] = e;
+        x->old_dir[k] = e;
+        x->now[k] = any ? 1u : 0u;
+    }
+    __syncthreads();
+    // ranks of the bricks that become occupied (fresh) and empty (freed), in brick order
+    const bool lists = t < ((K + 31u) & ~31u);  // whole warps
+    bool fresh = false, freed = false;
+    uint32_t e0 = kEmptyBit;
+    if (lists) {
+        if (t < K) e0 = s_free[t];
+        const bool w0 = !brick_empty(e0), n0 = t < K && s_slot[t] != 0u;
+        fresh = n0 && !w0;
+        freed = w0 && !n0;
+        const uint32_t mf = __ballot_sync(0xFFFFFFFFu, fresh), md = __ballot_sync(0xFFFFFFFFu, freed);
+        if (lane == 0) {
+            s_fresh[t >> 5] = mf;
+            s_freed[t >> 5] = md;
+        }
+    }
+    __syncthreads();
+    uint32_t rank_fresh = 0, rank_freed = 0, nfresh = 0, nfreed = 0;
+    for (uint32_t w = 0; w < (K + 31u) / 32u; ++w) {
+        const uint32_t below = w < (t >> 5) ? 0xFFFFFFFFu : (w == (t >> 5) ? (1u << lane) - 1u : 0u);
+        rank_fresh += __popc(s_fresh[w] & below);
+        rank_freed += __popc(s_freed[w] & below);
+        nfresh += __popc(s_fresh[w]);
+        nfreed += __popc(s_freed[w]);
+    }
+    const uint32_t reused = min(nfresh, nfreed + p.nfree);
+    const bool grow = p.slots_used + (nfresh - reused) > p.slot_capacity;
+    if (t == 0) {
+        x->fresh = nfresh;
+        x->freed = nfreed;
+        x->grow = grow ? 1u : 0u;
+        x->occ_delta = s_delta;
+    }
+    if (grow) return;  // block-uniform; nothing of the grid is written
+    uint32_t mine = kEmptyBit | 1u;  // distances follow
+    if (t < K) {
+        if (s_slot[t] != 0u && !fresh) mine = e0;
+        // the freed slots, in brick order, go to the end of the free list, which is used from its end
+        // (every old entry has been read before the last barrier)
+        if (freed) s_free[rank_freed] = e0;
+    }
+    __syncthreads();
+    if (t < K) {
+        if (fresh) {
+            const uint32_t r = rank_fresh;
+            mine = r < nfreed ? s_free[nfreed - 1u - r]
+                              : (r - nfreed < p.nfree ? x->free_slots[r - nfreed] : p.slots_used + (r - nfreed - p.nfree));
+        }
+        s_slot[t] = mine;
+    }
+    __syncthreads();
+    if (!active) return;
+    const uint32_t slot = s_slot[k];
+    if (lz == 0) dir[b] = slot;
+    if (brick_empty(slot)) return;
+    masks[(size_t)slot * 8 + lz] = word;
+    for (int32_t ly = 0; ly < 8; ++ly) {
+        T v[8];
+        if (!merged(ly, v) && was) continue;  // the row keeps its voxels in the same slot
+        T* out = payload + (size_t)slot * 512 + lz * 64 + ly * 8;
+        if (sizeof(T) == 1) {
+            uint2 q;
+            q.x = (uint32_t)v[0] | (uint32_t)v[1] << 8 | (uint32_t)v[2] << 16 | (uint32_t)v[3] << 24;
+            q.y = (uint32_t)v[4] | (uint32_t)v[5] << 8 | (uint32_t)v[6] << 16 | (uint32_t)v[7] << 24;
+            *reinterpret_cast<uint2*>(out) = q;
+        } else {
+            uint4* o4 = reinterpret_cast<uint4*>(out);
+            o4[0] = make_uint4((uint32_t)v[0], (uint32_t)v[1], (uint32_t)v[2], (uint32_t)v[3]);
+            o4[1] = make_uint4((uint32_t)v[4], (uint32_t)v[5], (uint32_t)v[6], (uint32_t)v[7]);
+        }
+    }
+}
+
 // Grows the slot arrays of `g` to at least `need` slots (doubling), copying the live ones.
 static int32_t grow_slots(Grid& g, uint64_t need, cudaStream_t st) {
     if (need <= g.slot_capacity) return VT_OK;
@@ -152,6 +343,78 @@ static int32_t grow_slots(Grid& g, uint64_t need, cudaStream_t st) {
     state().grid_epoch.fetch_add(1);  // the grid's device view changed
     g.slot_capacity = cap;
     return VT_OK;
+}
+
+// One small update.  The caller has checked the box; its grid is not read or written elsewhere.
+static int32_t update_small(Grid& g, const void* voxels, size_t elem, uint32_t order, const UpdateBox& u) {
+    State& S = state();
+    std::lock_guard<std::mutex> lk(S.update_mu);
+    if (!S.update_pin) {
+        if (cudaHostAlloc(&S.update_pin, sizeof(SmallExchange), cudaHostAllocMapped) != cudaSuccess ||
+            cudaHostGetDevicePointer(&S.update_pin_dev, S.update_pin, 0) != cudaSuccess) {
+            cudaGetLastError();
+            cudaFreeHost(S.update_pin);
+            S.update_pin = nullptr;
+            return fail(VT_ENOMEM, "vt_grid_update: page-locked exchange area");
+        }
+    }
+    SmallExchange* x = (SmallExchange*)S.update_pin;
+    SmallExchange* dx = (SmallExchange*)S.update_pin_dev;
+    cudaStream_t st = S.stream;
+    const int32_t bx = (int32_t)g.bx, by = (int32_t)g.by, bz = (int32_t)g.bz;
+    const uint32_t K = (uint32_t)(u.kx * u.ky * u.kz);
+    const BrickBox changed = {u.bx0, u.by0, u.bz0, u.kx, u.ky, u.kz};
+    const size_t bytes = (size_t)u.w * u.h * u.d * elem, smem = (bytes + 15) / 16 * 16;
+    memcpy(x->box, voxels, bytes);
+    const void* kernel = elem == 1 ? (const void*)update_small_kernel<uint8_t> : (const void*)update_small_kernel<uint32_t>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallBoxBytes);
+    void* scr = nullptr;
+    if (e == cudaSuccess) e = cudaMallocAsync(&scr, lattice_scratch_bytes(bx, by, bz), st);
+    if (e != cudaSuccess) return cuda_fail(e, "vt_grid_update: scratch");
+    LatticeScratch ls = carve_lattice_scratch(scr, bx, by, bz);
+    ls.deep = &dx->deep;
+    int32_t rc = VT_OK;
+    for (int attempt = 0;; ++attempt) {
+        SmallUpdate p;
+        p.nfree = (uint32_t)std::min<size_t>(g.free_slots.size(), K);
+        for (uint32_t i = 0; i < p.nfree; ++i) x->free_slots[i] = g.free_slots[g.free_slots.size() - 1 - i];
+        p.slots_used = (uint32_t)g.slots_used;
+        p.slot_capacity = (uint32_t)std::min<uint64_t>(g.slot_capacity, 0x7FFFFFFFu);
+        p.z_fastest = order == VT_ORDER_Z_FASTEST ? 1u : 0u;
+        const unsigned threads = std::max(256u, (K * 8 + 31) / 32 * 32);
+        if (elem == 1)
+            update_small_kernel<uint8_t><<<1, threads, smem, st>>>(g.view(), u, p, dx, g.dir, g.masks, (uint8_t*)g.payload);
+        else
+            update_small_kernel<uint32_t><<<1, threads, smem, st>>>(g.view(), u, p, dx, g.dir, g.masks, (uint32_t*)g.payload);
+        e = cudaGetLastError();
+        if (e == cudaSuccess) e = launch_brick_lattice(g.dir, g.oct, g.lng, ls, bx, by, bz, st, &changed);
+        if (e == cudaSuccess && g.deep) e = launch_brick_distance(g.dir, g.oct, ls, bx, by, bz, st, &changed);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        if (e != cudaSuccess) { rc = cuda_fail(e, "vt_grid_update"); break; }
+        if (!x->grow) break;
+        if (attempt) { rc = fail(VT_ECUDA, "vt_grid_update: slots"); break; }  // not reached: grown for it
+        const uint64_t reused = std::min<uint64_t>(x->fresh, x->freed + g.free_slots.size());
+        if ((rc = grow_slots(g, g.slots_used + (x->fresh - reused), st))) break;
+    }
+    if (rc == VT_OK && !g.deep && x->deep) {
+        g.deep = true;
+        e = launch_brick_distance(g.dir, g.oct, ls, bx, by, bz, st, &changed);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        if (e != cudaSuccess) rc = cuda_fail(e, "vt_grid_update: distances");
+    }
+    if (rc == VT_OK) {
+        // the free list as the device used it: this update's freed slots behind the others, both from
+        // the end
+        for (uint32_t k = 0; k < K; ++k)
+            if (!(x->old_dir[k] & kEmptyBit) && !x->now[k]) g.free_slots.push_back(x->old_dir[k]);
+        const uint64_t reused = std::min<uint64_t>(x->fresh, g.free_slots.size());
+        g.free_slots.resize(g.free_slots.size() - reused);
+        g.slots_used += x->fresh - reused;
+        g.nonempty += (uint64_t)x->fresh - x->freed;  // modular: a net decrease wraps back
+        g.occupied = (uint64_t)((long long)g.occupied + x->occ_delta);
+    }
+    cudaFreeAsync(scr, st);
+    return rc;
 }
 
 }  // namespace vt
@@ -188,6 +451,7 @@ extern "C" int32_t vt_grid_update(int32_t grid, const void* voxels, uint32_t ord
     u.kz = ((u.z0 + u.d - 1) >> 3) - u.bz0 + 1;
     const uint64_t K = (uint64_t)u.kx * u.ky * u.kz;
     const size_t box = (size_t)w * h * d * elem;
+    if (K <= kSmallBricks && box <= kSmallBoxBytes) return update_small(*g, voxels, elem, order, u);
     auto al = [](size_t v) { return (v + 255) / 256 * 256; };
     // scratch: box (x2 for reordering), words, payloads, flags, old entries, slots, delta, lattice
     // passes
