@@ -201,8 +201,8 @@ static void point_into_block(Grid& g, void* block, const BlockLayout& L, uint64_
     g.slot_capacity = slots;
 }
 
-// The brick build's launches on `stream` (captured or not): occupancy words, slot scan, compaction
-// into dir / masks / payload, distance field, octant words, long-box words.
+// The brick build's launches on `stream` (captured): occupancy words, slot scan, compaction into dir /
+// masks / payload, octant words, long-box words and distances below 15.
 static cudaError_t build_launches(const void* d_src, uint32_t format, const uint32_t* d_palette,
                                   bool nonzero, const Grid& g, const BuildScratch& s,
                                   cudaStream_t stream) {
@@ -213,17 +213,17 @@ static cudaError_t build_launches(const void* d_src, uint32_t format, const uint
         e = launch_brick_compact(d_src, format, nx, ny, nz, s, g.dir, g.masks, g.payload, stream);
     const int32_t bx = (int32_t)g.bx, by = (int32_t)g.by, bz = (int32_t)g.bz;
     if (e == cudaSuccess) e = launch_brick_lattice(g.dir, g.oct, g.lng, s.lattice, bx, by, bz, stream);
-    if (e == cudaSuccess)
-        e = launch_brick_distance(g.dir, g.oct, s.lattice, bx, by, bz, stream, nullptr, true);
     return e;
 }
 
 // ---------------------------------------------------------------------------------------------
-// Small grids (vtrace's 16^3 chunk textures, .vox models): the build's twenty-odd launches cost
-// more than their work, so they are captured once per grid shape into a CUDA graph that reads a
-// fixed input buffer and builds into a fixed template of the grid's allocation (every brick has a
-// slot).  A build copies its voxels in, replays the graph, and copies the template into the new
-// grid's allocation.  Builds of small grids are serialised by g_small_mu.
+// Small grids.  Up to 64 bricks (vtrace's 16^3 chunk textures): one block builds everything but the
+// lattice tables, straight into the grid's allocation, from a page-locked exchange area that the host
+// copies the voxels to (or from device memory).  Up to 512 (.vox models): the build's launches are
+// captured once per grid shape into a CUDA graph that reads a fixed input buffer and builds into a
+// fixed template of the grid's allocation (every brick has a slot); a build copies its voxels in,
+// replays the graph, and copies the template into the new grid's allocation.  Builds of small grids are
+// serialised by g_small_mu.
 // ---------------------------------------------------------------------------------------------
 constexpr uint64_t kSmallGridBricks = 512;  // 64^3 voxels: at most 1 MiB of unused slots
 constexpr size_t kSmallGraphs = 64;
@@ -238,6 +238,19 @@ struct SmallBuild {
     cudaGraphExec_t exec = nullptr;
     uint64_t last_use = 0;
 };
+
+// Page-locked exchange area of chunk builds, and their lattice passes' scratch (device).
+struct ChunkExchange {
+    unsigned long long counts[2];
+    uint32_t deep, pad[3];
+    uint32_t palette[256];
+    uint4 voxels[kChunkBricks * 512 * 4 / 16];
+};
+static ChunkExchange* g_chunk = nullptr;
+static ChunkExchange* g_chunk_dev = nullptr;
+static void* g_chunk_scratch = nullptr;
+// at most three words of occupancy bits per brick, and padding
+constexpr size_t kChunkScratchBytes = 4096;
 
 static std::mutex g_small_mu;
 static std::vector<SmallBuild> g_small;
@@ -256,6 +269,52 @@ void release_small_builds() {
     std::lock_guard<std::mutex> lk(g_small_mu);
     for (SmallBuild& b : g_small) small_free(b);
     g_small.clear();
+    cudaFreeHost(g_chunk);
+    cudaFree(g_chunk_scratch);
+    g_chunk = g_chunk_dev = nullptr;
+    g_chunk_scratch = nullptr;
+}
+
+// A grid of up to kChunkBricks bricks.  `src`: the dense voxels in the order given, in device memory,
+// or in host memory when `src_host`.  `g` has its allocation.
+static int32_t build_chunk(const void* src, bool src_host, uint32_t order, const uint32_t* palette_host,
+                           Grid& g, cudaStream_t stream) {
+    if (!g_chunk) {
+        void *h = nullptr, *d = nullptr, *scratch = nullptr;
+        if (cudaHostAlloc(&h, sizeof(ChunkExchange), cudaHostAllocMapped) != cudaSuccess ||
+            cudaHostGetDevicePointer(&d, h, 0) != cudaSuccess ||
+            cudaMalloc(&scratch, kChunkScratchBytes) != cudaSuccess) {
+            cudaGetLastError();
+            cudaFreeHost(h);
+            return fail(VT_ENOMEM, "chunk build exchange area");
+        }
+        g_chunk = (ChunkExchange*)h;
+        g_chunk_dev = (ChunkExchange*)d;
+        g_chunk_scratch = scratch;
+    }
+    const int32_t bx = (int32_t)g.bx, by = (int32_t)g.by, bz = (int32_t)g.bz;
+    static_assert(kChunkBricks * 13 + 128 <= kChunkScratchBytes, "lattice scratch of a chunk");
+    if (src_host) memcpy(g_chunk->voxels, src, (size_t)g.nx * g.ny * g.nz * (g.format == VT_PAYLOAD_U8 ? 1 : 4));
+    if (g.format == VT_PAYLOAD_U8) memcpy(g_chunk->palette, palette_host, 1024);
+    LatticeScratch ls = carve_lattice_scratch(g_chunk_scratch, bx, by, bz);
+    ls.deep = &g_chunk_dev->deep;
+    cudaError_t e = launch_build_chunk(src_host ? (const void*)g_chunk_dev->voxels : src, g.format,
+                                       order == VT_ORDER_Z_FASTEST, g_chunk_dev->palette, (int32_t)g.nx,
+                                       (int32_t)g.ny, (int32_t)g.nz, g.palette, g.dir, g.masks, g.payload,
+                                       g_chunk_dev->counts, stream);
+    if (e == cudaSuccess) e = launch_brick_lattice(g.dir, g.oct, g.lng, ls, bx, by, bz, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    if (e == cudaSuccess && g_chunk->deep) {
+        g.deep = true;
+        e = launch_brick_distance(g.dir, g.oct, ls, bx, by, bz, stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    }
+    if (e != cudaSuccess) return cuda_fail(e, "chunk build");
+    g.occupied = g_chunk->counts[0];
+    g.nonempty = g_chunk->counts[1];
+    g.bytes = g.block_bytes;
+    g.slots_used = g.nonempty;
+    return VT_OK;
 }
 
 static int32_t small_entry(const Grid& shape, bool nonzero, SmallBuild*& out) {
@@ -329,14 +388,11 @@ static int32_t small_entry(const Grid& shape, bool nonzero, SmallBuild*& out) {
     return VT_OK;
 }
 
-// `src`: the dense voxels, in device memory, or in host memory when `src_host`.
-static int32_t build_small(const void* src, bool src_host, const uint32_t* palette_host,
+// `src`: the dense voxels, in device memory, or in host memory when `src_host`; x fastest unless the
+// grid has at most kChunkBricks bricks.
+static int32_t build_small(const void* src, bool src_host, uint32_t order, const uint32_t* palette_host,
                            bool nonzero, std::unique_ptr<Grid>& g, cudaStream_t stream) {
     std::lock_guard<std::mutex> lk(g_small_mu);
-    SmallBuild* b = nullptr;
-    int32_t rc = small_entry(*g, nonzero, b);
-    if (rc) return rc;
-    b->last_use = ++g_small_clock;
     const size_t elem = g->format == VT_PAYLOAD_U8 ? 1 : 4;
     const BlockLayout L = block_layout(g->bricks, g->bricks, g->format);
     // small blocks come from the stream-ordered pool (freed after a device synchronisation, like
@@ -348,6 +404,11 @@ static int32_t build_small(const void* src, bool src_host, const uint32_t* palet
     }
     point_into_block(*g, block, L, g->bricks);
     g->pooled = true;
+    if (g->bricks <= kChunkBricks) return build_chunk(src, src_host, order, palette_host, *g, stream);
+    SmallBuild* b = nullptr;
+    int32_t rc = small_entry(*g, nonzero, b);
+    if (rc) return rc;
+    b->last_use = ++g_small_clock;
     uint32_t hc[5] = {0, 0, 0, 0, 0};
     cudaError_t e = cudaMemcpyAsync(b->in, src, (size_t)g->nx * g->ny * g->nz * elem,
                                     src_host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice,
@@ -359,10 +420,16 @@ static int32_t build_small(const void* src, bool src_host, const uint32_t* palet
     if (e == cudaSuccess) e = cudaMemcpyAsync(block, b->tmpl, L.total, cudaMemcpyDeviceToDevice, stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(hc, b->counts, 20, cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    if (e == cudaSuccess && hc[4]) {  // bricks far from all occupied ones: settle their distances
+        g->deep = true;
+        const int32_t bx = (int32_t)g->bx, by = (int32_t)g->by, bz = (int32_t)g->bz;
+        const BuildScratch s = carve_build_scratch(b->scratch, bx, by, bz);
+        e = launch_brick_distance(g->dir, g->oct, s.lattice, bx, by, bz, stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    }
     if (e != cudaSuccess) return cuda_fail(e, "small grid build");
     g->nonempty = (uint64_t)hc[2] | ((uint64_t)hc[3] << 32);
     g->occupied = (uint64_t)hc[0] | ((uint64_t)hc[1] << 32);
-    g->deep = hc[4] != 0u;
     g->bytes = g->block_bytes;
     g->slots_used = g->nonempty;
     return VT_OK;
@@ -388,16 +455,16 @@ static bool nonzero_palette(uint32_t format, const uint32_t* palette_host) {
     return nonzero;
 }
 
-static bool small_grid(uint32_t nx, uint32_t ny, uint32_t nz) {
-    return (uint64_t)((nx + 7) / 8) * ((ny + 7) / 8) * ((nz + 7) / 8) <= kSmallGridBricks;
+static uint64_t brick_count(uint32_t nx, uint32_t ny, uint32_t nz) {
+    return (uint64_t)((nx + 7) / 8) * ((ny + 7) / 8) * ((nz + 7) / 8);
 }
 
-static int32_t build_small_from_host(const void* voxels, uint32_t format,
+static int32_t build_small_from_host(const void* voxels, uint32_t format, uint32_t order,
                                      const uint32_t* palette_host, uint32_t nx, uint32_t ny,
                                      uint32_t nz, cudaStream_t stream, std::unique_ptr<Grid>& out) {
     std::unique_ptr<Grid> g = grid_shell(format, nx, ny, nz);
-    const int32_t rc = build_small(voxels, true, palette_host, nonzero_palette(format, palette_host),
-                                   g, stream);
+    const int32_t rc = build_small(voxels, true, order, palette_host,
+                                   nonzero_palette(format, palette_host), g, stream);
     if (rc) {
         g->release();
         return rc;
@@ -414,7 +481,7 @@ int32_t build_grid(const void* d_src, uint32_t format, const uint32_t* palette_h
     const bool nonzero = nonzero_palette(format, palette_host);
     int32_t rc = VT_OK;
     if (g->bricks <= kSmallGridBricks) {
-        if ((rc = build_small(d_src, false, palette_host, nonzero, g, stream))) {
+        if ((rc = build_small(d_src, false, VT_ORDER_X_FASTEST, palette_host, nonzero, g, stream))) {
             g->release();
             return rc;
         }
@@ -731,9 +798,11 @@ static int32_t create_from_host(const void* data, size_t elem, uint32_t format, 
     const size_t bytes = (size_t)nx * ny * nz * elem;
     const int nbuf = order == VT_ORDER_Z_FASTEST ? 2 : 1;
     cudaStream_t st = state().stream;
-    if (order == VT_ORDER_X_FASTEST && small_grid(nx, ny, nz)) {  // straight into the build graph's input
+    const uint64_t bricks = brick_count(nx, ny, nz);
+    if (bricks <= kChunkBricks || (order == VT_ORDER_X_FASTEST && bricks <= kSmallGridBricks)) {
+        // straight into the small build's input
         std::unique_ptr<Grid> g;
-        if ((rc = build_small_from_host(data, format, palette, nx, ny, nz, st, g))) return rc;
+        if ((rc = build_small_from_host(data, format, order, palette, nx, ny, nz, st, g))) return rc;
         return register_grid(std::move(g));
     }
     void* d = nullptr;

@@ -264,12 +264,14 @@ __global__ void __launch_bounds__(256) brick_words_kernel(const void* __restrict
 }
 
 // Exclusive scan of up to kScanBlock items per block, of their bit counts with BITS; block totals go
-// to `sums`.
+// to `sums`.  `zero` (single-block launches): a word to clear.
 template <bool BITS>
 __global__ void __launch_bounds__(kScanThreads) scan_block_kernel(const uint32_t* __restrict__ in,
                                                                   uint32_t* __restrict__ out,
                                                                   uint64_t n,
-                                                                  uint32_t* __restrict__ sums) {
+                                                                  uint32_t* __restrict__ sums,
+                                                                  uint32_t* __restrict__ zero) {
+    if (zero && threadIdx.x == 0) *zero = 0u;
     __shared__ uint32_t warp_tot[kScanThreads / 32];
     const uint64_t base = (uint64_t)blockIdx.x * kScanBlock + (uint64_t)threadIdx.x * kScanItems;
     uint32_t v[kScanItems], local = 0;
@@ -312,13 +314,16 @@ __global__ void scan_add_kernel(uint32_t* __restrict__ out, uint64_t n,
     if (i < n) out[i] += block_offsets[i / kScanBlock];
 }
 
-// In-place exclusive scan of `n` block totals; `next` holds the totals one level up.
-static cudaError_t scan_totals(uint32_t* sums, uint64_t n, uint32_t* next, cudaStream_t stream) {
+// In-place exclusive scan of `n` block totals; `next` holds the totals one level up, `total` takes
+// the sum of them all.
+static cudaError_t scan_totals(uint32_t* sums, uint64_t n, uint32_t* next, uint32_t* total,
+                               cudaStream_t stream) {
     const uint64_t blocks = (n + kScanBlock - 1) / kScanBlock;
-    scan_block_kernel<false><<<(unsigned)blocks, kScanThreads, 0, stream>>>(sums, sums, n, next);
+    scan_block_kernel<false><<<(unsigned)blocks, kScanThreads, 0, stream>>>(
+        sums, sums, n, blocks == 1 ? total : next, nullptr);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || blocks == 1) return e;
-    e = scan_totals(next, blocks, next + align_up(blocks, 64), stream);
+    e = scan_totals(next, blocks, next + align_up(blocks, 64), total, stream);
     if (e != cudaSuccess) return e;
     scan_add_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(sums, n, next);
     return cudaGetLastError();
@@ -329,23 +334,18 @@ __device__ __forceinline__ uint32_t first_slot(const uint32_t* offsets, const ui
     return __ldg(offsets + w) + __ldg(block_sums + w / kScanBlock);
 }
 
-// counts[1] = occupied bricks (counts[0], the occupied voxels, is summed by the words pass).
-__global__ void brick_count_kernel(const uint32_t* __restrict__ occ, const uint32_t* __restrict__ offsets,
-                                   const uint32_t* __restrict__ block_sums, uint64_t n,
-                                   unsigned long long* __restrict__ counts) {
-    counts[1] = (unsigned long long)first_slot(offsets, block_sums, n - 1) + (uint32_t)__popc(occ[n - 1]);
-}
-
 cudaError_t launch_brick_scan(const BuildScratch& s, uint64_t bricks, cudaStream_t stream) {
     // the totals of the lowest level are scanned in place; the compaction adds them to its words'
-    // offsets as it reads them
+    // offsets as it reads them.  counts[1] = occupied bricks: below 2^31, its low word (the words
+    // pass clears both counts).
     const uint64_t n = occ_count(bricks), blocks = (n + kScanBlock - 1) / kScanBlock;
-    scan_block_kernel<true><<<(unsigned)blocks, kScanThreads, 0, stream>>>(s.occ, s.offsets, n, s.block_sums);
+    uint32_t* total = (uint32_t*)(s.counts + 1);
+    scan_block_kernel<true><<<(unsigned)blocks, kScanThreads, 0, stream>>>(
+        s.occ, s.offsets, n, blocks == 1 ? total : s.block_sums, blocks == 1 ? s.block_sums : nullptr);
     cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = scan_totals(s.block_sums, blocks, s.block_sums + align_up(blocks, 64), stream);
-    if (e != cudaSuccess) return e;
-    brick_count_kernel<<<1, 1, 0, stream>>>(s.occ, s.offsets, s.block_sums, n, s.counts);
-    return cudaGetLastError();
+    if (e == cudaSuccess && blocks > 1)
+        e = scan_totals(s.block_sums, blocks, s.block_sums + align_up(blocks, 64), total, stream);
+    return e;
 }
 
 cudaError_t launch_brick_words(const void* src, uint32_t format, const uint32_t* d_palette,
@@ -354,7 +354,7 @@ cudaError_t launch_brick_words(const void* src, uint32_t format, const uint32_t*
     const int32_t bx = (nx + 7) / 8, by = (ny + 7) / 8, bz = (nz + 7) / 8;
     const uint64_t bricks = (uint64_t)bx * by * bz;
     const unsigned blocks = (unsigned)occ_count(bricks);
-    cudaError_t e = cudaMemsetAsync(s.counts, 0, sizeof(unsigned long long), stream);
+    cudaError_t e = cudaMemsetAsync(s.counts, 0, 2 * sizeof(unsigned long long), stream);
     if (e != cudaSuccess) return e;
     if (format == VT_PAYLOAD_U8 && nonzero_occupancy)
         brick_words_kernel<VT_PAYLOAD_U8, true><<<blocks, 256, 0, stream>>>(
@@ -430,6 +430,123 @@ cudaError_t launch_brick_compact(const void* src, uint32_t format, int32_t nx, i
         brick_compact_kernel<VT_PAYLOAD_RGBA8><<<blocks, 256, 0, stream>>>(
             src, nx, ny, nz, bx, by, bricks, s.words, s.occ, s.offsets, s.block_sums, dir, masks, payload,
             s.staged);
+    return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------------------------
+// Chunk textures (up to 64 bricks: vtrace's 16^3 chunks, 32^3): words, slots, masks, payloads and
+// directory in one block, a thread per row of eight voxels, from a dense array in either order that is
+// read once into shared memory.  Bound by the latency of one block and of its reads (page-locked host
+// memory or device memory): 7.3 us for a 16^3 RGBA8 chunk, cold (12 with a thread per slice), where the
+// words, scan, count and compaction kernels took 22 and the graph also copied its input and a template.
+// ---------------------------------------------------------------------------------------------
+constexpr uint32_t kChunkThreads = 512;
+
+template <uint32_t FMT>
+__global__ void __launch_bounds__(kChunkThreads) build_chunk_kernel(
+    const void* __restrict__ src, uint32_t z_fastest, const uint32_t* __restrict__ palette, int32_t nx,
+    int32_t ny, int32_t nz, int32_t bx, int32_t by, uint32_t bricks, uint32_t* __restrict__ pal_out,
+    uint32_t* __restrict__ dir, uint64_t* __restrict__ masks, void* __restrict__ payload,
+    unsigned long long* __restrict__ counts) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr size_t E = FMT == VT_PAYLOAD_RGBA8 ? 4 : 1;
+    __shared__ uint32_t s_alpha[8];
+    __shared__ uint32_t s_any[kChunkBricks / 32];  // bricks with an occupied voxel
+    __shared__ uint32_t s_count;
+    __shared__ uint8_t s_bits[kChunkBricks * 64];  // occupancy of each row
+    const uint32_t t = threadIdx.x, lane = t & 31u;
+    const size_t bytes = (size_t)nx * ny * nz * E, vec = ((uintptr_t)src & 15u) == 0 ? bytes / 16 : 0;
+    for (size_t i = t; i < vec; i += kChunkThreads)
+        reinterpret_cast<uint4*>(smem_raw)[i] = reinterpret_cast<const uint4*>(src)[i];
+    for (size_t i = vec * 16 + t; i < bytes; i += kChunkThreads) smem_raw[i] = ((const unsigned char*)src)[i];
+    if (FMT == VT_PAYLOAD_U8 && t < 256) {
+        const uint32_t c = palette[t];
+        pal_out[t] = c;
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, (c >> 24) != 0u);
+        if (lane == 0) s_alpha[t >> 5] = m;
+    }
+    if (t < kChunkBricks / 32) s_any[t] = 0u;
+    if (t == 0) s_count = 0u;
+    __syncthreads();
+    const int32_t ex = z_fastest ? nz * ny : 1, ey = z_fastest ? nz : nx, ez = z_fastest ? 1 : nx * ny;
+    // row r: brick r >> 6, z-slice (r >> 3) & 7, y r & 7; voxels past the grid's edge are 0
+    auto row = [&](uint32_t r, uint32_t v[8]) -> int32_t {  // number of its voxels inside the grid
+        const BrickCoord c = brick_coord(r >> 6, bx, by);
+        const int32_t x0 = c.bxi * 8, y = c.byi * 8 + (int32_t)(r & 7u), z = c.bzi * 8 + (int32_t)((r >> 3) & 7u);
+        const int32_t n = y < ny && z < nz ? min(8, nx - x0) : 0;
+        const int32_t at = ex * x0 + ey * y + ez * z;  // at most 32768 voxels
+#pragma unroll
+        for (int32_t k = 0; k < 8; ++k)
+            v[k] = k < n ? (FMT == VT_PAYLOAD_U8 ? (uint32_t)smem_raw[at + k * ex]
+                                                 : reinterpret_cast<const uint32_t*>(smem_raw)[at + k * ex])
+                         : 0u;
+        return n;
+    };
+    const uint32_t rows = bricks * 64;
+    for (uint32_t r = t; r < rows; r += kChunkThreads) {  // whole warps: half a brick each
+        uint32_t v[8], bits = 0;
+        const int32_t n = row(r, v);
+#pragma unroll
+        for (int32_t k = 0; k < 8; ++k) {
+            const bool o = FMT == VT_PAYLOAD_U8 ? k < n && ((s_alpha[v[k] >> 5] >> (v[k] & 31u)) & 1u) : (v[k] >> 24) != 0u;
+            bits |= (uint32_t)o << k;
+        }
+        s_bits[r] = (uint8_t)bits;
+        const uint32_t count = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)__popc(bits));
+        if (lane == 0 && count) {
+            atomicOr(&s_any[r >> 11], 1u << ((r >> 6) & 31u));
+            atomicAdd(&s_count, count);
+        }
+    }
+    __syncthreads();
+    if (t == 0) {
+        uint32_t total = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < kChunkBricks / 32; ++w) total += __popc(s_any[w]);
+        counts[0] = s_count;
+        counts[1] = total;
+    }
+    for (uint32_t r = t; r < rows; r += kChunkThreads) {
+        const uint32_t k = r >> 6, in = r & 63u;
+        uint32_t slot = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < kChunkBricks / 32; ++w)
+            slot += __popc(w < (k >> 5) ? s_any[w] : (w == (k >> 5) ? s_any[w] & ((1u << (k & 31u)) - 1u) : 0u));
+        const bool full = (s_any[k >> 5] >> (k & 31u)) & 1u;
+        if (in == 0) dir[k] = full ? slot : kEmptyBit;  // distance filled in by the lattice passes
+        if (!full) continue;
+        ((uint8_t*)masks)[(size_t)slot * 64 + in] = s_bits[r];
+        uint32_t v[8];
+        row(r, v);
+        if (FMT == VT_PAYLOAD_U8) {
+            ((uint2*)payload)[(size_t)slot * 64 + in] = make_uint2(v[0] | v[1] << 8 | v[2] << 16 | v[3] << 24,
+                                                                   v[4] | v[5] << 8 | v[6] << 16 | v[7] << 24);
+        } else {
+            uint4* out = (uint4*)payload + ((size_t)slot * 64 + in) * 2;
+            out[0] = make_uint4(v[0], v[1], v[2], v[3]);
+            out[1] = make_uint4(v[4], v[5], v[6], v[7]);
+        }
+    }
+}
+
+cudaError_t launch_build_chunk(const void* src, uint32_t format, bool z_fastest, const uint32_t* palette,
+                               int32_t nx, int32_t ny, int32_t nz, uint32_t* pal_out, uint32_t* dir,
+                               uint64_t* masks, void* payload, unsigned long long* counts,
+                               cudaStream_t stream) {
+    const int32_t bx = (nx + 7) / 8, by = (ny + 7) / 8, bz = (nz + 7) / 8;
+    const uint32_t bricks = (uint32_t)(bx * by * bz);
+    const size_t elem = format == VT_PAYLOAD_U8 ? 1 : 4, smem = (size_t)nx * ny * nz * elem;
+    const void* kernel = format == VT_PAYLOAD_U8 ? (const void*)build_chunk_kernel<VT_PAYLOAD_U8>
+                                                 : (const void*)build_chunk_kernel<VT_PAYLOAD_RGBA8>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(kChunkBricks * 512 * elem));
+    if (e != cudaSuccess) return e;
+    if (format == VT_PAYLOAD_U8)
+        build_chunk_kernel<VT_PAYLOAD_U8><<<1, kChunkThreads, smem, stream>>>(
+            src, z_fastest, palette, nx, ny, nz, bx, by, bricks, pal_out, dir, masks, payload, counts);
+    else
+        build_chunk_kernel<VT_PAYLOAD_RGBA8><<<1, kChunkThreads, smem, stream>>>(
+            src, z_fastest, palette, nx, ny, nz, bx, by, bricks, pal_out, dir, masks, payload, counts);
     return cudaGetLastError();
 }
 

@@ -98,6 +98,15 @@ cudaError_t launch_brick_compact(const void* src, uint32_t format, int32_t nx, i
                                  int32_t nz, const BuildScratch& s, uint32_t* dir,
                                  uint64_t* masks, void* payload, cudaStream_t stream);
 
+// Words, slots, masks, payloads, directory and palette of a grid of up to kChunkBricks bricks in one
+// block.  `src` (either element order), `palette` and `counts` (occupied voxels, occupied bricks) are
+// device-addressable; the lattice passes follow.
+constexpr uint32_t kChunkBricks = 64;
+cudaError_t launch_build_chunk(const void* src, uint32_t format, bool z_fastest, const uint32_t* palette,
+                               int32_t nx, int32_t ny, int32_t nz, uint32_t* pal_out, uint32_t* dir,
+                               uint64_t* masks, void* payload, unsigned long long* counts,
+                               cudaStream_t stream);
+
 // Phase 4: octant words, long-box words and the distances below 15 of empty bricks, for every
 // brick or (changed != nullptr) for the bricks a change of occupancy inside `changed` can affect.
 // *s.deep tells afterwards whether a brick of those has no occupied brick within 14: its directory
@@ -107,9 +116,9 @@ cudaError_t launch_brick_lattice(uint32_t* dir, uint32_t* oct, uint32_t* lng,
                                  cudaStream_t stream, const BrickBox* changed = nullptr);
 // Phase 5: distances (up to 31) of the bricks whose octant word is at the cap in all octants, after
 // launch_brick_lattice on the same scratch, or of every empty brick (oct == nullptr: no lattice pass
-// before).  With only_if_deep the kernels return at once unless *s.deep is set (not with `changed`).
+// before).
 cudaError_t launch_brick_distance(uint32_t* dir, const uint32_t* oct, const LatticeScratch& s,
                                   int32_t bx, int32_t by, int32_t bz, cudaStream_t stream,
-                                  const BrickBox* changed = nullptr, bool only_if_deep = false);
+                                  const BrickBox* changed = nullptr);
 
 }  // namespace vt

@@ -15,7 +15,7 @@
 // and the centred cube of radius r < 15 is the union of the eight octants' cubes of side r + 1, so
 //   D         = the smallest K of the eight octants when that is below 15
 // Bricks whose eight octants all reach the cap (empty in all directions for 15 bricks) are left to
-// the separable distance passes at the end of this file, which run only when there are any.
+// the separable distance passes at the end of this file, which the host launches when there are any.
 //
 // A block takes 32 bricks along the axis x 8 x 8 rows.  It reads the 36 x 36 rows within reach as
 // 62-bit windows, builds the ORs of 2^p x 2^p rows (p = 0..3) in shared memory, from which M(k, q)
@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(kLatticeThreads) lattice_yz_kernel(
 // separable transform.  Pass xy takes, per brick, the minimum over rows y' of max(|y' - y|, distance
 // along x in row y') from the x rows (two word reads and a find-first-set per side); pass z the
 // minimum over z' of max(|z' - z|, pass xy).  Both walk outward and stop once the offset reaches the
-// best value found.  They return at once when `deep` is given and no brick set it.
+// best value found.
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ bool box_brick(const BrickBox& box, int32_t bx, int32_t by, int32_t& x,
                                           int32_t& y, int32_t& z, uint64_t& b) {
@@ -370,9 +370,7 @@ __device__ __forceinline__ int32_t row_distance(const uint32_t* __restrict__ row
 __global__ void __launch_bounds__(256) lattice_distance_xy_kernel(const uint32_t* __restrict__ rows,
                                                                   uint8_t* __restrict__ out,
                                                                   int32_t bx, int32_t by,
-                                                                  BrickBox box,
-                                                                  const uint32_t* __restrict__ deep) {
-    if (deep && *deep == 0u) return;
+                                                                  BrickBox box) {
     int32_t x, y, z;
     uint64_t b;
     if (!box_brick(box, bx, by, x, y, z, b)) return;
@@ -390,9 +388,7 @@ __global__ void __launch_bounds__(256) lattice_distance_z_kernel(uint32_t* __res
                                                                  const uint32_t* __restrict__ oct,
                                                                  const uint8_t* __restrict__ in,
                                                                  int32_t bx, int32_t by, int32_t bz,
-                                                                 BrickBox box,
-                                                                 const uint32_t* __restrict__ deep) {
-    if (deep && *deep == 0u) return;
+                                                                 BrickBox box) {
     int32_t x, y, z;
     uint64_t b;
     if (!box_brick(box, bx, by, x, y, z, b)) return;
@@ -494,7 +490,7 @@ cudaError_t launch_brick_lattice(uint32_t* dir, uint32_t* oct, uint32_t* lng,
 
 cudaError_t launch_brick_distance(uint32_t* dir, const uint32_t* oct, const LatticeScratch& s,
                                   int32_t bx, int32_t by, int32_t bz, cudaStream_t stream,
-                                  const BrickBox* changed, bool only_if_deep) {
+                                  const BrickBox* changed) {
     // distances change only within 31 bricks of a change; pass z reads pass xy up to 31 bricks away
     // along z, which reads the x rows up to 31 away along y
     const int32_t R = (int32_t)kMaxBrickDistance;
@@ -503,10 +499,9 @@ cudaError_t launch_brick_distance(uint32_t* dir, const uint32_t* oct, const Latt
     const BrickBox w1 = grow(w, 0, 0, R, bx, by, bz);
     if (!oct || changed)  // the rows of launch_brick_lattice reach less far
         launch_rows(dir, s, bx, by, bz, grow(w1, R, R, 0, bx, by, bz), stream);
-    const uint32_t* deep = only_if_deep ? s.deep : nullptr;
     auto blocks = [](const BrickBox& b) { return (unsigned)(((uint64_t)b.nx * b.ny * b.nz + 255) / 256); };
-    lattice_distance_xy_kernel<<<blocks(w1), 256, 0, stream>>>(s.rows[0], s.dist, bx, by, w1, deep);
-    lattice_distance_z_kernel<<<blocks(w), 256, 0, stream>>>(dir, oct, s.dist, bx, by, bz, w, deep);
+    lattice_distance_xy_kernel<<<blocks(w1), 256, 0, stream>>>(s.rows[0], s.dist, bx, by, w1);
+    lattice_distance_z_kernel<<<blocks(w), 256, 0, stream>>>(dir, oct, s.dist, bx, by, bz, w);
     return cudaGetLastError();
 }
 

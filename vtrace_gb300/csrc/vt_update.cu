@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(256) update_scatter_kernel(GridView g, UpdateB
 
 // ---- small boxes: everything but the lattice passes in one block
 
-constexpr uint32_t kSmallBricks = 128;          // affected bricks: eight threads each
+constexpr uint32_t kSmallBricks = 128;          // affected bricks
 constexpr size_t kSmallBoxBytes = 128u << 10;   // voxels of the box, in shared memory
 
 // Exchange area in page-locked memory.
@@ -155,8 +155,8 @@ struct SmallUpdate {
     uint32_t z_fastest;
 };
 
-// Bound by the latency of one block (a 16^3 chunk is 64 threads' work) and of its reads over the host
-// link: 14 us for a 16^3 u8 chunk, cold.  A chunk paged into the resident 1024^3 grid takes 57 us in
+// A thread per row of eight voxels.  Bound by the latency of one block and of its reads over the host
+// link: 7.6 us for a 16^3 u8 chunk, cold (14 us with a thread per slice).  A chunk paged into the resident 1024^3 grid takes 50 us in
 // all against 110 us with an upload, the reorder, the merge, three copies back, a wait, the slots'
 // upload and the scatter around the same lattice passes.
 template <typename T>
@@ -166,41 +166,47 @@ __global__ void __launch_bounds__(1024) update_small_kernel(GridView g, UpdateBo
                                                             uint64_t* __restrict__ masks,
                                                             T* __restrict__ payload) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* box = reinterpret_cast<T*>(smem_raw);
+    const T* box = reinterpret_cast<const T*>(smem_raw);
     __shared__ uint32_t s_alpha[8];            // palette entries that are occupied, one bit each
     __shared__ uint32_t s_fresh[4], s_freed[4];
-    __shared__ uint32_t s_slot[kSmallBricks], s_free[kSmallBricks];
+    __shared__ uint32_t s_slot[kSmallBricks], s_free[kSmallBricks], s_old[kSmallBricks];
+    __shared__ uint8_t s_bits[kSmallBricks * 64];  // occupancy of each row after the update
     __shared__ int s_delta;
     const uint32_t K = (uint32_t)(u.kx * u.ky * u.kz), t = threadIdx.x, lane = t & 31u;
     const uint32_t n16 = (uint32_t)(((size_t)u.w * u.h * u.d * sizeof(T) + 15) / 16);
     for (uint32_t i = t; i < n16; i += blockDim.x) reinterpret_cast<uint4*>(smem_raw)[i] = x->box[i];
-    if (sizeof(T) == 1) {
-        for (uint32_t i = t; i < 256; i += blockDim.x) {
-            const uint32_t m = __ballot_sync(0xFFFFFFFFu, (g.palette[i] >> 24) != 0u);
-            if (lane == 0) s_alpha[i >> 5] = m;
-        }
+    // brick k: (bx0 + k % kx, ...)
+    auto brick_at = [&](uint32_t k, int32_t& bxi, int32_t& byi, int32_t& bzi) {
+        bxi = u.bx0 + (int32_t)(k % (uint32_t)u.kx);
+        byi = u.by0 + (int32_t)(k / (uint32_t)u.kx % (uint32_t)u.ky);
+        bzi = u.bz0 + (int32_t)(k / (uint32_t)(u.kx * u.ky));
+        return (size_t)bxi + (size_t)g.bx * ((size_t)byi + (size_t)g.by * bzi);
+    };
+    for (uint32_t k = t; k < K; k += blockDim.x) {
+        int32_t bxi, byi, bzi;
+        const uint32_t e = dir[brick_at(k, bxi, byi, bzi)];
+        s_old[k] = e;
+        s_slot[k] = 0u;
+        x->old_dir[k] = e;
+    }
+    if (sizeof(T) == 1 && t < 256) {  // the block has at least 256 threads
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, (g.palette[t] >> 24) != 0u);
+        if (lane == 0) s_alpha[t >> 5] = m;
     }
     if (t == 0) s_delta = 0;
     __syncthreads();
-    // the slice of this thread: brick k, z-slice lz
-    const uint32_t k = t >> 3;
-    const int32_t lz = (int32_t)(t & 7u);
-    const bool active = k < K;
-    const int32_t bxi = u.bx0 + (int32_t)(k % (uint32_t)u.kx);
-    const int32_t byi = u.by0 + (int32_t)(k / (uint32_t)u.kx % (uint32_t)u.ky);
-    const int32_t bzi = u.bz0 + (int32_t)(k / (uint32_t)(u.kx * u.ky));
-    const size_t b = (size_t)bxi + (size_t)g.bx * ((size_t)byi + (size_t)g.by * bzi);
-    const uint32_t e = active ? dir[b] : kEmptyBit;
-    const bool was = !brick_empty(e);
-    const int32_t z = bzi * 8 + lz;
-    const bool z_in = z >= u.z0 && z < u.z0 + u.d;
     const size_t ex = p.z_fastest ? (size_t)u.d * u.h : 1, ey = p.z_fastest ? (size_t)u.d : (size_t)u.w,
                  ez = p.z_fastest ? 1 : (size_t)u.w * u.h;
-    // voxels of row ly after the update; false when the box does not touch the row
-    auto merged = [&](int32_t ly, T v[8]) {
-        const int32_t y = byi * 8 + ly;
-        const bool in = z_in && y >= u.y0 && y < u.y0 + u.h;
-        const T* old = payload + (size_t)(was ? e : 0u) * 512 + lz * 64 + ly * 8;
+    // row r: brick r >> 6, z-slice (r >> 3) & 7, y r & 7: its voxels after the update; false when the
+    // box does not touch it
+    auto merged = [&](uint32_t r, T v[8]) {
+        int32_t bxi, byi, bzi;
+        brick_at(r >> 6, bxi, byi, bzi);
+        const uint32_t e = s_old[r >> 6];
+        const bool was = !brick_empty(e);
+        const int32_t y = byi * 8 + (int32_t)(r & 7u), z = bzi * 8 + (int32_t)((r >> 3) & 7u);
+        const bool in = z >= u.z0 && z < u.z0 + u.d && y >= u.y0 && y < u.y0 + u.h;
+        const T* old = payload + ((size_t)(was ? e : 0u) * 64 + (r & 63u)) * 8;
 #pragma unroll
         for (int32_t lx = 0; lx < 8; ++lx) {
             const int32_t vx = bxi * 8 + lx;
@@ -211,35 +217,28 @@ __global__ void __launch_bounds__(1024) update_small_kernel(GridView g, UpdateBo
         }
         return in;
     };
-    uint64_t word = 0, old_word = 0;
-    if (active) {
-        if (was) old_word = masks[(size_t)e * 8 + lz];
-        word = old_word;
-#pragma unroll 2
-        for (int32_t ly = 0; ly < 8; ++ly) {
-            T v[8];
-            if (!merged(ly, v)) continue;
-            uint32_t bits = 0;
+    const uint32_t rows = K * 64;
+    for (uint32_t r = t; r < rows; r += blockDim.x) {  // whole warps: half a brick each
+        const uint32_t e = s_old[r >> 6];
+        const uint32_t before = brick_empty(e) ? 0u : (uint32_t)((const uint8_t*)masks)[(size_t)e * 64 + (r & 63u)];
+        uint32_t bits = before;
+        T v[8];
+        if (merged(r, v)) {
+            bits = 0;
 #pragma unroll
             for (int32_t lx = 0; lx < 8; ++lx) {
                 const bool o = sizeof(T) == 1 ? (s_alpha[(uint32_t)v[lx] >> 5] >> ((uint32_t)v[lx] & 31u)) & 1u
                                               : ((uint32_t)v[lx] >> 24) != 0u;
                 bits |= (uint32_t)o << lx;
             }
-            word = (word & ~(0xFFull << (8 * ly))) | ((uint64_t)bits << (8 * ly));
         }
-    }
-    const int delta = __reduce_add_sync(0xFFFFFFFFu, __popcll(word) - __popcll(old_word));
-    if (lane == 0 && delta) atomicAdd(&s_delta, delta);
-    // lanes 8j .. 8j + 7 hold one brick
-    uint32_t any = word != 0ull;
-#pragma unroll
-    for (int s = 1; s < 8; s <<= 1) any |= __shfl_xor_sync(0xFFFFFFFFu, any, s);
-    if (active && lz == 0) {
-        s_slot[k] = any ? 1u : 0u;
-        s_free[k] = e;
-        x->old_dir[k] = e;
-        x->now[k] = any ? 1u : 0u;
+        s_bits[r] = (uint8_t)bits;
+        const uint32_t some = __ballot_sync(0xFFFFFFFFu, bits != 0u);
+        const int delta = __reduce_add_sync(0xFFFFFFFFu, __popc(bits) - __popc(before));
+        if (lane == 0) {
+            if (some) atomicOr(&s_slot[r >> 6], 1u);
+            if (delta) atomicAdd(&s_delta, delta);
+        }
     }
     __syncthreads();
     // ranks of the bricks that become occupied (fresh) and empty (freed), in brick order
@@ -247,7 +246,10 @@ __global__ void __launch_bounds__(1024) update_small_kernel(GridView g, UpdateBo
     bool fresh = false, freed = false;
     uint32_t e0 = kEmptyBit;
     if (lists) {
-        if (t < K) e0 = s_free[t];
+        if (t < K) {
+            e0 = s_old[t];
+            x->now[t] = s_slot[t];
+        }
         const bool w0 = !brick_empty(e0), n0 = t < K && s_slot[t] != 0u;
         fresh = n0 && !w0;
         freed = w0 && !n0;
@@ -279,7 +281,6 @@ __global__ void __launch_bounds__(1024) update_small_kernel(GridView g, UpdateBo
     if (t < K) {
         if (s_slot[t] != 0u && !fresh) mine = e0;
         // the freed slots, in brick order, go to the end of the free list, which is used from its end
-        // (every old entry has been read before the last barrier)
         if (freed) s_free[rank_freed] = e0;
     }
     __syncthreads();
@@ -292,15 +293,17 @@ __global__ void __launch_bounds__(1024) update_small_kernel(GridView g, UpdateBo
         s_slot[t] = mine;
     }
     __syncthreads();
-    if (!active) return;
-    const uint32_t slot = s_slot[k];
-    if (lz == 0) dir[b] = slot;
-    if (brick_empty(slot)) return;
-    masks[(size_t)slot * 8 + lz] = word;
-    for (int32_t ly = 0; ly < 8; ++ly) {
+    for (uint32_t r = t; r < rows; r += blockDim.x) {
+        const uint32_t k = r >> 6, in = r & 63u, slot = s_slot[k];
+        if (in == 0) {
+            int32_t bxi, byi, bzi;
+            dir[brick_at(k, bxi, byi, bzi)] = slot;
+        }
+        if (brick_empty(slot)) continue;
+        ((uint8_t*)masks)[(size_t)slot * 64 + in] = s_bits[r];
         T v[8];
-        if (!merged(ly, v) && was) continue;  // the row keeps its voxels in the same slot
-        T* out = payload + (size_t)slot * 512 + lz * 64 + ly * 8;
+        if (!merged(r, v) && !brick_empty(s_old[k])) continue;  // the row keeps its voxels in the same slot
+        T* out = payload + ((size_t)slot * 64 + in) * 8;
         if (sizeof(T) == 1) {
             uint2 q;
             q.x = (uint32_t)v[0] | (uint32_t)v[1] << 8 | (uint32_t)v[2] << 16 | (uint32_t)v[3] << 24;
@@ -381,7 +384,7 @@ static int32_t update_small(Grid& g, const void* voxels, size_t elem, uint32_t o
         p.slots_used = (uint32_t)g.slots_used;
         p.slot_capacity = (uint32_t)std::min<uint64_t>(g.slot_capacity, 0x7FFFFFFFu);
         p.z_fastest = order == VT_ORDER_Z_FASTEST ? 1u : 0u;
-        const unsigned threads = std::max(256u, (K * 8 + 31) / 32 * 32);
+        const unsigned threads = std::min(1024u, std::max(256u, K * 64));
         if (elem == 1)
             update_small_kernel<uint8_t><<<1, threads, smem, st>>>(g.view(), u, p, dx, g.dir, g.masks, (uint8_t*)g.payload);
         else
