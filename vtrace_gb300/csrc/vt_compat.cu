@@ -31,14 +31,18 @@ namespace vt {
 
 constexpr uint32_t kMaxTextures = 65536;  // lib/common.h:35
 
+// What the pixel kernel reads of an instance: the rows of inverse(model)'s linear part each with the
+// camera in model space `om` (the same for every pixel), the cube's planes -0.5 - om and 0.5 - om.
 struct CompatInstance {
-    float minv[12];  // inverse(model), rows 0..2 of the 4x4 (row-major)
+    float4 row[3];   // inverse(model) row r columns 0..2, om[r]
+    float lo[3];
+    float near;      // at most the slab entry parameter tn of any pixel's ray (0: no bound)
+    float hi[3];
     int32_t texture;
     int32_t tx0, ty0, tx1, ty1;  // 16 x 16-pixel tiles its pixels can fall in (inclusive; empty
                                  // when tx0 > tx1)
-    float near;  // at most the slab entry parameter tn of any pixel's ray (0: no bound)
-    int32_t pad;
 };
+static_assert(sizeof(CompatInstance) == 96, "float4 loads");
 
 constexpr int32_t kTile = 16;
 // Bitmasks larger than this are not built; every tile then visits every instance.
@@ -134,6 +138,16 @@ struct InstanceCursor {
     }
 };
 
+__device__ __forceinline__ float rcp_approx(float x) {  // within one unit in the last place
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// Bound by instruction issue: 1000 x 1000 pixels over 1,314 chunk instances 147 -> 131 us (0.128 -> 0.111
+// G warp instructions) with the camera and planes in model space taken from the record and most of the
+// six divisions per instance and pixel gone.
+//
 // Blocks of 128 threads cover 16 x 8 pixels, two per 16 x 16 binning tile.  8 blocks per SM
 // (64 registers instead of 72): 3-7% shorter ticks on the pager world.
 __global__ void __launch_bounds__(128, 8) compat_kernel(const GridView* __restrict__ views,
@@ -168,40 +182,63 @@ __global__ void __launch_bounds__(128, 8) compat_kernel(const GridView* __restri
     for (int32_t i = cur.next(); i >= 0; i = cur.next()) {
         if (!inside) continue;
         const CompatInstance& I = inst[i];
-        if (I.texture < 0) continue;  // draws nothing (only reached without bins)
-        if (I.near >= depth) continue;  // tn >= near >= depth: fails the depth test below
-        const GridView g = views[I.texture];
-        float om[3], dm[3];
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-            const float* m = I.minv + 4 * r;
-            om[r] = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(m[0], f.cam[0]), __fmul_rn(m[1], f.cam[1])),
-                                        __fmul_rn(m[2], f.cam[2])),
-                              m[3]);
-            dm[r] = __fadd_rn(__fadd_rn(__fmul_rn(m[0], dw[0]), __fmul_rn(m[1], dw[1])), __fmul_rn(m[2], dw[2]));
+        const float4 lo = *reinterpret_cast<const float4*>(I.lo);  // and near
+        if (lo.w >= depth) continue;  // tn >= near >= depth: fails the depth test below
+        const float4 hi = *reinterpret_cast<const float4*>(I.hi);  // and the texture
+        if (__float_as_int(hi.w) < 0) continue;  // draws nothing (only reached without bins)
+        const float4 r0 = I.row[0], r1 = I.row[1], r2 = I.row[2];
+        const float om[3] = {r0.w, r1.w, r2.w};
+        const float dm[3] = {
+            __fadd_rn(__fadd_rn(__fmul_rn(r0.x, dw[0]), __fmul_rn(r0.y, dw[1])), __fmul_rn(r0.z, dw[2])),
+            __fadd_rn(__fadd_rn(__fmul_rn(r1.x, dw[0]), __fmul_rn(r1.y, dw[1])), __fmul_rn(r1.z, dw[2])),
+            __fadd_rn(__fadd_rn(__fmul_rn(r2.x, dw[0]), __fmul_rn(r2.y, dw[1])), __fmul_rn(r2.z, dw[2]))};
+        // Slab test against the unit cube [-0.5, 0.5]^3, first with approximate reciprocals (within
+        // 2^-22 of the quotients; a margin of 1e-5 is taken): it rejects what certainly misses, starts
+        // behind the camera or lies behind the pixel's depth, and where it leaves no doubt about the
+        // entry face and the exit, one division gives the exact entry parameter instead of six.
+        float tn;
+        int ax;
+        bool sure = fminf(fminf(fabsf(dm[0]), fabsf(dm[1])), fabsf(dm[2])) > 1e-30f;
+        const bool px_ = dm[0] > 0.0f, py_ = dm[1] > 0.0f, pz_ = dm[2] > 0.0f;
+        const float nx = px_ ? lo.x : hi.x, ny = py_ ? lo.y : hi.y, nz = pz_ ? lo.z : hi.z;
+        if (sure) {
+            const float rx = rcp_approx(dm[0]), ry = rcp_approx(dm[1]), rz = rcp_approx(dm[2]);
+            const float ex = nx * rx, ey = ny * ry, ez = nz * rz;
+            const float tnm = fmaxf(fmaxf(ex, ey), ez);
+            const float tfm = fminf(fminf((px_ ? hi.x : lo.x) * rx, (py_ ? hi.y : lo.y) * ry), (pz_ ? hi.z : lo.z) * rz);
+            const float under = tnm * 0.99999f;
+            if (tnm < 0.0f || tfm < 0.0f || under > tfm || under >= depth) continue;
+            const bool cx = ex >= under, cy = ey >= under, cz = ez >= under;
+            ax = cx ? 0 : (cy ? 1 : 2);
+            sure = (int)cx + (int)cy + (int)cz == 1 && tfm > tnm * 1.00001f && tnm > 1e-30f && tnm < 1e30f;
+            tn = __fdiv_rn(cx ? nx : (cy ? ny : nz), cx ? dm[0] : (cy ? dm[1] : dm[2]));
         }
-        // slab test against the unit cube [-0.5, 0.5]^3
-        float tn = -INFINITY, tf = INFINITY;
-        int ax = -1;
-        bool miss = false;
+        if (!sure) {
+            const float l[3] = {lo.x, lo.y, lo.z}, h[3] = {hi.x, hi.y, hi.z};
+            float tf = INFINITY;
+            tn = -INFINITY;
+            ax = -1;
+            bool miss = false;
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            if (dm[a] == 0.0f) {
-                if (om[a] < -0.5f || om[a] > 0.5f) miss = true;
-                continue;
+            for (int a = 0; a < 3; ++a) {
+                if (dm[a] == 0.0f) {
+                    if (om[a] < -0.5f || om[a] > 0.5f) miss = true;
+                    continue;
+                }
+                const float ta = __fdiv_rn(l[a], dm[a]);
+                const float tb = __fdiv_rn(h[a], dm[a]);
+                const float t0 = ta < tb ? ta : tb, t1 = ta < tb ? tb : ta;
+                if (t0 > tn) {
+                    tn = t0;
+                    ax = a;
+                }
+                if (t1 < tf) tf = t1;
             }
-            const float ta = __fdiv_rn(__fsub_rn(-0.5f, om[a]), dm[a]);
-            const float tb = __fdiv_rn(__fsub_rn(0.5f, om[a]), dm[a]);
-            const float lo = ta < tb ? ta : tb, hi = ta < tb ? tb : ta;
-            if (lo > tn) {
-                tn = lo;
-                ax = a;
-            }
-            if (hi < tf) tf = hi;
+            // camera inside the cube: only back faces face it, and those are culled
+            if (miss || tn > tf || tf < 0.0f || tn <= 0.0f) continue;
         }
-        // camera inside the cube: only back faces face it, and those are culled
-        if (miss || tn > tf || tf < 0.0f || tn <= 0.0f) continue;
         if (!(tn < depth)) continue;  // depth test LESS against the nearest hit so far
+        const GridView g = views[__float_as_int(hi.w)];
         const float size[3] = {__int2float_rn(g.nx), __int2float_rn(g.ny), __int2float_rn(g.nz)};
         float pos[3];
 #pragma unroll
@@ -295,6 +332,33 @@ static __host__ __device__ bool invert4(const double* m, double* inv) {
     return true;
 }
 
+// Rows 0..2 of invert4 for a matrix whose bottom row is (0, 0, 0, 1), columns of `a` first: what is left
+// of its cofactors once the products with exact zeros are gone (adding one changes at most the sign of a
+// zero, which nothing downstream tells apart), in the same order, so the same values at a third of the
+// binary64 work.  The caller checks the row and that every element is finite.
+static __device__ __forceinline__ bool invert_affine(const double* a, double* inv) {
+    double r[16];
+    r[0] = a[5] * a[10] - a[9] * a[6];
+    r[4] = -a[4] * a[10] + a[8] * a[6];
+    r[8] = a[4] * a[9] - a[8] * a[5];
+    r[1] = -a[1] * a[10] + a[9] * a[2];
+    r[5] = a[0] * a[10] - a[8] * a[2];
+    r[9] = -a[0] * a[9] + a[8] * a[1];
+    r[2] = a[1] * a[6] - a[5] * a[2];
+    r[6] = -a[0] * a[6] + a[4] * a[2];
+    r[10] = a[0] * a[5] - a[4] * a[1];
+    r[12] = -a[4] * a[9] * a[14] + a[4] * a[10] * a[13] + a[8] * a[5] * a[14] - a[8] * a[6] * a[13] - a[12] * a[5] * a[10] + a[12] * a[6] * a[9];
+    r[13] = a[0] * a[9] * a[14] - a[0] * a[10] * a[13] - a[8] * a[1] * a[14] + a[8] * a[2] * a[13] + a[12] * a[1] * a[10] - a[12] * a[2] * a[9];
+    r[14] = -a[0] * a[5] * a[14] + a[0] * a[6] * a[13] + a[4] * a[1] * a[14] - a[4] * a[2] * a[13] - a[12] * a[1] * a[6] + a[12] * a[2] * a[5];
+    const double det = a[0] * r[0] + a[1] * r[4] + a[2] * r[8];
+    if (!(det != 0.0) || !isfinite(det)) return false;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) inv[4 * c + k] = r[4 * c + k] / det;
+    return true;
+}
+
 // column-major product c = a * b
 static void mul4(const double* a, const double* b, double* c) {
     for (int col = 0; col < 4; ++col)
@@ -370,42 +434,160 @@ static CullFrame cull_frame(const double* dm, const double* cam, int32_t width, 
     return cf;
 }
 
-// Tile rectangle of an instance (model matrix md, column-major; its inverse mi).  Returns false
-// when no pixel can see it.
+// Camera in model space (inverse model matrix mi), and from it what both culling tests need: the
+// squared distance d2 of the camera to the unit cube there and the squared Frobenius norm `fro` of the
+// inverse's linear part.  The products are binary64 (they cancel); the rest is binary32, whose rounding
+// (2^-20 relative, taken generously) the callers' margins cover.
+struct ModelCamera {
+    float d2, fro;
+};
+
+static __device__ ModelCamera model_camera(const CullFrame& cf, const double* mi) {
+    ModelCamera c = {0.0f, 0.0f};
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        const float om = (float)(mi[0 * 4 + r] * cf.cam[0] + mi[1 * 4 + r] * cf.cam[1] +
+                                 mi[2 * 4 + r] * cf.cam[2] + mi[3 * 4 + r]);
+        const float e = fmaxf(fabsf(om) - 0.5f, 0.0f);
+        c.d2 += e * e;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float m = (float)mi[k * 4 + r];
+            c.fro += m * m;
+        }
+    }
+    return c;
+}
+
 // A lower bound of the slab entry parameter tn (the distance along the unit-length pixel ray) of
 // every pixel's ray, for rejecting the instance behind a pixel's depth before its slab test: the
 // camera's distance to the cube in model space over a bound of the inverse's spectral norm
-// (sqrt(|Minv|_1 |Minv|_inf)), less 1%.  The pixel kernel's binary32 tn is within about
-// cond(M) 2^-21 of the exact one relative to its size, so the 1% holds it above the bound while
-// cond(M) (Frobenius) stays below 1024 and the camera is not within 1/256 of the cube; otherwise 0.
-static __host__ __device__ float instance_near(const CullFrame& cf, const double* md,
-                                               const double* mi) {
+// (sqrt(|Minv|_1 |Minv|_inf)), less 1.1%.  The pixel kernel's binary32 tn is within about
+// cond(M) 2^-21 of the exact one relative to its size, so a margin of 1% holds it above the bound while
+// cond(M) (Frobenius) stays below 1024 and the camera is not within 1/256 of the cube, otherwise 0; the
+// rest of the margin is for the binary32 arithmetic here.
+static __device__ float instance_near(const CullFrame& cf, const float* m, const double* mi,
+                                      const ModelCamera& mc) {
     if (!cf.ok) return 0.0f;
-    double d2 = 0.0, fm = 0.0, fi = 0.0, n1 = 0.0, ninf = 0.0;
+    float fm = 0.0f, n1 = 0.0f, ninf = 0.0f;
+#pragma unroll
     for (int r = 0; r < 3; ++r) {
-        const double om = mi[0 * 4 + r] * cf.cam[0] + mi[1 * 4 + r] * cf.cam[1] +
-                          mi[2 * 4 + r] * cf.cam[2] + mi[3 * 4 + r];
-        const double e = fmax(fabs(om) - 0.5, 0.0);
-        d2 += e * e;
-        double row = 0.0, col = 0.0;
+        float row = 0.0f, col = 0.0f;
+#pragma unroll
         for (int k = 0; k < 3; ++k) {
-            fm += md[k * 4 + r] * md[k * 4 + r];
-            fi += mi[k * 4 + r] * mi[k * 4 + r];
-            row += fabs(mi[k * 4 + r]);  // row r of the inverse's linear part
-            col += fabs(mi[r * 4 + k]);  // column r
+            fm += m[k * 4 + r] * m[k * 4 + r];
+            row += fabsf((float)mi[k * 4 + r]);  // row r of the inverse's linear part
+            col += fabsf((float)mi[r * 4 + k]);  // column r
         }
-        ninf = fmax(ninf, row);
-        n1 = fmax(n1, col);
+        ninf = fmaxf(ninf, row);
+        n1 = fmaxf(n1, col);
     }
-    const double dist = sqrt(d2), cond = sqrt(fm) * sqrt(fi), n2 = sqrt(n1 * ninf);
-    if (!(dist > 1.0 / 256.0) || !(cond <= 1024.0) || !(n2 > 0.0) || !isfinite(dist)) return 0.0f;
-    const float near = (float)(0.99 * dist / n2);
+    const float dist = sqrtf(mc.d2), cond = sqrtf(fm) * sqrtf(mc.fro), n2 = sqrtf(n1) * sqrtf(ninf);
+    if (!(dist > 1.001f / 256.0f) || !(cond <= 1023.0f) || !(n2 > 0.0f) || !isfinite(dist)) return 0.0f;
+    const float near = 0.989f * dist / n2;
     return isfinite(near) ? near : 0.0f;
 }
 
-static __host__ __device__ bool instance_tiles(const CullFrame& cf, const double* md,
-                                               const double* mi, int32_t& tx0, int32_t& ty0,
-                                               int32_t& tx1, int32_t& ty1) {
+// Tile rectangle of an instance in binary32: 1 and the rectangle, 0 when no pixel can see it, -1 when
+// the error bounds here are too wide (instance_tiles then decides).
+//
+// instance_tiles with every quantity's rounding bounded: a point of the cube has q within E (per
+// coordinate) of its counterpart in the hull of the computed corners, where E = 2^-20 |row of B^-1|_1 S
+// and S bounds the terms of X - cam (binary32 sums of at most seven terms and products err by less than
+// 8 x 2^-24 of their sum of magnitudes; twice that is taken).  Visible points have q.z >= eps, so their
+// counterparts have q.z >= eps / 2 provided eps >= 64 E.z: the rectangle of the hull clipped there,
+// each vertex p widened by (2 E.x + 2 |p.x / p.z| E.z) / p.z, holds all their projections.
+static __device__ int instance_tiles_f32(const CullFrame& cf, const float* m, const double* md,
+                                         const ModelCamera& mc, int32_t& tx0, int32_t& ty0,
+                                         int32_t& tx1, int32_t& ty1) {
+    if (!cf.ok) return -1;
+    if (!(mc.d2 > 1e-12f) || !(mc.fro > 0.0f) || !isfinite(mc.d2) || !isfinite(mc.fro)) return -1;
+    // 1% below the binary64 path's bound
+    const float eps = 0.495f * sqrtf(mc.d2 / mc.fro) / (float)cf.len_max;
+    float S = 0.0f, t[3], bi[9], E[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        t[r] = (float)(md[3 * 4 + r] - cf.cam[r]);
+        S = fmaxf(S, fabsf(t[r]) + 0.5f * (fabsf(m[r]) + fabsf(m[4 + r]) + fabsf(m[8 + r])));
+    }
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        float n = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            bi[3 * r + k] = (float)cf.binv[3 * r + k];
+            n += fabsf(bi[3 * r + k]);
+        }
+        E[r] = 0x1p-20f * n * S;
+    }
+    if (!(eps >= 64.0f * E[2]) || !isfinite(S)) return -1;
+    // corners in q space
+    float q[8][3];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        float x[3];
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+            x[r] = ((k & 1) ? 0.5f : -0.5f) * m[r] + ((k & 2) ? 0.5f : -0.5f) * m[4 + r] +
+                   ((k & 4) ? 0.5f : -0.5f) * m[8 + r] + t[r];
+#pragma unroll
+        for (int r = 0; r < 3; ++r) q[k][r] = bi[3 * r] * x[0] + bi[3 * r + 1] * x[1] + bi[3 * r + 2] * x[2];
+    }
+    const float zc = 0.5f * eps;
+    float xmin = INFINITY, xmax = -INFINITY, ymin = INFINITY, ymax = -INFINITY;
+    bool any = false, cut = false;
+    auto take = [&](float x, float y, float z) {
+        const float r = 1.0f / z, xn = x * r, yn = y * r;
+        const float wx = 2.0f * (E[0] + fabsf(xn) * E[2]) * r, wy = 2.0f * (E[1] + fabsf(yn) * E[2]) * r;
+        xmin = fminf(xmin, xn - wx);
+        xmax = fmaxf(xmax, xn + wx);
+        ymin = fminf(ymin, yn - wy);
+        ymax = fmaxf(ymax, yn + wy);
+        any = true;
+    };
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        if (q[k][2] >= zc)
+            take(q[k][0], q[k][1], q[k][2]);
+        else
+            cut = true;
+    }
+    if (!any) return 0;  // the whole cube is behind the camera
+    if (cut) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const int j = k | (1 << a);
+                if (j == k) continue;  // each edge once, from its lower corner
+                const float sa = q[k][2] - zc, sb = q[j][2] - zc;
+                if ((sa < 0.0f) == (sb < 0.0f)) continue;
+                const float u = sa / (sa - sb);
+                take(q[k][0] + u * (q[j][0] - q[k][0]), q[k][1] + u * (q[j][1] - q[k][1]), zc);
+            }
+    }
+    if (!(isfinite(xmin) && isfinite(xmax) && isfinite(ymin) && isfinite(ymax))) return -1;
+    // xn -> px: px = (xn + 1) width / 2 - 0.5, and yn -> py with the same width; binary32 errs by less
+    // than a thousandth of a pixel on the screen (width <= 16384): the margin is 2 pixels and a half
+    const float hw = 0.5f * (float)cf.width;
+    const float px0 = floorf((xmin + 1.0f) * hw - 0.5f) - 2.5f, px1 = ceilf((xmax + 1.0f) * hw - 0.5f) + 2.5f;
+    const float py0 = floorf((ymin + 1.0f) * hw - 0.5f) - 2.5f, py1 = ceilf((ymax + 1.0f) * hw - 0.5f) + 2.5f;
+    if (px1 < 0.0f || py1 < 0.0f || px0 > (float)(cf.width - 1) || py0 > (float)(cf.height - 1)) return 0;
+    tx0 = (int32_t)(fmaxf(px0, 0.0f) / kTile);
+    tx1 = (int32_t)(fminf(px1, (float)(cf.width - 1)) / kTile);
+    ty0 = (int32_t)(fmaxf(py0, 0.0f) / kTile);
+    ty1 = (int32_t)(fminf(py1, (float)(cf.height - 1)) / kTile);
+    return 1;
+}
+
+// Tile rectangle of an instance (model matrix m, column-major), in binary64.  Returns false when no
+// pixel can see it.
+static __device__ __noinline__ bool instance_tiles(const CullFrame& cf, const float* m, int32_t& tx0,
+                                                   int32_t& ty0, int32_t& tx1, int32_t& ty1) {
+    double md[16], mi[16];
+    for (int k = 0; k < 16; ++k) md[k] = m[k];
+    md[15] = 1.0;
+    if (!invert4(md, mi)) return false;  // not reached: the caller has the inverse
     const int32_t ntx = (cf.width + kTile - 1) / kTile, nty = (cf.height + kTile - 1) / kTile;
     tx0 = 0;
     ty0 = 0;
@@ -472,6 +654,10 @@ static __host__ __device__ bool instance_tiles(const CullFrame& cf, const double
     return true;
 }
 
+// Bound by the latency of one binary64 inverse per thread and of the matrix' read over the host link:
+// 20 us for 1,314 instances, cold, against 49 us with the rectangle and the depth bound in binary64 and
+// the general inverse for every matrix.
+//
 // Device records of the instances (trace.vert:38-40: the texture id in the bits of element
 // [3][3], which reads as 1): inverse model matrix and tile rectangle, one thread per instance,
 // in draw order.  Instances with an unbound texture id or a singular matrix draw nothing
@@ -494,23 +680,39 @@ __global__ void __launch_bounds__(128) compat_prepare_kernel(const float* __rest
     const int32_t tid = __float_as_int(m[15]);
     CompatInstance ci;
 #pragma unroll
-    for (int k = 0; k < 12; ++k) ci.minv[k] = 0.0f;
+    for (int r = 0; r < 3; ++r) {
+        ci.row[r] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        ci.lo[r] = ci.hi[r] = 0.0f;
+    }
     ci.texture = -1;
     ci.tx0 = ci.ty0 = 1;  // empty rectangle: in no tile
     ci.tx1 = ci.ty1 = 0;
     ci.near = 0.0f;
-    ci.pad = 0;
     if (tid >= 0 && (uint32_t)tid < ntex) {
         double md[16], mi[16];
 #pragma unroll
         for (int k = 0; k < 16; ++k) md[k] = m[k];
         md[15] = 1.0;
-        if (invert4(md, mi)) {
-            for (int r = 0; r < 3; ++r)
-                for (int k = 0; k < 4; ++k) ci.minv[4 * r + k] = (float)mi[k * 4 + r];
+        bool affine = m[3] == 0.0f && m[7] == 0.0f && m[11] == 0.0f;
+#pragma unroll
+        for (int k = 0; k < 15; ++k) affine = affine && isfinite(m[k]);
+        if (affine ? invert_affine(md, mi) : invert4(md, mi)) {
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                const float a0 = (float)mi[r], a1 = (float)mi[4 + r], a2 = (float)mi[8 + r], a3 = (float)mi[12 + r];
+                const float om = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(a0, (float)cf.cam[0]),
+                                                               __fmul_rn(a1, (float)cf.cam[1])),
+                                                     __fmul_rn(a2, (float)cf.cam[2])), a3);
+                ci.row[r] = make_float4(a0, a1, a2, om);
+                ci.lo[r] = __fsub_rn(-0.5f, om);
+                ci.hi[r] = __fsub_rn(0.5f, om);
+            }
             ci.texture = tid;
-            ci.near = instance_near(cf, md, mi);
-            if (!instance_tiles(cf, md, mi, ci.tx0, ci.ty0, ci.tx1, ci.ty1)) {
+            const ModelCamera mc = model_camera(cf, mi);
+            ci.near = instance_near(cf, m, mi, mc);
+            int seen = instance_tiles_f32(cf, m, md, mc, ci.tx0, ci.ty0, ci.tx1, ci.ty1);
+            if (seen < 0) seen = instance_tiles(cf, insts + 16 * (size_t)i, ci.tx0, ci.ty0, ci.tx1, ci.ty1);
+            if (!seen) {
                 ci.tx0 = ci.ty0 = 1;
                 ci.tx1 = ci.ty1 = 0;
             }
