@@ -526,13 +526,16 @@ int32_t build_grid(const void* d_src, uint32_t format, const uint32_t* palette_h
         g->occupied = counts[0];
         const uint64_t slots = g->nonempty ? g->nonempty : 1;
         const BlockLayout L = block_layout(g->bricks, slots, format);
+        // from the stream-ordered pool, whose freed memory the next grid reuses: cudaMalloc and
+        // cudaFree of the 157 MB of a 1024^3 grid took 0.3 ms of a scene's change
         void* block = nullptr;
-        if (cudaMalloc(&block, L.total) != cudaSuccess) {
+        if (cudaMallocAsync(&block, L.total, stream) != cudaSuccess) {
             cudaGetLastError();
-            rc = fail(VT_ENOMEM, "cudaMalloc(brick grid) failed");
+            rc = fail(VT_ENOMEM, "cudaMallocAsync(brick grid) failed");
             break;
         }
         point_into_block(*g, block, L, slots);
+        g->pooled = true;
         if (g->palette) {
             e = cudaMemcpyAsync(g->palette, d_palette, 1024, cudaMemcpyDeviceToDevice, stream);
             if (e != cudaSuccess) { rc = cuda_fail(e, "cudaMemcpy(palette)"); break; }
@@ -707,6 +710,11 @@ void vt_shutdown(void) {
     s.aux_start = nullptr;
     for (cudaEvent_t ev : s.chunk_events) cudaEventDestroy(ev);
     s.chunk_events.clear();
+    // give the pool's memory back
+    cudaStreamSynchronize(s.stream);
+    cudaMemPool_t pool;
+    if (cudaDeviceGetDefaultMemPool(&pool, s.device) != cudaSuccess || cudaMemPoolTrimTo(pool, 0) != cudaSuccess)
+        cudaGetLastError();
     cudaStreamDestroy(s.stream);
     s.stream = nullptr;
     s.inited = false;
