@@ -156,7 +156,8 @@ int32_t vt_device_info(int32_t* device, int32_t* sm_count, uint64_t* free_bytes,
 void* vt_get_stream(void);
 
 /* Launch shape of a tracing entry point.  persistent = 0: one thread per ray, rays packed in
- * 8 x 4 pixel tiles per warp.  persistent = 1: resident warps keep one ray per lane and refill
+ * 8 x 4 pixel tiles per warp (launches too small to fill the chip give each warp fewer rays, and ray
+ * buffers below 196,608 rays always take this form).  persistent = 1: resident warps keep one ray per lane and refill
  * lanes whose rays have ended with new work once at least `refill_min` lanes are idle (1..32;
  * 32 = only when the whole warp is idle), with at most `blocks_per_sm` 256-thread blocks per SM
  * (0 = as many as fit).  VT_KERNEL_BATCH is always persistent; its refill_min 32 (the default)

@@ -82,6 +82,8 @@ struct State {
         tune_batch{32, 0, 1, 0, VT_TILE_8X4, 4}, tune_path{8, 0, 1, 1, VT_TILE_8X4, 4};
 };
 
+// Smallest ray buffer that the persistent form takes.
+constexpr uint64_t kPersistentRays = 196608;
 constexpr uint32_t kCounterRing = 4096;
 // Work counter for one persistent launch (zeroed by the launcher on its stream).
 unsigned long long* next_counter();

@@ -175,7 +175,8 @@ template <bool STATS>
 __global__ void __launch_bounds__(kBatchTileThreads, 9) batch_tile_kernel(const BatchView* __restrict__ table,
                                                          uint32_t nviews, uint64_t units,
                                                          unsigned long long* __restrict__ counter,
-                                                         Counters* __restrict__ counters) {
+                                                         Counters* __restrict__ counters,
+                                                         uint32_t lanes) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BatchView* views = reinterpret_cast<BatchView*>(smem_raw);
     {
@@ -192,7 +193,8 @@ __global__ void __launch_bounds__(kBatchTileThreads, 9) batch_tile_kernel(const 
         if (lane == 0) u = atomicAdd(counter, 1ull);
         u = __shfl_sync(0xFFFFFFFFu, u, 0);
         if (u >= units) break;
-        const uint64_t item = u * 32u + lane;  // views begin at multiples of 32 items
+        if (lane >= lanes) continue;  // small launches spread their items over more warps
+        const uint64_t item = u * lanes + lane;  // views begin at multiples of 32 items
         uint32_t lo = 0, hi = nviews - 1;
         while (lo < hi) {
             const uint32_t mid = (lo + hi + 1) >> 1;
@@ -204,10 +206,11 @@ __global__ void __launch_bounds__(kBatchTileThreads, 9) batch_tile_kernel(const 
         const BatchView& V = views[lo];
         const uint64_t local = item - V.begin + V.first_item;
         const uint64_t ts = local >> 5;
+        const uint32_t l = (uint32_t)local & 31u;
         const uint64_t tile = ts / V.spp;
         const uint32_t sample = (uint32_t)(ts - tile * V.spp);
-        const uint32_t px = ((uint32_t)(tile % V.tiles_x) << V.wx_log) + (lane & ((1u << V.wx_log) - 1u));
-        const uint32_t py = (uint32_t)(tile / V.tiles_x) * (32u >> V.wx_log) + (lane >> V.wx_log);
+        const uint32_t px = ((uint32_t)(tile % V.tiles_x) << V.wx_log) + (l & ((1u << V.wx_log) - 1u));
+        const uint32_t py = (uint32_t)(tile / V.tiles_x) * (32u >> V.wx_log) + (l >> V.wx_log);
         if (px < V.cam.width && py < V.cam.height) {
             float jx, jy, o[3], d[3];
             jitter(V.seed, V.view_id, px, py, sample, jx, jy);
@@ -314,7 +317,8 @@ unsigned batch_blocks(uint32_t n, uint64_t total, const TraceTuning& tune) {
         per_sm = 1;
     }
     if (tune.blocks_per_sm > 0) per_sm = std::min(per_sm, tune.blocks_per_sm);
-    const uint64_t need = (total + threads - 1) / threads;
+    const uint64_t per_block = batch_tile_form(tune) ? threads / 32 * lanes_per_warp(total, state().sm_count) : threads;
+    const uint64_t need = (total + per_block - 1) / per_block;
     return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)state().sm_count * per_sm, need));
 }
 
@@ -323,10 +327,11 @@ cudaError_t launch_batch(const BatchView* d_table, uint32_t n, uint64_t total,
                          cudaStream_t stream) {
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), stream);
     if (e != cudaSuccess) return e;
-    if (batch_tile_form(tune))
+    if (batch_tile_form(tune)) {
+        const uint32_t lanes = lanes_per_warp(total, state().sm_count);
         batch_tile_kernel<false><<<blocks, kBatchTileThreads, (size_t)n * sizeof(BatchView), stream>>>(
-            d_table, n, total / 32, counter, nullptr);
-    else
+            d_table, n, total / lanes, counter, nullptr, lanes);
+    } else
         batch_kernel<<<blocks, 256, (size_t)n * sizeof(BatchView), stream>>>(d_table, n, total,
                                                                              counter, tune.refill_min);
     return cudaGetLastError();
@@ -484,7 +489,7 @@ int32_t vt_batch_stats(int32_t batch, vt_trace_stats* stats) {
         tile.refill_min = 32;
         const unsigned blocks = batch_blocks(b->nviews, b->total, tile);
         batch_tile_kernel<true><<<blocks, kBatchTileThreads, b->smem, st>>>(
-            b->d_table, b->nviews, b->total / 32, cursor, dc);
+            b->d_table, b->nviews, b->total / 32, cursor, dc, 32u);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(&hc, dc, sizeof(Counters), cudaMemcpyDeviceToHost, st);

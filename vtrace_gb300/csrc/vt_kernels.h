@@ -22,6 +22,20 @@ struct TraceTuning {
     uint32_t block_warps = 4;  // render tile launch: warps per block (1, 2, 4, 8)
 };
 
+// Rays per warp of a launch with one thread per ray.  A launch whose rays fill only a few warps per SM
+// takes as long as its longest warp: the lanes of a warp take turns in the traversal (walks and
+// crossings, chains of different length), so spreading the rays over more warps shortens it until
+// about thirteen warps per SM share the issue slots.  96 x 64 pixels of a 256^3 scene with shadows:
+// 75.8 us with 32 rays per warp, 59.4 with 8, 53.3 with 4, 53.0 with 2; 160 x 120: 77.8, 61.4, 61.5,
+// 64.1; 320 x 240: 79.9, 88.1 (16: 82.8); 4,099 rays in a 512^3 scene: 53.2, 41.0, 40.9, 34.8; 64,000:
+// 63.5, 89.0 (16: 71.7).  So: rays over thirteen and a half warps per SM, to the nearest power of two.
+__host__ __device__ inline uint32_t lanes_per_warp(uint64_t rays, int sm_count) {
+    const uint64_t warps = (uint64_t)sm_count * 27 / 2;
+    uint32_t lanes = 2;
+    while (lanes < 32 && rays * 181 / 128 >= warps * (lanes * 2)) lanes *= 2;
+    return lanes;
+}
+
 // Render in two passes (primary rays, then the queued shadow rays); stream-ordered scratch.
 cudaError_t launch_render_wavefront(const GridView& g, const vt_camera& cam,
                                     const LightView& light, uint4* out, cudaStream_t stream);

@@ -120,24 +120,27 @@ constexpr int kUnitWait = 4;
 
 // Resident-warp tracing of `n` rays: a ray per lane, lanes whose rays ended refilled from `counter`
 // once `refill_min` of the warp's lanes are idle.  `io.load(item, o, d)` gives an item's ray and
-// `io.store(item, R, status)` takes its result; every lane of the warp calls this together.
+// `io.store(item, R, status)` takes its result; every lane of the warp calls this together.  Only the
+// first `lanes` lanes take rays (lanes_per_warp()).
 template <class Io>
 __device__ __forceinline__ void trace_persistent(const GridView& g, const Io& io, uint64_t n,
                                                  unsigned long long* __restrict__ counter,
-                                                 uint32_t refill_min) {
+                                                 uint32_t refill_min, uint32_t lanes) {
     const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t all = lanes >= 32u ? 0xFFFFFFFFu : (1u << lanes) - 1u;
+    const int refill = (int)min(refill_min, lanes);
     LaneRay R;
     bool busy = false;
     typename Io::Index idx = 0;
     bool more = true;
     int wait_w = 0, wait_c = 0;  // warp-uniform: iterations a unit kind was passed over
     for (;;) {
-        uint32_t idle = __ballot_sync(0xFFFFFFFFu, !busy);
-        while (more && __popc(idle) >= (int)refill_min) {
+        uint32_t idle = __ballot_sync(0xFFFFFFFFu, !busy) & all;
+        while (more && __popc(idle) >= refill) {
             uint64_t item;
             const uint64_t base = warp_fetch(counter, idle, lane, item);
             if (base + __popc(idle) >= n) more = false;
-            if (!busy && item < n) {
+            if (!busy && lane < lanes && item < n) {
                 float o[3], d[3];
                 io.load((typename Io::Index)item, o, d);
                 const int st = ray_begin(g, o, d, R);
@@ -148,9 +151,9 @@ __device__ __forceinline__ void trace_persistent(const GridView& g, const Io& io
                     io.store((typename Io::Index)item, R, st);
                 }
             }
-            idle = __ballot_sync(0xFFFFFFFFu, !busy);
+            idle = __ballot_sync(0xFFFFFFFFu, !busy) & all;
         }
-        if (!more && idle == 0xFFFFFFFFu) break;
+        if (!more && idle == all) break;
         // One kind of unit per pass: the lanes whose next unit is the more common kind (walk or
         // crossing) run it, the others wait, unless their kind has already waited kUnitWait
         // passes.  A warp then issues one kind's instructions per pass instead of both; every

@@ -566,13 +566,14 @@ __device__ __forceinline__ float sun_ndl(const PathParams& P, uint32_t face) {
 // and the bounce ray appended to the queue of vertex 1.
 __global__ void __launch_bounds__(128, 8) wave_primary_kernel(
     GridView g, vt_camera cam, PathParams P, uint32_t s0, uint32_t sn, uint32_t tiles_x,
-    uint64_t total, vt_ray* __restrict__ nq, uint32_t* __restrict__ nqid,
+    uint64_t total, uint32_t lanes, vt_ray* __restrict__ nq, uint32_t* __restrict__ nqid,
     unsigned int* __restrict__ nqn, WaveState* __restrict__ st, float4* __restrict__ samples,
     unsigned long long* __restrict__ rays_out) {
-    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint64_t thread = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint64_t t = (thread >> 5) * lanes + (thread & 31u);
     bool valid = false;
     uint32_t px = 0, py = 0, smp = 0;
-    if (t < total) {  // t = (tile * sn + sample) * 32 + pixel of the 8 x 4 tile
+    if ((thread & 31u) < lanes && t < total) {  // t = (tile * sn + sample) * 32 + pixel of the 8 x 4 tile
         const uint32_t l = (uint32_t)(t & 31u);
         const uint64_t ts = t >> 5;
         smp = (uint32_t)(ts % sn);
@@ -686,14 +687,18 @@ __global__ void __launch_bounds__(kWaveThreads, 9) wave_trace_kernel(
     GridView g, PathParams P, const vt_ray* __restrict__ q, const unsigned int* __restrict__ qn,
     uint4* __restrict__ hits, const float* __restrict__ so, const uint32_t* __restrict__ sid,
     const unsigned int* __restrict__ sqn, uint8_t* __restrict__ blocked,
-    unsigned long long* __restrict__ counter, uint32_t refill_min,
+    unsigned long long* __restrict__ counter, uint32_t refill_min, int sm_count,
     unsigned long long* __restrict__ rays_out) {
     const uint32_t nb = *qn, ns = *sqn;
     if (rays_out && blockIdx.x == 0 && threadIdx.x == 0)
         atomicAdd(rays_out, (unsigned long long)nb + ns);
     const WaveIo io{g, reinterpret_cast<const float2*>(q), hits, nb, so, sid, blocked,
                     P.sun_dir[0], P.sun_dir[1], P.sun_dir[2]};
-    trace_persistent(g, io, (uint64_t)nb + ns, counter, refill_min);
+    // few rays: spread over more warps, the first of each SM's blocks
+    const uint64_t n = (uint64_t)nb + ns;
+    const uint32_t lanes = lanes_per_warp(n, sm_count);
+    if (lanes < 32u && (uint64_t)(blockIdx.x * (kWaveThreads / 32) + (threadIdx.x >> 5)) * lanes >= n) return;
+    trace_persistent(g, io, n, counter, refill_min, lanes);
 }
 
 // The light of a path's queued sun ray (state S, before its throughput changes), if it is unblocked.
@@ -856,7 +861,8 @@ static cudaError_t launch_path_wave(const GridView& g, const vt_camera& cam, con
         cudaError_t r = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
         if (r != cudaSuccess) return r;
         wave_trace_kernel<<<tblocks, kWaveThreads, 0, st>>>(g, P, q, bounces, hits, sq, sid, suns, blocked,
-                                                            counter, tune.refill_min, rays);
+                                                            counter, tune.refill_min,
+                                                            sm_count, rays);
         return cudaGetLastError();
     };
     for (uint32_t s0 = 0; s0 < P.spp && e == cudaSuccess; s0 += sn) {
@@ -864,8 +870,9 @@ static cudaError_t launch_path_wave(const GridView& g, const vt_camera& cam, con
         const uint64_t items = (uint64_t)tiles_x * tiles_y * n * 32;
         e = cudaMemsetAsync(qn, 0, kWaveCounters * 4, st);
         if (e != cudaSuccess) break;
-        wave_primary_kernel<<<(unsigned)((items + 127) / 128), 128, 0, st>>>(
-            g, cam, P, s0, n, tiles_x, items, q, qid, qn + 1, wst, samples, rays);
+        const uint32_t lanes = lanes_per_warp(items, sm_count);  // 32 / lanes warps per tile and sample
+        wave_primary_kernel<<<(unsigned)((items / lanes + 3) / 4), 128, 0, st>>>(
+            g, cam, P, s0, n, tiles_x, items, lanes, q, qid, qn + 1, wst, samples, rays);
         e = cudaGetLastError();
         for (uint32_t b = 1; b <= P.max_bounces && e == cudaSuccess; ++b) {
             // queue lengths: qn[b] paths at vertex b, qn[b + 1] bounce rays, sqn[b] sun rays of vertex b

@@ -3,6 +3,7 @@
 
 #include <algorithm>
 
+#include "vt_api_internal.h"
 #include "vt_device.cuh"
 #include "vt_kernels.h"
 
@@ -16,23 +17,26 @@ namespace vt {
 constexpr int kTileW = 16, kTileH = 8, kTileThreads = 128;
 
 // Warp tile and block arrangement of a render launch: warp tiles of (1 << wx_log) x
-// (32 >> wx_log) pixels, bx x by of them per block.
+// (lanes >> wx_log) pixels, bx x by of them per block; a warp's lanes from `lanes` on are idle.
 struct RenderShape {
-    uint32_t wx_log, bx, by;
+    uint32_t wx_log, bx, by, lanes;
     uint32_t block_w() const { return bx << wx_log; }
-    uint32_t block_h() const { return by * (32u >> wx_log); }
+    uint32_t block_h() const { return by * (lanes >> wx_log); }
 };
 
-static RenderShape render_shape(const TraceTuning* tune) {
+static RenderShape render_shape(const TraceTuning* tune, uint64_t pixels) {
     static const uint32_t kLog[4] = {3, 2, 4, 5};  // VT_TILE_8X4, 4X8, 16X2, 32X1
-    const uint32_t wx_log = tune && tune->tile_shape < 4 ? kLog[tune->tile_shape] : 3u;
+    uint32_t wx_log = tune && tune->tile_shape < 4 ? kLog[tune->tile_shape] : 3u;
     uint32_t warps = tune ? tune->block_warps : 4u;
     if (warps != 1 && warps != 2 && warps != 8) warps = 4;
+    // small images with the default tile: fewer pixels per warp, in tiles of 4 x 4, 4 x 2, 2 x 2 or 2 x 1
+    uint32_t lanes = 32;
+    if (wx_log == 3 && (lanes = lanes_per_warp(pixels, state().sm_count)) < 32) wx_log = lanes >= 8 ? 2 : 1;
     // warps along x: the power of two that brings the block closest to twice as wide as high
-    RenderShape best{wx_log, 1, warps};
+    RenderShape best{wx_log, 1, warps, lanes};
     double best_err = 1e30;
     for (uint32_t bx = 1; bx <= warps; bx <<= 1) {
-        const RenderShape r{wx_log, bx, warps / bx};
+        const RenderShape r{wx_log, bx, warps / bx, lanes};
         const double aspect = (double)r.block_w() / (double)r.block_h();
         const double err = aspect > 2.0 ? aspect / 2.0 : 2.0 / aspect;
         if (err < best_err) {
@@ -53,11 +57,12 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 8 : 4) render_kernel
                                                      uint32_t row0, uint32_t row1,
                                                      RenderShape shape) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t wx = 1u << shape.wx_log, wy = 32u >> shape.wx_log;
+    const uint32_t wx = 1u << shape.wx_log, wy = shape.lanes >> shape.wx_log;
     const uint32_t px = blockIdx.x * (shape.bx * wx) + (warp % shape.bx) * wx + (lane & (wx - 1u));
     const uint32_t py = row0 + blockIdx.y * (shape.by * wy) + (warp / shape.bx) * wy + (lane >> shape.wx_log);
-    const uint32_t vmask = __ballot_sync(0xFFFFFFFFu, px < cam.width && py < row1);
-    if (px >= cam.width || py >= row1) return;
+    const bool inside = px < cam.width && py < row1 && lane < shape.lanes;
+    const uint32_t vmask = __ballot_sync(0xFFFFFFFFu, inside);
+    if (!inside) return;
     Tally<STATS> tl;
     tl.bind(counters, g.bricks);
     const HitRec h = render_pixel<STATS>(g, cam, light, px, py, vmask, tl);
@@ -69,9 +74,11 @@ template <bool STATS>
 __global__ void __launch_bounds__(256) trace_rays_kernel(GridView g,
                                                          const float2* __restrict__ rays,
                                                          uint64_t n, uint4* __restrict__ out,
-                                                         Counters* __restrict__ counters) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+                                                         Counters* __restrict__ counters,
+                                                         uint32_t lanes) {
+    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint64_t i = (t >> 5) * lanes + (t & 31u);
+    if ((t & 31u) >= lanes || i >= n) return;
     Tally<STATS> tl;
     tl.bind(counters, g.bricks);
     // 24-byte rays: three 8-byte loads
@@ -87,7 +94,7 @@ cudaError_t launch_render(const GridView& g, const vt_camera& cam, const LightVi
                           uint32_t row1, const TraceTuning* tune) {
     if (row1 == 0 || row1 > cam.height) row1 = cam.height;
     if (row0 >= row1) return cudaSuccess;
-    const RenderShape sh = render_shape(tune);
+    const RenderShape sh = render_shape(tune, (uint64_t)cam.width * (row1 - row0));
     const unsigned threads = 32u * sh.bx * sh.by;
     dim3 grid((cam.width + sh.block_w() - 1) / sh.block_w(),
               (row1 - row0 + sh.block_h() - 1) / sh.block_h());
@@ -103,12 +110,14 @@ cudaError_t launch_render(const GridView& g, const vt_camera& cam, const LightVi
 cudaError_t launch_trace_rays(const GridView& g, const vt_ray* rays, uint64_t n, uint4* out,
                               Counters* counters, cudaStream_t stream) {
     if (n == 0) return cudaSuccess;
-    const uint64_t blocks = (n + 255) / 256;
+    // blocks of 128 threads: 1-2% shorter than 32 for a few thousand rays
+    const uint32_t lanes = lanes_per_warp(n, state().sm_count);
+    const uint64_t warps = (n + lanes - 1) / lanes, blocks = (warps + 3) / 4;
     const float2* r2 = reinterpret_cast<const float2*>(rays);
     if (counters)
-        trace_rays_kernel<true><<<(unsigned)blocks, 256, 0, stream>>>(g, r2, n, out, counters);
+        trace_rays_kernel<true><<<(unsigned)blocks, 128, 0, stream>>>(g, r2, n, out, counters, lanes);
     else
-        trace_rays_kernel<false><<<(unsigned)blocks, 256, 0, stream>>>(g, r2, n, out, nullptr);
+        trace_rays_kernel<false><<<(unsigned)blocks, 128, 0, stream>>>(g, r2, n, out, nullptr, lanes);
     return cudaGetLastError();
 }
 
@@ -265,7 +274,7 @@ constexpr int kRayThreads = 128;
 __global__ void __launch_bounds__(kRayThreads, 9) trace_rays_persistent_kernel(
     GridView g, const float2* __restrict__ rays, uint64_t n, uint4* __restrict__ out,
     unsigned long long* __restrict__ counter, uint32_t refill_min) {
-    trace_persistent(g, BufferIo{g, rays, out}, n, counter, refill_min);
+    trace_persistent(g, BufferIo{g, rays, out}, n, counter, refill_min, 32u);
 }
 
 static int resident_blocks(const void* kernel, int threads = 256) {
