@@ -43,13 +43,24 @@ struct BatchLane {
 
 constexpr int kRayQueued = 3;
 
+// Sample `i` of a view: its 16-byte record, or only its colour (COLOURS: the service averages colours
+// and reads nothing else).
+template <bool COLOURS>
+__device__ __forceinline__ void batch_store(const BatchView& V, uint32_t i, const HitRec& h) {
+    if (COLOURS)
+        reinterpret_cast<uint32_t*>(V.out)[i] = h.w3;
+    else
+        V.out[i] = make_uint4(h.w0, h.w1, h.w2, h.w3);
+}
+
 // A ray of the lane ended with `st`: write the sample record, or queue the shadow ray.
+template <bool COLOURS>
 __device__ __forceinline__ void batch_finish(const BatchView& V, BatchLane& s, int st) {
     if (s.kind == 1) {
         HitRec h = ray_record(V.g, s.R, st, VT_SKY_RGBA);
         float nd;
         if (st != kRayHit || !V.light.enabled || !face_lit(h, V.light, nd)) {
-            V.out[s.pix] = make_uint4(h.w0, h.w1, h.w2, h.w3);
+            batch_store<COLOURS>(V, s.pix, h);
             s.kind = 0;
             return;
         }
@@ -62,7 +73,7 @@ __device__ __forceinline__ void batch_finish(const BatchView& V, BatchLane& s, i
             return;
         }
         h.w3 = shade_rgba(h.w3, nd, 1.0f, V.light.ambient);
-        V.out[s.pix] = make_uint4(h.w0, h.w1, h.w2, h.w3);
+        batch_store<COLOURS>(V, s.pix, h);
         s.kind = 0;
         return;
     }
@@ -70,10 +81,11 @@ __device__ __forceinline__ void batch_finish(const BatchView& V, BatchLane& s, i
     HitRec h = s.prim;
     h.w3 = shade_rgba(h.w3, s.ndl, shadowed ? 0.0f : 1.0f, V.light.ambient);
     h.w1 |= (VT_HIT_FLAG_SHADOW_RAY | (shadowed ? VT_HIT_FLAG_SHADOWED : 0u)) << 24;
-    V.out[s.pix] = make_uint4(h.w0, h.w1, h.w2, h.w3);
+    batch_store<COLOURS>(V, s.pix, h);
     s.kind = 0;
 }
 
+template <bool COLOURS>
 __global__ void __launch_bounds__(256, 4) batch_kernel(const BatchView* __restrict__ table,
                                                     uint32_t nviews, uint64_t total,
                                                     unsigned long long* __restrict__ counter,
@@ -152,7 +164,7 @@ __global__ void __launch_bounds__(256, 4) batch_kernel(const BatchView* __restri
                 s.pend = 0;
                 st = ray_begin(V.g, o, d, s.R);
             } else {
-                batch_finish(V, s, st);
+                batch_finish<COLOURS>(V, s, st);
                 st = kRayQueued;
             }
         }
@@ -171,7 +183,7 @@ constexpr int kBatchTileThreads = 128;
 // STATS: the counting build (every reference iteration walked, traversal counters gathered into
 // `counters`; same records), for the roofline's algorithmic bytes.  Nine blocks per SM at 56
 // registers: 16 views over 8 scenes 2.52 ms, ten blocks at 48 (small spills) 2.55, eight 2.53.
-template <bool STATS>
+template <bool STATS, bool COLOURS>
 __global__ void __launch_bounds__(kBatchTileThreads, 9) batch_tile_kernel(const BatchView* __restrict__ table,
                                                          uint32_t nviews, uint64_t units,
                                                          unsigned long long* __restrict__ counter,
@@ -216,8 +228,7 @@ __global__ void __launch_bounds__(kBatchTileThreads, 9) batch_tile_kernel(const 
             jitter(V.seed, V.view_id, px, py, sample, jx, jy);
             raygen(V.cam, px, py, jx, jy, o, d);
             const HitRec h = shade_ray<STATS>(V.g, V.light, o, d, tl);
-            V.out[((py * V.cam.width) + px) * V.spp + sample - V.rec_offset] =
-                make_uint4(h.w0, h.w1, h.w2, h.w3);
+            batch_store<COLOURS>(V, ((py * V.cam.width) + px) * V.spp + sample - V.rec_offset, h);
         }
     }
     if (STATS) tl.flush(counters);
@@ -299,16 +310,14 @@ unsigned batch_blocks(uint32_t n, uint64_t total, const TraceTuning& tune) {
     // a full table (256 views x 208 B) is above the 48 KiB of dynamic shared memory a launch
     // gets without opting in; set on every call (cheap), so that a re-created context has it too
     const int table_max = (int)(kMaxBatchViews * sizeof(BatchView));
-    if (cudaFuncSetAttribute((const void*)batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             table_max) != cudaSuccess ||
-        cudaFuncSetAttribute((const void*)batch_tile_kernel<false>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, table_max) != cudaSuccess ||
-        cudaFuncSetAttribute((const void*)batch_tile_kernel<true>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, table_max) != cudaSuccess)
-        cudaGetLastError();
+    for (const void* k : {(const void*)batch_kernel<false>, (const void*)batch_kernel<true>,
+                          (const void*)batch_tile_kernel<false, false>, (const void*)batch_tile_kernel<false, true>,
+                          (const void*)batch_tile_kernel<true, false>})
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, table_max) != cudaSuccess)
+            cudaGetLastError();
     int per_sm = 0;
     const void* kernel =
-        batch_tile_form(tune) ? (const void*)batch_tile_kernel<false> : (const void*)batch_kernel;
+        batch_tile_form(tune) ? (const void*)batch_tile_kernel<false, false> : (const void*)batch_kernel<false>;
     const int threads = batch_tile_form(tune) ? kBatchTileThreads : 256;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) !=
             cudaSuccess ||
@@ -324,16 +333,18 @@ unsigned batch_blocks(uint32_t n, uint64_t total, const TraceTuning& tune) {
 
 cudaError_t launch_batch(const BatchView* d_table, uint32_t n, uint64_t total,
                          unsigned long long* counter, const TraceTuning& tune, unsigned blocks,
-                         cudaStream_t stream) {
+                         cudaStream_t stream, bool colours) {
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), stream);
     if (e != cudaSuccess) return e;
+    const size_t smem = (size_t)n * sizeof(BatchView);
     if (batch_tile_form(tune)) {
         const uint32_t lanes = lanes_per_warp(total, state().sm_count);
-        batch_tile_kernel<false><<<blocks, kBatchTileThreads, (size_t)n * sizeof(BatchView), stream>>>(
-            d_table, n, total / lanes, counter, nullptr, lanes);
-    } else
-        batch_kernel<<<blocks, 256, (size_t)n * sizeof(BatchView), stream>>>(d_table, n, total,
-                                                                             counter, tune.refill_min);
+        auto* k = colours ? batch_tile_kernel<false, true> : batch_tile_kernel<false, false>;
+        k<<<blocks, kBatchTileThreads, smem, stream>>>(d_table, n, total / lanes, counter, nullptr, lanes);
+    } else {
+        auto* k = colours ? batch_kernel<true> : batch_kernel<false>;
+        k<<<blocks, 256, smem, stream>>>(d_table, n, total, counter, tune.refill_min);
+    }
     return cudaGetLastError();
 }
 
@@ -488,7 +499,7 @@ int32_t vt_batch_stats(int32_t batch, vt_trace_stats* stats) {
         TraceTuning tile = b->tune;
         tile.refill_min = 32;
         const unsigned blocks = batch_blocks(b->nviews, b->total, tile);
-        batch_tile_kernel<true><<<blocks, kBatchTileThreads, b->smem, st>>>(
+        batch_tile_kernel<true, false><<<blocks, kBatchTileThreads, b->smem, st>>>(
             b->d_table, b->nviews, b->total / 32, cursor, dc, 32u);
         e = cudaGetLastError();
     }

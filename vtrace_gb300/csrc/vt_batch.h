@@ -44,9 +44,10 @@ BatchView make_batch_view(const Grid& g, const vt_camera& cam, const vt_light* l
 uint32_t tile_wx_log(uint32_t tile_shape);
 // Blocks of a persistent batched launch over `total` items with an `n`-view table.
 unsigned batch_blocks(uint32_t n, uint64_t total, const TraceTuning& tune);
-// Counter reset + persistent kernel over a device view table.
+// Counter reset + persistent kernel over a device view table.  `colours`: each sample's RGBA8 alone, 4
+// bytes, at the record's index in `out`.
 cudaError_t launch_batch(const BatchView* d_table, uint32_t n, uint64_t total,
                          unsigned long long* counter, const TraceTuning& tune, unsigned blocks,
-                         cudaStream_t stream);
+                         cudaStream_t stream, bool colours = false);
 
 }  // namespace vt
