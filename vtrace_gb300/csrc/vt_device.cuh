@@ -348,7 +348,10 @@ struct SkipRay {
 // Set-up past dda_setup_axis.
 __device__ __forceinline__ void skip_setup(const float d[3], float len, SkipRay& R) {
     R.oshift = (R.stx < 0 ? 4u : 0u) | (R.sty < 0 ? 8u : 0u) | (R.stz < 0 ? 16u : 0u);
-    R.rl = __fdividef(1.0f, len);  // only estimates use it: 0.4% faster than the rounded reciprocal
+    // Only estimates use it: one approximate instruction (the rounded reciprocal: 0.4% of every traversal; a
+    // frame of rays that hit in their first voxel 25.7 -> 24.6 us against __fdividef).  The root of a sum
+    // of squares is 0 or at least 2^-75, so flushing subnormals changes nothing.
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(R.rl) : "f"(len));
     // largest |component|, ties to the lower axis
     const float ax = fabsf(d[0]), ay = fabsf(d[1]), az = fabsf(d[2]);
     R.dom = ax >= ay ? (ax >= az ? 0 : 2) : (ay >= az ? 1 : 2);
