@@ -63,32 +63,33 @@ __global__ void __launch_bounds__(256) update_merge_kernel(GridView g, UpdateBox
     const uint32_t e = g.dir[b];
     const bool was = !brick_empty(e);
     const int32_t z = bzi * 8 + lz;
-    uint64_t word = 0;
+    // Only cells inside the box get new occupancy: the others keep their bits, whatever value stands for a
+    // cell that is not stored (an empty brick has no payload; index 0 may be opaque), and cells past the
+    // grid's faces have none.
+    const uint64_t old_word = was ? g.masks[(size_t)e * 8 + lz] : 0ull;
+    uint64_t word = old_word;
     T* out = payload + k * 512 + lz * 64;
     for (int32_t ly = 0; ly < 8; ++ly) {
         const int32_t y = byi * 8 + ly;
         for (int32_t lx = 0; lx < 8; ++lx) {
             const int32_t x = bxi * 8 + lx;
             T v = 0;
-            if (x < g.nx && y < g.ny && z < g.nz) {
-                if (x >= u.x0 && x < u.x0 + u.w && y >= u.y0 && y < u.y0 + u.h && z >= u.z0 &&
-                    z < u.z0 + u.d) {
-                    v = src[(size_t)(x - u.x0) + (size_t)u.w * ((size_t)(y - u.y0) + (size_t)u.h * (z - u.z0))];
-                } else if (was) {
-                    const size_t li = (size_t)lx + 8 * (ly + 8 * lz);
-                    if (sizeof(T) == 1)
-                        v = (T)g.payload8[(size_t)e * 512 + li];
-                    else
-                        v = (T)g.payload32[(size_t)e * 512 + li];
-                }
+            if (x >= u.x0 && x < u.x0 + u.w && y >= u.y0 && y < u.y0 + u.h && z >= u.z0 && z < u.z0 + u.d) {
+                v = src[(size_t)(x - u.x0) + (size_t)u.w * ((size_t)(y - u.y0) + (size_t)u.h * (z - u.z0))];
+                const uint32_t rgba = sizeof(T) == 1 ? g.palette[(uint32_t)v] : (uint32_t)v;
+                const uint64_t bit = 1ull << (ly * 8 + lx);
+                word = (rgba >> 24) ? word | bit : word & ~bit;
+            } else if (was) {
+                const size_t li = (size_t)lx + 8 * (ly + 8 * lz);
+                if (sizeof(T) == 1)
+                    v = (T)g.payload8[(size_t)e * 512 + li];
+                else
+                    v = (T)g.payload32[(size_t)e * 512 + li];
             }
-            const uint32_t rgba = sizeof(T) == 1 ? g.palette[(uint32_t)v] : (uint32_t)v;
-            if (rgba >> 24) word |= 1ull << (ly * 8 + lx);
             out[ly * 8 + lx] = v;
         }
     }
     words[k * 8 + lz] = word;
-    const uint64_t old_word = was ? g.masks[(size_t)e * 8 + lz] : 0ull;
     const long long delta = (long long)__popcll(word) - (long long)__popcll(old_word);
     if (delta) atomicAdd((unsigned long long*)occ_delta, (unsigned long long)delta);
     // the brick's flag: OR of its 8 slices (lanes 8j..8j+7 of a warp hold one brick, and are
@@ -197,9 +198,9 @@ __global__ void __launch_bounds__(1024) update_small_kernel(GridView g, UpdateBo
     __syncthreads();
     const size_t ex = p.z_fastest ? (size_t)u.d * u.h : 1, ey = p.z_fastest ? (size_t)u.d : (size_t)u.w,
                  ez = p.z_fastest ? 1 : (size_t)u.w * u.h;
-    // row r: brick r >> 6, z-slice (r >> 3) & 7, y r & 7: its voxels after the update; false when the
-    // box does not touch it
-    auto merged = [&](uint32_t r, T v[8]) {
+    // row r: brick r >> 6, z-slice (r >> 3) & 7, y r & 7: its voxels after the update, and which of them
+    // the box holds (a bit each; 0 when it does not touch the row)
+    auto merged = [&](uint32_t r, T v[8]) -> uint32_t {
         int32_t bxi, byi, bzi;
         brick_at(r >> 6, bxi, byi, bzi);
         const uint32_t e = s_old[r >> 6];
@@ -207,24 +208,27 @@ __global__ void __launch_bounds__(1024) update_small_kernel(GridView g, UpdateBo
         const int32_t y = byi * 8 + (int32_t)(r & 7u), z = bzi * 8 + (int32_t)((r >> 3) & 7u);
         const bool in = z >= u.z0 && z < u.z0 + u.d && y >= u.y0 && y < u.y0 + u.h;
         const T* old = payload + ((size_t)(was ? e : 0u) * 64 + (r & 63u)) * 8;
+        uint32_t held = 0;
 #pragma unroll
         for (int32_t lx = 0; lx < 8; ++lx) {
             const int32_t vx = bxi * 8 + lx;
-            if (in && vx >= u.x0 && vx < u.x0 + u.w)
+            if (in && vx >= u.x0 && vx < u.x0 + u.w) {
                 v[lx] = box[ex * (size_t)(vx - u.x0) + ey * (size_t)(y - u.y0) + ez * (size_t)(z - u.z0)];
-            else
+                held |= 1u << lx;
+            } else {
                 v[lx] = was ? old[lx] : (T)0;
+            }
         }
-        return in;
+        return held;
     };
     const uint32_t rows = K * 64;
     for (uint32_t r = t; r < rows; r += blockDim.x) {  // whole warps: half a brick each
         const uint32_t e = s_old[r >> 6];
         const uint32_t before = brick_empty(e) ? 0u : (uint32_t)((const uint8_t*)masks)[(size_t)e * 64 + (r & 63u)];
-        uint32_t bits = before;
+        uint32_t bits = 0;
         T v[8];
-        if (merged(r, v)) {
-            bits = 0;
+        const uint32_t held = merged(r, v);
+        if (held) {
 #pragma unroll
             for (int32_t lx = 0; lx < 8; ++lx) {
                 const bool o = sizeof(T) == 1 ? (s_alpha[(uint32_t)v[lx] >> 5] >> ((uint32_t)v[lx] & 31u)) & 1u
@@ -232,6 +236,7 @@ __global__ void __launch_bounds__(1024) update_small_kernel(GridView g, UpdateBo
                 bits |= (uint32_t)o << lx;
             }
         }
+        bits = (bits & held) | (before & ~held);  // cells outside the box keep theirs (see update_merge_kernel)
         s_bits[r] = (uint8_t)bits;
         const uint32_t some = __ballot_sync(0xFFFFFFFFu, bits != 0u);
         const int delta = __reduce_add_sync(0xFFFFFFFFu, __popc(bits) - __popc(before));
