@@ -630,6 +630,20 @@ void* host_mapped(void* p) {
     return a.devicePointer;
 }
 
+Source source_of(const void* p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return Source::kPageable;
+    }
+    if (a.type == cudaMemoryTypeDevice) return Source::kDevice;
+    return a.type == cudaMemoryTypeUnregistered ? Source::kPageable : Source::kOrdered;
+}
+
+cudaError_t wait_for_source(Source s, cudaStream_t stream) {
+    return s == Source::kOrdered ? cudaStreamSynchronize(stream) : cudaSuccess;
+}
+
 void* device_address(void* p) {
     cudaPointerAttributes a;
     if (!p || cudaPointerGetAttributes(&a, p) != cudaSuccess) {
@@ -810,7 +824,12 @@ static int32_t create_from_host(const void* data, size_t elem, uint32_t format, 
     const int nbuf = order == VT_ORDER_Z_FASTEST ? 2 : 1;
     cudaStream_t st = state().stream;
     const uint64_t bricks = brick_count(nx, ny, nz);
-    if (bricks <= kChunkBricks || (order == VT_ORDER_X_FASTEST && bricks <= kSmallGridBricks)) {
+    // a chunk's voxels are read by the host, those of other small grids by a copy on the stream
+    const Source src = bricks <= kChunkBricks ? source_of(data) : Source::kPageable;
+    if (bricks <= kChunkBricks ? src != Source::kDevice
+                               : order == VT_ORDER_X_FASTEST && bricks <= kSmallGridBricks) {
+        const cudaError_t e = wait_for_source(src, st);
+        if (e != cudaSuccess) return cuda_fail(e, "dense grid upload");
         // straight into the small build's input
         std::unique_ptr<Grid> g;
         if ((rc = build_small_from_host(data, format, order, palette, nx, ny, nz, st, g))) return rc;

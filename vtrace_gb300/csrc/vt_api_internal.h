@@ -112,6 +112,13 @@ void* host_mapped(void* p);
 // through its device mapping; nullptr for memory the device cannot reach (pageable host memory,
 // unknown pointers).
 void* device_address(void* p);
+// What a call that reads a caller's "host" array by the host itself, instead of by a copy on a stream, has
+// to tell apart: pageable memory, which such a copy reads before it returns as well; page-locked or managed
+// memory, which it reads behind the work queued on the stream, possibly what fills it (wait_for_source()
+// waits for that work); and device memory, which only a copy can read.
+enum class Source { kPageable, kOrdered, kDevice };
+Source source_of(const void* p);
+cudaError_t wait_for_source(Source s, cudaStream_t stream);
 LightView light_view(const vt_light* light);
 // Traversal counters of a counting launch as the ABI reports them.
 void stats_from(const Counters& c, vt_trace_stats* st);

@@ -354,7 +354,7 @@ static int32_t grow_slots(Grid& g, uint64_t need, cudaStream_t st) {
 }
 
 // One small update.  The caller has checked the box; its grid is not read or written elsewhere.
-static int32_t update_small(Grid& g, const void* voxels, size_t elem, uint32_t order, const UpdateBox& u) {
+static int32_t update_small(Grid& g, const void* voxels, Source src, size_t elem, uint32_t order, const UpdateBox& u) {
     State& S = state();
     std::lock_guard<std::mutex> lk(S.update_mu);
     if (!S.update_pin) {
@@ -373,9 +373,11 @@ static int32_t update_small(Grid& g, const void* voxels, size_t elem, uint32_t o
     const uint32_t K = (uint32_t)(u.kx * u.ky * u.kz);
     const BrickBox changed = {u.bx0, u.by0, u.bz0, u.kx, u.ky, u.kz};
     const size_t bytes = (size_t)u.w * u.h * u.d * elem, smem = (bytes + 15) / 16 * 16;
+    cudaError_t e = wait_for_source(src, st);
+    if (e != cudaSuccess) return cuda_fail(e, "vt_grid_update");
     memcpy(x->box, voxels, bytes);
     const void* kernel = elem == 1 ? (const void*)update_small_kernel<uint8_t> : (const void*)update_small_kernel<uint32_t>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallBoxBytes);
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallBoxBytes);
     void* scr = nullptr;
     if (e == cudaSuccess) e = cudaMallocAsync(&scr, lattice_scratch_bytes(bx, by, bz), st);
     if (e != cudaSuccess) return cuda_fail(e, "vt_grid_update: scratch");
@@ -459,7 +461,10 @@ extern "C" int32_t vt_grid_update(int32_t grid, const void* voxels, uint32_t ord
     u.kz = ((u.z0 + u.d - 1) >> 3) - u.bz0 + 1;
     const uint64_t K = (uint64_t)u.kx * u.ky * u.kz;
     const size_t box = (size_t)w * h * d * elem;
-    if (K <= kSmallBricks && box <= kSmallBoxBytes) return update_small(*g, voxels, elem, order, u);
+    if (K <= kSmallBricks && box <= kSmallBoxBytes) {
+        const Source src = source_of(voxels);
+        if (src != Source::kDevice) return update_small(*g, voxels, src, elem, order, u);
+    }
     auto al = [](size_t v) { return (v + 255) / 256 * 256; };
     // scratch: box (x2 for reordering), words, payloads, flags, old entries, slots, delta, lattice
     // passes
