@@ -8,6 +8,7 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "vt_api_internal.h"
@@ -140,11 +141,25 @@ void Grid::free_slot_arrays() {
     payload = nullptr;
 }
 
+void wait_for_device() {
+    const int device = state().device;
+    int current = -1;
+    if (cudaGetDevice(&current) == cudaSuccess && current == device) {
+        cudaDeviceSynchronize();
+        return;
+    }
+    cudaGetLastError();
+    // in a thread of its own: setting a device here and back would open a context on the caller's
+    std::thread([device] {
+        if (cudaSetDevice(device) == cudaSuccess) cudaDeviceSynchronize();
+    }).join();
+}
+
 void Grid::release() {
     free_slot_arrays();
     // directory, octant and long-box words, palette (and the first slot arrays)
     if (block && pooled) {
-        cudaDeviceSynchronize();
+        wait_for_device();
         cudaFreeAsync(block, state().stream);
     } else {
         cudaFree(block);

@@ -98,6 +98,10 @@ State& state();
 int32_t ensure_init();
 int32_t cuda_fail(cudaError_t e, const char* what);
 cudaStream_t pick_stream(void* stream);
+// Waits for all work on the library's device, the callers' own streams included, whatever device the
+// calling thread has current (a thread that never set one has device 0).  Memory goes back to the
+// stream-ordered pool only after it: unlike cudaFree, cudaFreeAsync does not wait for other streams.
+void wait_for_device();
 Grid* lookup_grid(int32_t id);
 int32_t register_grid(std::unique_ptr<Grid> g);
 int32_t check_dims(uint32_t nx, uint32_t ny, uint32_t nz);

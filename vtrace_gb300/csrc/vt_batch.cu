@@ -528,7 +528,7 @@ int32_t vt_batch_destroy(int32_t batch) {
         b = std::move(g_batches[batch]);
     }
     cudaStreamSynchronize(state().stream);
-    cudaDeviceSynchronize();
+    wait_for_device();
     batch_free(*b);
     return VT_OK;
 }
