@@ -156,13 +156,14 @@ int32_t vt_device_info(int32_t* device, int32_t* sm_count, uint64_t* free_bytes,
 void* vt_get_stream(void);
 
 /* Launch shape of a tracing entry point.  persistent = 0: one thread per ray, rays packed in
- * 8 x 4 pixel tiles per warp (launches too small to fill the chip give each warp fewer rays, and ray
- * buffers below 196,608 rays always take this form).  persistent = 1: resident warps keep one ray per lane and refill
- * lanes whose rays have ended with new work once at least `refill_min` lanes are idle (1..32;
- * 32 = only when the whole warp is idle), with at most `blocks_per_sm` 256-thread blocks per SM
- * (0 = as many as fit).  VT_KERNEL_BATCH is always persistent; its refill_min 32 (the default)
- * hands warps whole 8 x 4 tile units traced to the end in each lane.  vtrace_gb300.autotune picks
- * them per workload. */
+ * 8 x 4 pixel tiles per warp (launches too small to fill the chip give each warp fewer rays).
+ * persistent = 1: resident warps keep one ray per lane and refill lanes whose rays have ended with
+ * new work once at least `refill_min` lanes are idle (1..32; 32 = only when the whole warp is idle),
+ * with at most `blocks_per_sm` 256-thread blocks per SM (0 = as many as fit).  The built-in tuning of
+ * VT_KERNEL_TRACE_RAYS does so from 196,608 rays on and takes one thread per ray below; any other
+ * tuning installed for it holds at every size.  VT_KERNEL_BATCH is always persistent; its
+ * refill_min 32 (the default) hands warps whole 8 x 4 tile units traced to the end in each lane.
+ * vtrace_gb300.autotune picks them per workload. */
 typedef struct vt_tuning {
     uint32_t refill_min;
     int32_t blocks_per_sm;

@@ -99,7 +99,9 @@ cudaError_t launch_rays(const GridView& g, const vt_ray* rays, uint64_t n, uint4
     // Refilled warps pay from about 200,000 rays on: 256,000 rays in a 512^3 scene 124 us against 132 for
     // one thread per ray (in a 128^3 cave 65 against 62), 131,000 rays 92 against 88 (50 against 39),
     // 64,000 rays 74 against 63: a lane's state costs every unit, and there is little to refill with.
-    if (s.tune_rays.persistent && n >= kPersistentRays)
+    // That holds for the built-in shape; an installed one is taken at every size, or its choice between
+    // candidates on a small buffer would be noise.
+    if (s.tune_rays.persistent && (n >= kPersistentRays || !(s.tune_rays == kTuneRays)))
         return launch_trace_rays_persistent(g, rays, n, out, next_counter(), s.tune_rays,
                                             s.sm_count, stream);
     return launch_trace_rays(g, rays, n, out, nullptr, stream);

@@ -51,6 +51,9 @@ struct Grid {
     void release();
 };
 
+// Built-in launch shape of the ray buffers (see State).
+constexpr TraceTuning kTuneRays{8, 0, 1, 0, VT_TILE_8X4, 4};
+
 struct State {
     std::mutex mu;       // grid table and initialisation
     std::mutex host_mu;  // staging buffer of the *_host calls
@@ -78,11 +81,11 @@ struct State {
     std::atomic<uint32_t> counter_next{0};
     // defaults from sweeps on GB300: coherent camera rays keep their 8 x 4 tiles (refills would
     // mix tiles), incoherent ray buffers and path tracing refill a warp once 8 lanes are idle
-    TraceTuning tune_render{16, 0, 0, 0, VT_TILE_8X4, 4}, tune_rays{8, 0, 1, 0, VT_TILE_8X4, 4},
+    TraceTuning tune_render{16, 0, 0, 0, VT_TILE_8X4, 4}, tune_rays = kTuneRays,
         tune_batch{32, 0, 1, 0, VT_TILE_8X4, 4}, tune_path{8, 0, 1, 1, VT_TILE_8X4, 4};
 };
 
-// Smallest ray buffer that the persistent form takes.
+// Smallest ray buffer that the persistent form takes under the built-in tuning.
 constexpr uint64_t kPersistentRays = 196608;
 constexpr uint32_t kCounterRing = 4096;
 // Work counter for one persistent launch (zeroed by the launcher on its stream).

@@ -20,6 +20,10 @@ struct TraceTuning {
     uint32_t wavefront = 0;    // render only: shadow rays in a second pass over a compacted queue
     uint32_t tile_shape = 0;   // render tile launch: VT_TILE_* pixels per warp
     uint32_t block_warps = 4;  // render tile launch: warps per block (1, 2, 4, 8)
+    bool operator==(const TraceTuning& o) const {
+        return refill_min == o.refill_min && blocks_per_sm == o.blocks_per_sm && persistent == o.persistent &&
+               wavefront == o.wavefront && tile_shape == o.tile_shape && block_warps == o.block_warps;
+    }
 };
 
 // Rays per warp of a launch with one thread per ray.  A launch whose rays fill only a few warps per SM
