@@ -36,13 +36,17 @@ constexpr uint32_t kMaxTextures = 65536;  // lib/common.h:35
 struct CompatInstance {
     float4 row[3];   // inverse(model) row r columns 0..2, om[r]
     float lo[3];
-    float near;      // at most the slab entry parameter tn of any pixel's ray (0: no bound)
+    float near;      // at most the slab entry parameter tn of any pixel's ray (0: no bound; kExactSlab)
     float hi[3];
     int32_t texture;
     int32_t tx0, ty0, tx1, ty1;  // 16 x 16-pixel tiles its pixels can fall in (inclusive; empty
                                  // when tx0 > tx1)
 };
 static_assert(sizeof(CompatInstance) == 96, "float4 loads");
+
+// CompatInstance::near of an instance without a bound whose rays can have components, in model space, of
+// more than 2^125: their reciprocals are subnormal, which the approximate slab test's reciprocal returns as 0.
+constexpr float kExactSlab = -1.0f;
 
 constexpr int32_t kTile = 16;
 // Bitmasks larger than this are not built; every tile then visits every instance.
@@ -198,7 +202,7 @@ __global__ void __launch_bounds__(128, 8) compat_kernel(const GridView* __restri
         // entry face and the exit, one division gives the exact entry parameter instead of six.
         float tn;
         int ax;
-        bool sure = fminf(fminf(fabsf(dm[0]), fabsf(dm[1])), fabsf(dm[2])) > 1e-30f;
+        bool sure = lo.w != kExactSlab && fminf(fminf(fabsf(dm[0]), fabsf(dm[1])), fabsf(dm[2])) > 1e-30f;
         const bool px_ = dm[0] > 0.0f, py_ = dm[1] > 0.0f, pz_ = dm[2] > 0.0f;
         const float nx = px_ ? lo.x : hi.x, ny = py_ ? lo.y : hi.y, nz = pz_ ? lo.z : hi.z;
         if (sure) {
@@ -697,6 +701,7 @@ __global__ void __launch_bounds__(128) compat_prepare_kernel(const float* __rest
 #pragma unroll
         for (int k = 0; k < 15; ++k) affine = affine && isfinite(m[k]);
         if (affine ? invert_affine(md, mi) : invert4(md, mi)) {
+            bool huge = false;  // a row that can give a component above 2^125 (world rays have unit length)
 #pragma unroll
             for (int r = 0; r < 3; ++r) {
                 const float a0 = (float)mi[r], a1 = (float)mi[4 + r], a2 = (float)mi[8 + r], a3 = (float)mi[12 + r];
@@ -704,12 +709,13 @@ __global__ void __launch_bounds__(128) compat_prepare_kernel(const float* __rest
                                                                __fmul_rn(a1, (float)cf.cam[1])),
                                                      __fmul_rn(a2, (float)cf.cam[2])), a3);
                 ci.row[r] = make_float4(a0, a1, a2, om);
+                huge |= !(fabsf(a0) + fabsf(a1) + fabsf(a2) < 0x1p125f);
                 ci.lo[r] = __fsub_rn(-0.5f, om);
                 ci.hi[r] = __fsub_rn(0.5f, om);
             }
             ci.texture = tid;
             const ModelCamera mc = model_camera(cf, mi);
-            ci.near = instance_near(cf, m, mi, mc);
+            ci.near = huge ? kExactSlab : instance_near(cf, m, mi, mc);
             int seen = instance_tiles_f32(cf, m, md, mc, ci.tx0, ci.ty0, ci.tx1, ci.ty1);
             if (seen < 0) seen = instance_tiles(cf, insts + 16 * (size_t)i, ci.tx0, ci.ty0, ci.tx1, ci.ty1);
             if (!seen) {
