@@ -1,8 +1,11 @@
 """render_tick instances whose matrices lie near the ends of binary32's range, where the approximate
-arithmetic of the slab test leaves it: a plate 3e-39 thick, whose inverse has elements of 3e38 (the reciprocals
-of a ray's components in it are subnormal).  Every pixel equals the oracle's loop over every instance."""
+arithmetic of the culling and of the slab test leaves it: a plate 3e-39 thick, whose inverse has elements of
+3e38 (the reciprocals of a ray's components in it are subnormal), and a floor 3e37 long seen through a
+narrow projection (its far corners' products overflow).  Every pixel equals the oracle's loop over every
+instance."""
 import ctypes
 import math
+import struct
 
 import numpy as np
 import pytest
@@ -52,3 +55,18 @@ def test_thin_instances_equal_the_oracle(lib, monkeypatch, scale):  # noqa: F811
              instance(0, (0, 1, 0), scale, (-0.2, 0.1, -0.35), 0)]
     check(lib, monkeypatch, [PLATE, BLOCK], insts, perspective(math.radians(80.0), W / H, 0.01, 200.0),
           look_at((0.4, 0.3, 0.5), (0.0, 0.0, -1.0), (0.0, 1.0, 0.0)))
+
+
+@pytest.mark.parametrize("side", [-2e33, 2e33])
+@pytest.mark.parametrize("far", [1.5e37, 2e37])
+def test_huge_instances_equal_the_oracle(lib, monkeypatch, side, far):  # noqa: F811
+    fov, near = math.radians(2.0), 3e35
+    f, r, up = np.array([1, 0, -1]) / math.sqrt(2), np.array([1, 0, 1]) / math.sqrt(2), np.array([0, 1, 0])
+    k = math.tan(fov / 2) * W / H
+    a, b = (f * z + r * (z * k * xn) + up * side for z, xn in ((near, -0.8), (far, 0.8)))
+    M = np.eye(4)
+    M[:3] = np.stack([b - a, up * 1e22, r * (k * 0.3 * near), (a + b) / 2], 1)
+    cm = np.ascontiguousarray(M.T, np.float32).reshape(16)
+    cm[15] = struct.unpack("<f", struct.pack("<i", 0))[0]
+    check(lib, monkeypatch, [PLATE], [cm], perspective(fov, W / H, 0.01, 200.0),
+          look_at((0, 0, 0), (1, 0, -1), (0, 1, 0)))

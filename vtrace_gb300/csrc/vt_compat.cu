@@ -488,6 +488,7 @@ static __device__ float instance_near(const CullFrame& cf, const float* m, const
     }
     const float dist = sqrtf(mc.d2), cond = sqrtf(fm) * sqrtf(mc.fro), n2 = sqrtf(n1) * sqrtf(ninf);
     if (!(dist > 1.001f / 256.0f) || !(cond <= 1023.0f) || !(n2 > 0.0f) || !isfinite(dist)) return 0.0f;
+    if (!(fm > 1e-30f) || !(mc.fro > 1e-30f)) return 0.0f;  // subnormal squares: cond is not within 0.1%
     const float near = 0.989f * dist / n2;
     return isfinite(near) ? near : 0.0f;
 }
@@ -500,15 +501,17 @@ static __device__ float instance_near(const CullFrame& cf, const float* m, const
 // and S bounds the terms of X - cam (binary32 sums of at most seven terms and products err by less than
 // 8 x 2^-24 of their sum of magnitudes; twice that is taken).  Visible points have q.z >= eps, so their
 // counterparts have q.z >= eps / 2 provided eps >= 64 E.z: the rectangle of the hull clipped there,
-// each vertex p widened by (2 E.x + 2 |p.x / p.z| E.z) / p.z, holds all their projections.
+// each vertex p widened by (2 E.x + 2 |p.x / p.z| E.z) / p.z, holds all their projections.  The bounds are
+// relative: where a sum could overflow (|row of B^-1|_1 S of 10^37; infinities and NaN would drop out of the
+// minima) or lies near the subnormals (fro or eps of 10^-30), binary64 decides.
 static __device__ int instance_tiles_f32(const CullFrame& cf, const float* m, const double* md,
                                          const ModelCamera& mc, int32_t& tx0, int32_t& ty0,
                                          int32_t& tx1, int32_t& ty1) {
     if (!cf.ok) return -1;
-    if (!(mc.d2 > 1e-12f) || !(mc.fro > 0.0f) || !isfinite(mc.d2) || !isfinite(mc.fro)) return -1;
+    if (!(mc.d2 > 1e-12f) || !(mc.fro > 1e-30f) || !isfinite(mc.d2) || !isfinite(mc.fro)) return -1;
     // 1% below the binary64 path's bound
     const float eps = 0.495f * sqrtf(mc.d2 / mc.fro) / (float)cf.len_max;
-    float S = 0.0f, t[3], bi[9], E[3];
+    float S = 0.0f, t[3], bi[9], E[3], most = 0.0f;
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
         t[r] = (float)(md[3 * 4 + r] - cf.cam[r]);
@@ -523,8 +526,9 @@ static __device__ int instance_tiles_f32(const CullFrame& cf, const float* m, co
             n += fabsf(bi[3 * r + k]);
         }
         E[r] = 0x1p-20f * n * S;
+        most = fmaxf(most, n * S);
     }
-    if (!(eps >= 64.0f * E[2]) || !isfinite(S)) return -1;
+    if (!(eps >= 64.0f * E[2]) || !(eps > 1e-30f) || !(S < 1e37f) || !(most < 1e37f)) return -1;
     // corners in q space
     float q[8][3];
 #pragma unroll
