@@ -357,9 +357,13 @@ __device__ __forceinline__ void skip_setup(const float d[3], float len, SkipRay&
     R.dom = ax >= ay ? (ax >= az ? 0 : 2) : (ay >= az ? 1 : 2);
 }
 
-// Directions the skipping traversal hands to the literal loop: a NaN side distance, or none finite.
+// Directions the skipping traversal hands to the literal loop: a side distance that is NaN or negative, or
+// none finite.  The rounding of an entry test can leave a point just past the face a ray points to, which makes
+// that axis's first side negative: -inf where the direction's squares overflow, and -inf + inf is NaN, after
+// which no axis may step.  From sides of at least 0 every sum is a number, and an axis that steps has
+// a finite side or is one of three that are +inf.
 __device__ __forceinline__ bool skip_degenerate(float sx, float sy, float sz) {
-    return isnan(sx) || isnan(sy) || isnan(sz) || !(fminf(fminf(sx, sy), sz) < INFINITY);
+    return !(sx >= 0.0f) || !(sy >= 0.0f) || !(sz >= 0.0f) || !(fminf(fminf(sx, sy), sz) < INFINITY);
 }
 
 __device__ __forceinline__ uint32_t skip_brick(const GridView& g, const SkipRay& R) {
