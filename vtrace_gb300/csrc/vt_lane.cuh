@@ -53,9 +53,7 @@ __device__ __forceinline__ int ray_begin(const GridView& g, const float o[3], co
     dda_setup_axis(pos[2], d[2], g.nz, len, S.vz, S.stz, S.dlz, S.sz);
     if (skip_degenerate(S.sx, S.sy, S.sz)) {
         DDAResult r;
-        Tally<false> tl;
-        dda_literal<false>(g, S.vx, S.vy, S.vz, S.stx, S.sty, S.stz, S.dlx, S.dly, S.dlz, S.sx, S.sy,
-                           S.sz, r, tl);
+        dda_degenerate(g, S, r);
         S.vx = r.vx;
         S.vy = r.vy;
         S.vz = r.vz;
