@@ -371,24 +371,43 @@ cudaError_t launch_brick_words(const void* src, uint32_t format, const uint32_t*
 // A warp per 32 bricks.  Bound by copying the payloads: 102 MB and their words in and out in 42 us,
 // 5.9 TB/s (74 us with a thread per slice of every brick, of which nine in ten found an empty one;
 // 58 us with one brick at a time per warp).
-template <uint32_t FMT>
+//
+// Lattices of few bricks have few such warps, and a warp takes its bricks four after four: below
+// kSplitGroups groups of 32 each group is split over eight warps that take four bricks each
+// (vt_grid_build_u8_noalloc of 64^3 terrain 57.5 -> 40.6 us, of 256^3 67.5 -> 52.8, and 34.2 and 50.5
+// with the counts written here instead of by two copies; a graph-built 64^3 grid 79.9 -> 64.7; from 2,048
+// groups on, 384^3 and 512^3, the two measure the same).
+constexpr uint64_t kSplitGroups = 2048;
+
+template <uint32_t FMT, uint32_t SPLIT>
 __global__ void __launch_bounds__(256) brick_compact_kernel(
     const void* __restrict__ src, int32_t nx, int32_t ny, int32_t nz, int32_t bx, int32_t by,
     uint64_t bricks, const uint64_t* __restrict__ words, const uint32_t* __restrict__ occ,
     const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ block_sums,
     uint32_t* __restrict__ dir, uint64_t* __restrict__ masks, void* __restrict__ payload,
-    const void* __restrict__ staged) {
+    const void* __restrict__ staged, const unsigned long long* __restrict__ counts,
+    uint64_t* __restrict__ counts_out) {
     constexpr size_t E = FMT == VT_PAYLOAD_RGBA8 ? 4 : 1;
+    if (counts_out && blockIdx.x == 0 && threadIdx.x < 2) counts_out[threadIdx.x] = counts[1 - threadIdx.x];
     const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t group = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, b0 = group * 32;
+    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint64_t group = warp / SPLIT, b0 = group * 32;
     if (b0 >= bricks) return;  // whole warps
     uint32_t left = __ldg(occ + group);
     uint32_t slot = first_slot(offsets, block_sums, group);
-    if (b0 + lane < bricks)  // distance filled in by the lattice passes
+    const uint32_t part = (uint32_t)(warp % SPLIT);
+    if (part == 0u && b0 + lane < bricks)  // distance filled in by the lattice passes
         dir[b0 + lane] = (left >> lane) & 1u ? slot + __popc(left & ((1u << lane) - 1u)) : kEmptyBit;
     // four occupied bricks at a time, eight lanes each; staged blocks in pieces of 128 contiguous
     // bytes per brick and load, all of a lane's loads in flight together
     const uint32_t mine = lane >> 3, lz = lane & 7u;
+    if (SPLIT != 1u) {  // the bricks of this part: four from the 4 * part-th on
+        for (uint32_t k = 0; k < 4u * part; ++k) left &= left ? left - 1u : 0u;
+        uint32_t rest = left;
+        for (uint32_t k = 0; k < 4u; ++k) rest &= rest ? rest - 1u : 0u;
+        left ^= rest;
+        slot += 4u * part;
+    }
     for (; left; slot += 4) {
         uint32_t at = 32;
 #pragma unroll
@@ -418,18 +437,16 @@ __global__ void __launch_bounds__(256) brick_compact_kernel(
 
 cudaError_t launch_brick_compact(const void* src, uint32_t format, int32_t nx, int32_t ny,
                                  int32_t nz, const BuildScratch& s, uint32_t* dir,
-                                 uint64_t* masks, void* payload, cudaStream_t stream) {
+                                 uint64_t* masks, void* payload, cudaStream_t stream, uint64_t* counts_out) {
     const int32_t bx = (nx + 7) / 8, by = (ny + 7) / 8, bz = (nz + 7) / 8;
     const uint64_t bricks = (uint64_t)bx * by * bz;
-    const unsigned blocks = (unsigned)((occ_count(bricks) + 7) / 8);
-    if (format == VT_PAYLOAD_U8)
-        brick_compact_kernel<VT_PAYLOAD_U8><<<blocks, 256, 0, stream>>>(
-            src, nx, ny, nz, bx, by, bricks, s.words, s.occ, s.offsets, s.block_sums, dir, masks, payload,
-            s.staged);
-    else
-        brick_compact_kernel<VT_PAYLOAD_RGBA8><<<blocks, 256, 0, stream>>>(
-            src, nx, ny, nz, bx, by, bricks, s.words, s.occ, s.offsets, s.block_sums, dir, masks, payload,
-            s.staged);
+    const bool split = occ_count(bricks) < kSplitGroups;
+    const unsigned blocks = (unsigned)((occ_count(bricks) * (split ? 8 : 1) + 7) / 8);
+    auto* k = format == VT_PAYLOAD_U8
+                  ? (split ? brick_compact_kernel<VT_PAYLOAD_U8, 8> : brick_compact_kernel<VT_PAYLOAD_U8, 1>)
+                  : (split ? brick_compact_kernel<VT_PAYLOAD_RGBA8, 8> : brick_compact_kernel<VT_PAYLOAD_RGBA8, 1>);
+    k<<<blocks, 256, 0, stream>>>(src, nx, ny, nz, bx, by, bricks, s.words, s.occ, s.offsets, s.block_sums, dir,
+                                  masks, payload, s.staged, s.counts, counts_out);
     return cudaGetLastError();
 }
 

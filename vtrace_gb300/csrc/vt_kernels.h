@@ -111,10 +111,12 @@ cudaError_t launch_brick_scan(const BuildScratch& s, uint64_t bricks, cudaStream
 // the x and z axes.  grid.y = ceil(nx / 32) and grid.z = ny must stay within 65535.
 cudaError_t launch_transpose_xz(const void* src, void* dst, size_t elem, int32_t nx, int32_t ny,
                                 int32_t nz, cudaStream_t stream);
-// Phase 3: directory, compacted masks and payloads.
+// Phase 3: directory, compacted masks and payloads.  `counts_out` (device), or nullptr: occupied bricks,
+// occupied voxels.
 cudaError_t launch_brick_compact(const void* src, uint32_t format, int32_t nx, int32_t ny,
                                  int32_t nz, const BuildScratch& s, uint32_t* dir,
-                                 uint64_t* masks, void* payload, cudaStream_t stream);
+                                 uint64_t* masks, void* payload, cudaStream_t stream,
+                                 uint64_t* counts_out = nullptr);
 
 // Words, slots, masks, payloads, directory and palette of a grid of up to kChunkBricks bricks in one
 // block.  `src` (either element order), `palette` and `counts` (occupied voxels, occupied bricks) are

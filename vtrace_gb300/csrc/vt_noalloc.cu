@@ -82,12 +82,8 @@ extern "C" int32_t vt_grid_build_u8_noalloc(const uint8_t* d_voxels, const uint3
                            (int32_t)nz, s, st) != cudaSuccess ||
         launch_brick_scan(s, bricks, st) != cudaSuccess ||
         launch_brick_compact(d_voxels, VT_PAYLOAD_U8, (int32_t)nx, (int32_t)ny, (int32_t)nz, s,
-                             d_directory, d_masks, d_payload, st) != cudaSuccess ||
+                             d_directory, d_masks, d_payload, st, d_counts) != cudaSuccess ||
         launch_brick_distance(d_directory, nullptr, s.lattice, bx, by, bz, st) != cudaSuccess)
-        return VT_ECUDA;
-    // d_counts: occupied bricks, occupied voxels
-    if (cudaMemcpyAsync(d_counts, s.counts + 1, 8, cudaMemcpyDeviceToDevice, st) != cudaSuccess ||
-        cudaMemcpyAsync(d_counts + 1, s.counts, 8, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
         return VT_ECUDA;
     return VT_OK;
 }
