@@ -222,7 +222,7 @@ static void point_into_block(Grid& g, void* block, const BlockLayout& L, uint64_
 }
 
 // The brick build's launches on `stream` (captured): occupancy words, slot scan, compaction into dir /
-// masks / payload, octant words, long-box words and distances below 15.
+// masks / payload, octant words, long-box words and distances.
 static cudaError_t build_launches(const void* d_src, uint32_t format, const uint32_t* d_palette,
                                   bool nonzero, const Grid& g, const BuildScratch& s,
                                   cudaStream_t stream) {
@@ -246,6 +246,7 @@ static cudaError_t build_launches(const void* d_src, uint32_t format, const uint
 // serialised by g_small_mu.
 // ---------------------------------------------------------------------------------------------
 constexpr uint64_t kSmallGridBricks = 512;  // 64^3 voxels: at most 1 MiB of unused slots
+static_assert(kSmallGridBricks <= kDirectBricks && kChunkBricks <= kDirectBricks, "the lattice passes settle all distances");
 constexpr size_t kSmallGraphs = 64;
 
 struct SmallBuild {
@@ -324,12 +325,8 @@ static int32_t build_chunk(const void* src, bool src_host, uint32_t order, const
                                        g_chunk_dev->counts, stream);
     if (e == cudaSuccess) e = launch_brick_lattice(g.dir, g.oct, g.lng, ls, bx, by, bz, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    if (e == cudaSuccess && g_chunk->deep) {
-        g.deep = true;
-        e = launch_brick_distance(g.dir, g.oct, ls, bx, by, bz, stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    }
     if (e != cudaSuccess) return cuda_fail(e, "chunk build");
+    g.deep = g_chunk->deep != 0;
     g.occupied = g_chunk->counts[0];
     g.nonempty = g_chunk->counts[1];
     g.bytes = g.block_bytes;
@@ -440,14 +437,8 @@ static int32_t build_small(const void* src, bool src_host, uint32_t order, const
     if (e == cudaSuccess) e = cudaMemcpyAsync(block, b->tmpl, L.total, cudaMemcpyDeviceToDevice, stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(hc, b->counts, 20, cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    if (e == cudaSuccess && hc[4]) {  // bricks far from all occupied ones: settle their distances
-        g->deep = true;
-        const int32_t bx = (int32_t)g->bx, by = (int32_t)g->by, bz = (int32_t)g->bz;
-        const BuildScratch s = carve_build_scratch(b->scratch, bx, by, bz);
-        e = launch_brick_distance(g->dir, g->oct, s.lattice, bx, by, bz, stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    }
     if (e != cudaSuccess) return cuda_fail(e, "small grid build");
+    g->deep = hc[4] != 0;
     g->nonempty = (uint64_t)hc[2] | ((uint64_t)hc[3] << 32);
     g->occupied = (uint64_t)hc[0] | ((uint64_t)hc[1] << 32);
     g->bytes = g->block_bytes;

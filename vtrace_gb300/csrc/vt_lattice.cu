@@ -15,7 +15,8 @@
 // and the centred cube of radius r < 15 is the union of the eight octants' cubes of side r + 1, so
 //   D         = the smallest K of the eight octants when that is below 15
 // Bricks whose eight octants all reach the cap (empty in all directions for 15 bricks) are left to
-// the separable distance passes at the end of this file, which the host launches when there are any.
+// the separable distance passes at the end of this file, which the host launches when there are any; in
+// lattices of few bricks the x pass looks at all rows for them.
 //
 // A block takes 32 bricks along the axis x 8 x 8 rows.  It reads the 36 x 36 rows within reach as
 // 62-bit windows, builds the ORs of 2^p x 2^p rows (p = 0..3) in shared memory, from which M(k, q)
@@ -28,6 +29,8 @@
 // together 90 us where per-brick walks (distances, octants) and a pyramid of run minima (long
 // boxes) took 615 us; after a 16^3 chunk's update 28 us where they took 110 us.
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "vt_device.cuh"
 #include "vt_kernels.h"
@@ -196,7 +199,42 @@ __device__ __forceinline__ uint32_t run_backward(uint64_t m, uint32_t lane) {
     return (uint32_t)__clz((int)((uint32_t)((m << (48u - lane)) >> 32) | 0x10000u));
 }
 
-// Axis x: octant words, distances below 15 of empty bricks, and the long-box words along x.
+// Distance along x from brick x to the nearest occupied brick of its row, at most `cap` (<= 31).
+__device__ __forceinline__ int32_t row_distance(const uint32_t* __restrict__ row, int32_t rw,
+                                                int32_t x, int32_t cap) {
+    const int32_t w = x >> 5, b = x & 31;
+    const uint64_t mid = __ldg(row + w);
+    const uint64_t up = (mid | (w + 1 < rw ? (uint64_t)__ldg(row + w + 1) << 32 : 0ull)) >> b;
+    const uint64_t down = ((mid << 32) | (w > 0 ? (uint64_t)__ldg(row + w - 1) : 0ull)) << (31 - b);
+    const int32_t f = up ? __ffsll((long long)up) - 1 : cap;      // bit k: brick x + k
+    const int32_t g = down ? __clzll((long long)down) : cap;      // bit 63 - k: brick x - k
+    return min(cap, min(f, g));
+}
+
+// Distance of a brick over the rows in reach of a lattice of few bricks; four rows' loads in flight.
+__device__ __forceinline__ uint32_t direct_distance(const uint32_t* __restrict__ rows, int32_t x, int32_t y,
+                                                    int32_t z, int32_t by, int32_t bz, int32_t rw) {
+    constexpr int32_t R = (int32_t)kMaxBrickDistance;
+    int32_t best = R;
+    const int32_t y0 = max(y - R + 1, 0), y1 = min(y + R, by);
+    for (int32_t k = max(z - R + 1, 0); k < min(z + R, bz); ++k)
+#pragma unroll 4
+        for (int32_t j = y0; j < y1; ++j) {
+            const int32_t d = row_distance(rows + (uint64_t)(k * by + j) * rw, rw, x, R);
+            best = min(best, max(max(abs(j - y), abs(k - z)), d));
+        }
+    return (uint32_t)best;
+}
+
+// What the x pass does with the distance of a brick whose octants all reach the cap.
+enum class FarBricks {
+    kLater,  // 15: the distance passes settle it
+    kNone,   // 31: the lattice has at most 15 bricks along each axis, so those 14 around are all of it
+    kHere,   // looks at all rows
+};
+
+// Axis x: octant words, distances of empty bricks, and the long-box words along x.
+template <FarBricks FAR>
 __global__ void __launch_bounds__(kLatticeThreads) lattice_x_kernel(
     LatticeScratch s, uint32_t* __restrict__ dir, uint32_t* __restrict__ oct,
     uint32_t* __restrict__ lng, int32_t bx, int32_t by, int32_t bz, BrickBox w) {
@@ -259,8 +297,13 @@ __global__ void __launch_bounds__(kLatticeThreads) lattice_x_kernel(
             const uint64_t b = (uint64_t)x + (uint64_t)bx * ((uint64_t)y + (uint64_t)by * (uint64_t)z);
             oct[b] = ow;
             lng[b] = lw;
-            if (least) dir[b] = kEmptyBit | least;  // 15: the distance passes settle it
-            far |= least == (uint32_t)kCap;
+            uint32_t D = least;
+            if (least == (uint32_t)kCap) {
+                if (FAR == FarBricks::kNone) D = kMaxBrickDistance;
+                if (FAR == FarBricks::kHere) D = direct_distance(s.rows[0], x, y, z, by, bz, row_words(bx));
+                far = FAR != FarBricks::kNone;
+            }
+            if (least) dir[b] = kEmptyBit | D;
         }
     }
     if (far) *s.deep = 1u;
@@ -353,18 +396,6 @@ __device__ __forceinline__ bool box_brick(const BrickBox& box, int32_t bx, int32
     z = box.z0 + (int32_t)(r / (uint64_t)box.ny);
     b = (uint64_t)x + (uint64_t)bx * ((uint64_t)y + (uint64_t)by * (uint64_t)z);
     return true;
-}
-
-// Distance along x from brick x to the nearest occupied brick of its row, at most `cap` (<= 31).
-__device__ __forceinline__ int32_t row_distance(const uint32_t* __restrict__ row, int32_t rw,
-                                                int32_t x, int32_t cap) {
-    const int32_t w = x >> 5, b = x & 31;
-    const uint64_t mid = __ldg(row + w);
-    const uint64_t up = (mid | (w + 1 < rw ? (uint64_t)__ldg(row + w + 1) << 32 : 0ull)) >> b;
-    const uint64_t down = ((mid << 32) | (w > 0 ? (uint64_t)__ldg(row + w - 1) : 0ull)) << (31 - b);
-    const int32_t f = up ? __ffsll((long long)up) - 1 : cap;      // bit k: brick x + k
-    const int32_t g = down ? __clzll((long long)down) : cap;      // bit 63 - k: brick x - k
-    return min(cap, min(f, g));
 }
 
 __global__ void __launch_bounds__(256) lattice_distance_xy_kernel(const uint32_t* __restrict__ rows,
@@ -470,8 +501,13 @@ cudaError_t launch_brick_lattice(uint32_t* dir, uint32_t* oct, uint32_t* lng,
                                  cudaStream_t stream, const BrickBox* changed) {
     // above 48 KiB of dynamic shared memory: opted in on every call (cheap), so that a re-created
     // context has it too
-    cudaError_t e = cudaFuncSetAttribute((const void*)lattice_x_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLatticeShared);
+    auto* x_kernel = lattice_x_kernel<FarBricks::kLater>;
+    if (std::max({bx, by, bz}) <= kCap)
+        x_kernel = lattice_x_kernel<FarBricks::kNone>;
+    else if (!changed && (uint64_t)bx * by * bz <= kDirectBricks)  // (after a change not all rows are there)
+        x_kernel = lattice_x_kernel<FarBricks::kHere>;
+    cudaError_t e = cudaFuncSetAttribute((const void*)x_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)kLatticeShared);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute((const void*)lattice_yz_kernel,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLatticeShared);
@@ -481,8 +517,7 @@ cudaError_t launch_brick_lattice(uint32_t* dir, uint32_t* oct, uint32_t* lng,
     // there read rows up to 14 further out
     const BrickBox w = changed ? grow(*changed, kHalo, kHalo, kHalo, bx, by, bz) : all;
     launch_rows(dir, s, bx, by, bz, changed ? grow(w, kCap, kCap, kCap, bx, by, bz) : all, stream);
-    lattice_x_kernel<<<tiles(w.nx, w.ny, w.nz), kLatticeThreads, kLatticeShared, stream>>>(
-        s, dir, oct, lng, bx, by, bz, w);
+    x_kernel<<<tiles(w.nx, w.ny, w.nz), kLatticeThreads, kLatticeShared, stream>>>(s, dir, oct, lng, bx, by, bz, w);
     const unsigned ty = tiles(w.ny, w.nx, w.nz), tz = tiles(w.nz, w.nx, w.ny);
     lattice_yz_kernel<<<ty + tz, kLatticeThreads, kLatticeShared, stream>>>(s, oct, lng, bx, by, bz, w, ty);
     return cudaGetLastError();
