@@ -142,7 +142,8 @@ typedef struct vt_trace_stats {
 /* Select the CUDA device and create the library's stream.  Optional: every other call initialises
  * the library on device 0 when needed.  Returns VT_OK or VT_ECUDA. */
 int32_t vt_init(int32_t device);
-/* Free every grid, batch and buffer and destroy the library's stream. */
+/* Free every grid, batch and buffer, give the stream-ordered pool's memory back and destroy the
+ * library's stream. */
 void vt_shutdown(void);
 /* Message for the calling thread's most recent failed call ("" if none). */
 const char* vt_last_error(void);
@@ -205,7 +206,7 @@ int32_t vt_grid_create_u8(const uint8_t* voxels, const uint32_t* palette,
                           uint32_t nx, uint32_t ny, uint32_t nz);
 /* Same, with the voxel array already in device memory (x-fastest, nx*ny*nz bytes, left unchanged);
  * the palette is host memory.  The build runs on `stream`; the call returns after the build has
- * finished.  Device memory during any build of more than 512 bricks: besides the grid, about 75
+ * finished.  Device memory during any build of more than 512 bricks: besides the grid, about 64
  * bytes of scratch per brick and, when it fits, a staging buffer as large as the dense array
  * padded to whole bricks, released (to the stream-ordered pool) when the call returns; without
  * room for the staging buffer the build reads the dense array twice instead. */
@@ -229,6 +230,10 @@ int32_t vt_grid_create_rgba8(const uint8_t* rgba, uint32_t nx, uint32_t ny, uint
  * add_texture's, and VT_ORDER_Z_FASTEST is the geometrically faithful reading. */
 int32_t vt_grid_create(const void* voxels, uint32_t format, uint32_t order,
                        const uint32_t* palette, uint32_t nx, uint32_t ny, uint32_t nz);
+/* Free a grid, once all work on the library's device has ended (VT_EBUSY while a batch or a service
+ * references it).  Its memory goes back to the device's default stream-ordered pool, which keeps up to
+ * 4 GiB of freed memory for the next build: for everything else on the device that is taken
+ * (cudaMemGetInfo counts it) until vt_shutdown gives it back. */
 int32_t vt_grid_destroy(int32_t grid);
 /* Chunk paging (src/gen/pager.rs:52-78, one chunk per frame at src/render.rs:246-261): write a
  * w x h x d box of voxels (host memory, `order`; u8 palette indices for VT_PAYLOAD_U8 grids,
@@ -423,11 +428,13 @@ int32_t vt_batch_destroy(int32_t batch);
  * launch as launch slots free up; each piece's samples are averaged into its rows of the request's
  * RGBA8 image in the caller's host buffer, and a request is done when its last piece is.  Scene
  * brick grids stay resident in a cache built on first use, least-recently-used unreferenced scenes
- * evicted.  hbm_budget_bytes bounds the resident grids plus the launch slots' sample buffers
- * (max_inflight x max_samples_per_launch x 20 bytes, allocated at start) plus the temporary buffer
- * of any piece larger than a slot's; a scene is admitted against the size its grid would have with
- * every brick occupied, then counted at its real size.  While a scene's grid is built the device
- * also holds its voxel array and the build's scratch for a moment; those are outside the budget.
+ * evicted.  hbm_budget_bytes bounds the resident grids plus a charge of 20 bytes per sample for the
+ * launch slots' buffers (max_inflight x max_samples_per_launch; allocated at start, 8 bytes per sample) and
+ * for the temporary buffer of any piece larger than a slot's; a scene is admitted against the size its
+ * grid would have with every brick occupied, then counted at its real size.  While a scene's grid is
+ * built the device also holds its voxel array and the build's scratch for a moment; those are outside the
+ * budget, as is what evicted grids leave in the stream-ordered pool (at most 4 GiB, see
+ * vt_grid_destroy).
  * max_inflight = 1, max_views_per_launch = 1 and max_samples_per_piece = 0 is the plain
  * per-request baseline. */
 typedef struct vt_serve_config {

@@ -43,6 +43,12 @@
 
 namespace vt {
 
+// Bytes of a launch's buffers per sample, and the bytes per sample that the HBM budget is charged for
+// them: a fixed part of the budget's rule (include/vtrace.h), by which a budget that is refused stays refused
+// and scenes are evicted at the same point, and never less than what is allocated.
+constexpr uint64_t kSampleBytes = 8, kChargedBytes = 20;
+static_assert(kSampleBytes <= kChargedBytes, "the budget bounds the allocations");
+
 struct ResolveView {
     const uint32_t* samples;
     uchar4* image;
@@ -143,7 +149,7 @@ struct Slot {
     ResolveView* h_resolve = nullptr;
     unsigned long long* d_counter = nullptr;
     // RGBA8 colours of up to `cap` samples, then a staging image of `cap` pixels for outputs the
-    // resolve cannot write directly (8 of the 20 bytes per sample that the budget is charged)
+    // resolve cannot write directly (kSampleBytes each)
     void* buf = nullptr;
     uint64_t cap = 0;
     uint64_t extra_bytes = 0;  // budget reserved for a temporary of an oversized piece
@@ -303,7 +309,7 @@ bool Service::pack(Slot& slot, std::unique_lock<std::mutex>& lk) {
         if (!slot.pieces.empty() && samples + pc.samples > slot.cap) break;
         uint64_t extra = 0;
         if (pc.samples > slot.cap) {  // alone, and larger than the slot's buffers
-            extra = pc.samples * 20;
+            extra = pc.samples * kChargedBytes;
             if (extra + slot_bytes > cfg.hbm_budget_bytes) {
                 pending.pop_front();
                 q.pieces_pending--;
@@ -556,10 +562,10 @@ int32_t vt_serve_start(const vt_serve_config* cfg, int32_t* service_out) {
     s->tune.refill_min = cfg->refill_min;
     s->tune.blocks_per_sm = 0;
     s->tune.persistent = 1;
-    s->slot_bytes = cfg->max_inflight * cfg->max_samples_per_launch * 20;
+    s->slot_bytes = cfg->max_inflight * cfg->max_samples_per_launch * kChargedBytes;
     if (s->slot_bytes > cfg->hbm_budget_bytes)
         return fail(VT_ENOMEM, "vt_serve_start: the launch slots' sample buffers (max_inflight x "
-                               "max_samples_per_launch x 20 B) exceed the HBM budget");
+                               "max_samples_per_launch, charged 20 B each) exceed the HBM budget");
     s->slots.resize(cfg->max_inflight);
     for (Slot& sl : s->slots) {
         sl.cap = cfg->max_samples_per_launch;
@@ -570,7 +576,7 @@ int32_t vt_serve_start(const vt_serve_config* cfg, int32_t* service_out) {
         if (e == cudaSuccess) e = cudaMalloc(&sl.d_table, kMaxBatchViews * sizeof(BatchView));
         if (e == cudaSuccess) e = cudaMalloc(&sl.d_resolve, kMaxBatchViews * sizeof(ResolveView));
         if (e == cudaSuccess) e = cudaMalloc(&sl.d_counter, sizeof(unsigned long long));
-        if (e == cudaSuccess) e = cudaMalloc(&sl.buf, sl.cap * 8);
+        if (e == cudaSuccess) e = cudaMalloc(&sl.buf, sl.cap * kSampleBytes);
         if (e == cudaSuccess) e = cudaMallocHost(&sl.h_table, kMaxBatchViews * sizeof(BatchView));
         if (e == cudaSuccess) e = cudaMallocHost(&sl.h_resolve, kMaxBatchViews * sizeof(ResolveView));
         if (e != cudaSuccess) {
