@@ -6,8 +6,8 @@
 //   words   one thread per (brick, z-slice): reads 8 rows of 8 voxels and builds the 64-bit occupancy
 //           word; 32 consecutive bricks share one word of occupancy bits
 //   scan    exclusive prefix sum of those words' bit counts = each occupied brick's slot
-//   compact one warp per 32 bricks: copies the words and voxels of the occupied ones into their
-//           slots; writes the directory
+//   compact one warp per 32 bricks (eight in small lattices): copies the words and voxels of the
+//           occupied ones into their slots; writes the directory
 // In the words pass a warp's lanes are 32 consecutive bricks and a block's eight warps their eight
 // z-slices, so a load instruction reads 256 contiguous bytes of a row.  With lanes running over
 // the slices of four bricks it read eight pieces of 32 bytes from as many planes.

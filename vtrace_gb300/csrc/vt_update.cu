@@ -157,9 +157,10 @@ struct SmallUpdate {
 };
 
 // A thread per row of eight voxels.  Bound by the latency of one block and of its reads over the host
-// link: 7.6 us for a 16^3 u8 chunk, cold (14 us with a thread per slice).  A chunk paged into the resident 1024^3 grid takes 50 us in
-// all against 110 us with an upload, the reorder, the merge, three copies back, a wait, the slots'
-// upload and the scatter around the same lattice passes.
+// link: 7.6 us for a 16^3 u8 chunk, cold (14 us with a thread per slice).  A chunk paged into the resident
+// 1024^3 grid takes 48 us in all against 110 us with an upload, the reorder, the merge, three copies back, a
+// wait, the slots' upload and the scatter around the same lattice passes (the first update after a build, which
+// grows the slots, 355 us).
 template <typename T>
 __global__ void __launch_bounds__(1024) update_small_kernel(GridView g, UpdateBox u, SmallUpdate p,
                                                             SmallExchange* __restrict__ x,
