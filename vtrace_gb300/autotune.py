@@ -10,7 +10,8 @@ fastest and installs it with vt_set_tuning.  The search spaces:
                refilled once 8, 16 or 32 lanes are idle (the compaction interval); persistent
                warps taking whole tiles and tracing their queued shadow rays 32 at a time
   trace_rays   one thread per ray, or persistent warps with a refill threshold of 1, 4, 8, 16, 24
-               or 32 idle lanes and 2 or as many as fit resident blocks per SM
+               or 32 idle lanes and 2 or as many as fit resident blocks per SM (8 idle lanes and as
+               many as fit is the built-in tuning, which takes one thread per ray below 196,608 rays)
   batch        whole tile units per warp over 8x4, 4x8, 16x2 and 32x1-pixel tiles, or per-lane
                refill at 4, 8 or 16 idle lanes, with 2 or as many as fit resident blocks per SM
 
